@@ -6,6 +6,7 @@
 #include <functional>
 #include <cstring>
 #include <new>
+#include <vector>
 
 #include "hd_ctx.h"
 
@@ -88,6 +89,8 @@ hd_status hd_create(const hd_config* cfg, hd_ctx** out)
     hd_status st = guarded(c, [&] {
         Table& t = c->t;
         t.g = c->g;
+        // a page for every virtual page: the pool is direct-mapped
+        t.direct = uint64_t(conf.pool_pages) > c->g.total_vpages ? uint32_t(c->g.total_vpages * HD_PAGE_SIZE) : 0u;
         // 64 bytes past the last page: a node read at its physical offset
         // stays inside the allocation even in a corrupt table
         HD_CUDA(cudaMalloc(&t.pool, size_t(conf.pool_pages) * HD_PAGE_SIZE * 4 + 64));
@@ -98,6 +101,13 @@ hd_status hd_create(const hd_config* cfg, hd_ctx** out)
         // poolTop, free-list count, claim limit
         HD_CUDA(cudaMalloc(&t.pool_top, 16));
         HD_CUDA(cudaMalloc(&t.free_pages, size_t(conf.pool_pages) * 4));
+        t.free_phys = t.free_pages;
+        t.page_ids = t.page_table;
+        if (t.direct) {
+            t.free_phys = t.page_ids = nullptr;
+            HD_CUDA(cudaMalloc(&t.free_phys, size_t(conf.pool_pages) * 4));
+            HD_CUDA(cudaMalloc(&t.page_ids, c->g.total_vpages * 4));
+        }
         HD_CUDA(cudaMalloc(&t.error, 16));
         HD_CUDA(cudaMalloc(&t.level_nodes, HD_MAX_DEPTH * 8));
         HD_CUDA(cudaMalloc(&c->d_root, 4));
@@ -121,6 +131,10 @@ hd_status hd_destroy(hd_ctx* c)
     cudaStreamSynchronize(c->stream);
     hd::batch_release(c);
     hd::color_release(c);
+    if (c->t.direct) {
+        cudaFree(c->t.free_phys);
+        cudaFree(c->t.page_ids);
+    }
     cudaFree(c->t.pool);
     cudaFree(c->t.bloom);
     cudaFree(c->t.page_table);
@@ -511,7 +525,7 @@ hd_status hd_memory_stats(hd_ctx* c, uint64_t* out)
     if (!c || !out)
         return HD_ERR_INVALID;
     out[0] = uint64_t(c->cfg.pool_pages) * HD_PAGE_SIZE * 4 + kPageTableEntries * 4 + c->g.total_buckets * 4 +
-             uint64_t(c->cfg.pool_pages) * kBloomWords * 4;
+             uint64_t(c->cfg.pool_pages) * kBloomWords * 4 + (c->t.direct ? c->g.total_vpages * 4 : 0);
     const ColorTable& ct = c->ct;
     out[1] = ct.cap_nodes * 4 + ct.cap_leaves * sizeof(LeafDesc) + ct.cap_blocks * 8 + ct.cap_macros * 8 +
              ct.cap_weights * 4;
@@ -542,14 +556,18 @@ hd_status hd_export_table(hd_ctx* c, uint32_t* bs, uint32_t* pt, uint32_t* pool,
         cudaStream_t st = c->stream;
         if (bs)
             HD_CUDA(cudaMemcpyAsync(bs, c->t.bucket_sizes, c->g.total_buckets * 4, cudaMemcpyDeviceToHost, st));
-        if (pt)
-            HD_CUDA(cudaMemcpyAsync(pt, c->t.page_table, c->g.total_vpages * 4, cudaMemcpyDeviceToHost, st));
-        if (pool) {
-            const uint64_t top = read_scalar(c->t.pool_top, st);
-            uint64_t words = top * HD_PAGE_SIZE;
-            if (words > pool_cap)
-                words = pool_cap;
-            HD_CUDA(cudaMemcpyAsync(pool, c->t.pool, words * 4, cudaMemcpyDeviceToHost, st));
+        if (pt || pool) {
+            const uint64_t top = pool ? read_scalar(c->t.pool_top, st) : 0;
+            const uint64_t pages = std::min<uint64_t>(top, pool_cap / HD_PAGE_SIZE);
+            // a capacity that ends inside a page
+            const uint64_t rest = pages < top ? pool_cap % HD_PAGE_SIZE : 0;
+            if (rest) {
+                std::vector<uint32_t> whole((pages + 1) * HD_PAGE_SIZE);
+                download_pages(c, pt, whole.data(), pages + 1);
+                std::memcpy(pool, whole.data(), pool_cap * 4);
+            } else {
+                download_pages(c, pt, pool, pages);
+            }
         }
         if (full)
             HD_CUDA(cudaMemcpyAsync(full, c->t.full_nodes, c->cfg.depth * 4, cudaMemcpyDeviceToHost, st));
@@ -568,8 +586,7 @@ hd_status hd_import_table(hd_ctx* c, const uint32_t* bs, const uint32_t* pt, con
         check_table(c->g, pt, bs, uint32_t(pool_words / HD_PAGE_SIZE), root, "the imported table");
         table_reset(c);
         HD_CUDA(cudaMemcpyAsync(c->t.bucket_sizes, bs, c->g.total_buckets * 4, cudaMemcpyHostToDevice, st));
-        HD_CUDA(cudaMemcpyAsync(c->t.page_table, pt, c->g.total_vpages * 4, cudaMemcpyHostToDevice, st));
-        HD_CUDA(cudaMemcpyAsync(c->t.pool, pool, pool_words * 4, cudaMemcpyHostToDevice, st));
+        upload_pages(c, pt, pool, pool_words / HD_PAGE_SIZE);
         HD_CUDA(cudaMemcpyAsync(c->t.full_nodes, full, c->cfg.depth * 4, cudaMemcpyHostToDevice, st));
         const uint32_t top[2] = {uint32_t(pool_words / HD_PAGE_SIZE), 0};
         HD_CUDA(cudaMemcpyAsync(c->t.pool_top, top, 8, cudaMemcpyHostToDevice, st));

@@ -122,6 +122,14 @@ void check_table(const Geom& g, const uint32_t* pt, const uint32_t* bs, uint32_t
 bool valid_root(const Geom& g, uint32_t root, uint32_t pt_entry);
 void bloom_clear_level(hd_ctx* c, uint32_t level);
 
+// hd_table.cu: the table's pages to and from host arrays as exports and files
+// hold them: `pages` pages by their numbers (page 0 the null page) and a
+// page table of total_vpages numbers.  Either output of download_pages may
+// be null.  download_pages waits for its copies; upload_pages expects a
+// table just reset.
+void download_pages(hd_ctx* c, uint32_t* h_page_table, uint32_t* h_pool, uint64_t pages);
+void upload_pages(hd_ctx* c, const uint32_t* h_page_table, const uint32_t* h_pool, uint64_t pages);
+
 // hd_io.cu: keeps a copy of the BasicDAG words (host or device pointer)
 void keep_basic(hd_ctx* c, const uint32_t* words, uint64_t n);
 

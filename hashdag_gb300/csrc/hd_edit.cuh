@@ -628,7 +628,7 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
     // the bucket's page-table entries, lane p holding page p's (the warp owns
     // the bucket for the run: only its own appends map pages here)
     const uint32_t vpage0 = vbase >> kPageShift, cap_pages = t.g.capacity(level) >> kPageShift;
-    uint32_t pt_lane = lane < cap_pages ? __ldcg(t.page_table + vpage0 + lane) : 0u;
+    uint32_t pt_lane = lane < cap_pages ? t.page_cg(vpage0 + lane) : 0u;
     uint32_t used_entries = 0, next_slot = 0;
     bool failed = false;
     uint32_t j = j0;
@@ -712,7 +712,7 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
                     ok = 0;
                 } else {
                     const uint32_t phys =
-                        a_mapped && (pos >> kPageShift) < 32 ? a_phys : __ldcg(t.page_table + vpage0 + (pos >> kPageShift));
+                        a_mapped && (pos >> kPageShift) < 32 ? a_phys : t.page_cg(vpage0 + (pos >> kPageShift));
                     uint32_t* dst = t.pool + (uint64_t(phys) << kPageShift) + (pos & (kPage - 1));
                     for (uint32_t k = 0; k < n; k++)
                         __stcg(dst + k, q[k]);
@@ -737,7 +737,7 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
         S = __shfl_sync(0xffffffffu, S, 0);
         // an append that reached a new page mapped it: refresh that lane
         if (appended && lane < cap_pages && lane * kPage < S && lane * kPage + kPage > S_before)
-            pt_lane = __ldcg(t.page_table + vpage0 + lane);
+            pt_lane = t.page_cg(vpage0 + lane);
         foa++;
         added += appended;
         if (!ok) {

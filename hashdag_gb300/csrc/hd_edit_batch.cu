@@ -844,17 +844,28 @@ void copy_table(hd_ctx* to, hd_ctx* from)
 {
     cudaStream_t st = from->stream;
     HD_CUDA(cudaStreamSynchronize(to->stream));
-    const uint32_t top_from = read_scalar(from->t.pool_top, st);
-    const uint32_t top_to = read_scalar(to->t.pool_top, to->stream);
-    if (top_to > top_from)
-        HD_CUDA(cudaMemsetAsync(to->t.pool + uint64_t(top_from) * kPage, 0, uint64_t(top_to - top_from) * kPage * 4,
+    if (from->t.direct) {
+        // pages lie anywhere in a direct-mapped pool: all of it
+        HD_CUDA(cudaMemcpyAsync(to->t.pool, from->t.pool, uint64_t(from->g.pool_pages) * kPage * 4,
+                                cudaMemcpyDeviceToDevice, st));
+        HD_CUDA(cudaMemcpyAsync(to->t.bloom, from->t.bloom, uint64_t(from->g.pool_pages) * kBloomWords * 4,
+                                cudaMemcpyDeviceToDevice, st));
+        HD_CUDA(cudaMemcpyAsync(to->t.page_ids, from->t.page_ids, from->g.total_vpages * 4, cudaMemcpyDeviceToDevice,
                                 st));
-    HD_CUDA(cudaMemcpyAsync(to->t.pool, from->t.pool, uint64_t(top_from) * kPage * 4, cudaMemcpyDeviceToDevice, st));
-    if (top_to > top_from)
-        HD_CUDA(cudaMemsetAsync(to->t.bloom + uint64_t(top_from) * kBloomWords, 0,
-                                uint64_t(top_to - top_from) * kBloomWords * 4, st));
-    HD_CUDA(cudaMemcpyAsync(to->t.bloom, from->t.bloom, uint64_t(top_from) * kBloomWords * 4, cudaMemcpyDeviceToDevice,
-                            st));
+    } else {
+        const uint32_t top_from = read_scalar(from->t.pool_top, st);
+        const uint32_t top_to = read_scalar(to->t.pool_top, to->stream);
+        if (top_to > top_from)
+            HD_CUDA(cudaMemsetAsync(to->t.pool + uint64_t(top_from) * kPage, 0,
+                                    uint64_t(top_to - top_from) * kPage * 4, st));
+        HD_CUDA(
+            cudaMemcpyAsync(to->t.pool, from->t.pool, uint64_t(top_from) * kPage * 4, cudaMemcpyDeviceToDevice, st));
+        if (top_to > top_from)
+            HD_CUDA(cudaMemsetAsync(to->t.bloom + uint64_t(top_from) * kBloomWords, 0,
+                                    uint64_t(top_to - top_from) * kBloomWords * 4, st));
+        HD_CUDA(cudaMemcpyAsync(to->t.bloom, from->t.bloom, uint64_t(top_from) * kBloomWords * 4,
+                                cudaMemcpyDeviceToDevice, st));
+    }
     HD_CUDA(cudaMemcpyAsync(to->t.page_table, from->t.page_table, from->g.total_vpages * 4, cudaMemcpyDeviceToDevice,
                             st));
     HD_CUDA(cudaMemcpyAsync(to->t.bucket_sizes, from->t.bucket_sizes, from->g.total_buckets * 4,

@@ -117,22 +117,27 @@ __global__ void k_gc_release(Table t, uint32_t level, const uint32_t* __restrict
         const uint32_t size = sizes[bucket], cap = g.capacity(level);
         for (uint32_t off = (size + kPage - 1) & ~(kPage - 1); off < cap; off += kPage) {
             const uint32_t vp = g.make_ptr(level, bucket, off) >> kPageShift;
-            const uint32_t p = t.page_table[vp];
+            const uint32_t p = t.page_ids[vp];
             if (p) {
+                const uint32_t k = atomicAdd(free_count, 1u);
+                t.free_pages[k] = p;
+                if (t.direct) {
+                    t.free_phys[k] = vp + 1;
+                    t.page_ids[vp] = 0;
+                }
                 t.page_table[vp] = 0;
-                t.free_pages[atomicAdd(free_count, 1u)] = p;
             }
         }
     }
 }
 
-// Zeroes the pages free_pages[from, to) and their Bloom filters.
+// Zeroes the pages [from, to) of the free list and their Bloom filters.
 __global__ void k_zero_pages(Table t, uint32_t from, uint32_t to)
 {
     const uint64_t n = uint64_t(to - from) * kPage;
     HD_GRID_STRIDE(i, n)
     {
-        const uint32_t p = t.free_pages[from + uint32_t(i / kPage)];
+        const uint32_t p = t.free_phys[from + uint32_t(i / kPage)];
         t.pool[uint64_t(p) * kPage + (i % kPage)] = 0;
         if (i % kPage < kBloomWords)
             t.bloom[uint64_t(p) * kBloomWords + (i % kPage)] = 0;

@@ -247,8 +247,7 @@ hd_status hd_save_snapshot(hd_ctx* c, const char* path, const hd_dag_info* info)
             full(c->cfg.depth);
         std::vector<uint64_t> level_nodes(HD_MAX_DEPTH);
         HD_CUDA(cudaMemcpyAsync(level_nodes.data(), c->t.level_nodes, HD_MAX_DEPTH * 8, cudaMemcpyDeviceToHost, st));
-        HD_CUDA(cudaMemcpyAsync(pool.data(), c->t.pool, pool.size() * 4, cudaMemcpyDeviceToHost, st));
-        HD_CUDA(cudaMemcpyAsync(pt.data(), c->t.page_table, pt.size() * 4, cudaMemcpyDeviceToHost, st));
+        download_pages(c, pt.data(), pool.data(), pool_top);
         HD_CUDA(cudaMemcpyAsync(bs.data(), c->t.bucket_sizes, bs.size() * 4, cudaMemcpyDeviceToHost, st));
         HD_CUDA(cudaMemcpyAsync(full.data(), c->t.full_nodes, full.size() * 4, cudaMemcpyDeviceToHost, st));
         const uint64_t* tops = c->ctop;
@@ -375,8 +374,7 @@ hd_status hd_load_snapshot(hd_ctx* c, const char* path, hd_dag_info* info)
         }
         check_table(g, pt.data(), extension ? bs.data() : nullptr, pool_top, root, in.path);
         table_reset(c);
-        HD_CUDA(cudaMemcpyAsync(c->t.pool, pool.data(), pool.size() * 4, cudaMemcpyHostToDevice, st));
-        HD_CUDA(cudaMemcpyAsync(c->t.page_table, pt.data(), pt.size() * 4, cudaMemcpyHostToDevice, st));
+        upload_pages(c, pt.data(), pool.data(), pool_top);
         HD_CUDA(cudaMemcpyAsync(c->t.bucket_sizes, bs.data(), bs.size() * 4, cudaMemcpyHostToDevice, st));
         HD_CUDA(cudaMemcpyAsync(c->t.full_nodes, full.data(), full.size() * 4, cudaMemcpyHostToDevice, st));
         HD_CUDA(cudaMemcpyAsync(c->t.level_nodes, level_nodes.data(), HD_MAX_DEPTH * 8, cudaMemcpyHostToDevice, st));

@@ -111,6 +111,8 @@ void table_reset(hd_ctx* c)
     HD_CUDA(cudaMemsetAsync(c->t.pool, 0, size_t(g.pool_pages) * kPage * 4 + 64, c->stream));
     HD_CUDA(cudaMemsetAsync(c->t.bloom, 0, size_t(g.pool_pages) * kBloomWords * 4, c->stream));
     HD_CUDA(cudaMemsetAsync(c->t.page_table, 0, kPageTableEntries * 4, c->stream));
+    if (c->t.direct)
+        HD_CUDA(cudaMemsetAsync(c->t.page_ids, 0, g.total_vpages * 4, c->stream));
     HD_CUDA(cudaMemsetAsync(c->t.bucket_sizes, 0, g.total_buckets * 4, c->stream));
     HD_CUDA(cudaMemsetAsync(c->t.full_nodes, 0, HD_MAX_DEPTH * 4, c->stream));
     HD_CUDA(cudaMemsetAsync(c->t.level_nodes, 0, HD_MAX_DEPTH * 8, c->stream));
@@ -119,6 +121,94 @@ void table_reset(hd_ctx* c)
     HD_CUDA(cudaMemcpyAsync(c->t.pool_top, top, 8, cudaMemcpyHostToDevice, c->stream));
     set_claim_limit(c, false);
     HD_CUDA(cudaMemsetAsync(c->d_root, 0, 4, c->stream));
+}
+
+// ---------------------------------------------------------------------------
+// Tables in host memory and in files number their pages in claim order
+// (1, 2, ...), with a page table of those numbers.  That is how a pool filled
+// in claim order lies; the pages of a direct-mapped one are gathered on the
+// way out and spread on the way in by their numbers (page_ids), kIoPages at a
+// time through a staging buffer.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kIoPages = 32768; // 64 MB
+
+__global__ void k_direct_entries(Table t, uint64_t n)
+{
+    HD_GRID_STRIDE(i, n) t.page_table[i] = t.page_ids[i] ? uint32_t(i) + 1 : 0;
+}
+
+// Copies the pages of a direct-mapped pool whose number is in [a, b) to (OUT)
+// or from the staging buffer: a warp looks at 32 virtual pages at a time and
+// copies those in range one after the other.
+template <bool OUT>
+__global__ void k_move_pages(Table t, uint64_t n, uint32_t a, uint32_t b, uint32_t* __restrict__ staging)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warp = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
+    const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+    for (uint64_t v0 = warp * 32; v0 < n; v0 += warps * 32) {
+        const uint32_t e = v0 + lane < n ? t.page_ids[v0 + lane] : 0u;
+        uint32_t todo = __ballot_sync(0xffffffffu, e != 0 && e >= a && e < b);
+        while (todo) {
+            const uint32_t k = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t page = __shfl_sync(0xffffffffu, e, k);
+            uint4* in_pool = reinterpret_cast<uint4*>(t.pool + (v0 + k + 1) * kPage);
+            uint4* in_staging = reinterpret_cast<uint4*>(staging + uint64_t(page - a) * kPage);
+            for (uint32_t w = lane; w < kPage / 4; w += 32) {
+                if (OUT)
+                    in_staging[w] = in_pool[w];
+                else
+                    in_pool[w] = in_staging[w];
+            }
+        }
+    }
+}
+
+void download_pages(hd_ctx* c, uint32_t* h_page_table, uint32_t* h_pool, uint64_t pages)
+{
+    cudaStream_t st = c->stream;
+    const uint64_t nv = c->g.total_vpages;
+    if (h_page_table)
+        HD_CUDA(cudaMemcpyAsync(h_page_table, c->t.page_ids, nv * 4, cudaMemcpyDeviceToHost, st));
+    if (h_pool && pages && !c->t.direct)
+        HD_CUDA(cudaMemcpyAsync(h_pool, c->t.pool, pages * kPage * 4, cudaMemcpyDeviceToHost, st));
+    if (h_pool && pages && c->t.direct) {
+        uint32_t* staging = c->scratch.get<uint32_t>("io_staging", std::min<uint64_t>(pages, kIoPages) * kPage);
+        for (uint64_t a = 0; a < pages; a += kIoPages) {
+            const uint64_t n = std::min<uint64_t>(pages - a, kIoPages);
+            HD_CUDA(cudaMemsetAsync(staging, 0, n * kPage * 4, st)); // the null page and pages on the free list
+            k_move_pages<true><<<grid_for(nv, 256), 256, 0, st>>>(c->t, nv, uint32_t(a), uint32_t(a + n), staging);
+            HD_LAUNCH_CHECK();
+            HD_CUDA(cudaMemcpyAsync(h_pool + a * kPage, staging, n * kPage * 4, cudaMemcpyDeviceToHost, st));
+        }
+    }
+    HD_CUDA(cudaStreamSynchronize(st));
+    c->scratch.drop("io_staging");
+}
+
+void upload_pages(hd_ctx* c, const uint32_t* h_page_table, const uint32_t* h_pool, uint64_t pages)
+{
+    cudaStream_t st = c->stream;
+    const uint64_t nv = c->g.total_vpages;
+    HD_CUDA(cudaMemcpyAsync(c->t.page_ids, h_page_table, nv * 4, cudaMemcpyHostToDevice, st));
+    if (!c->t.direct) {
+        HD_CUDA(cudaMemcpyAsync(c->t.pool, h_pool, pages * kPage * 4, cudaMemcpyHostToDevice, st));
+        return;
+    }
+    k_direct_entries<<<grid_for(nv, 256), 256, 0, st>>>(c->t, nv);
+    HD_LAUNCH_CHECK();
+    if (pages) {
+        uint32_t* staging = c->scratch.get<uint32_t>("io_staging", std::min<uint64_t>(pages, kIoPages) * kPage);
+        for (uint64_t a = 0; a < pages; a += kIoPages) {
+            const uint64_t n = std::min<uint64_t>(pages - a, kIoPages);
+            HD_CUDA(cudaMemcpyAsync(staging, h_pool + a * kPage, n * kPage * 4, cudaMemcpyHostToDevice, st));
+            k_move_pages<false><<<grid_for(nv, 256), 256, 0, st>>>(c->t, nv, uint32_t(a), uint32_t(a + n), staging);
+            HD_LAUNCH_CHECK();
+        }
+    }
+    HD_CUDA(cudaStreamSynchronize(st));
+    c->scratch.drop("io_staging");
 }
 
 void set_claim_limit(hd_ctx* c, bool gc)

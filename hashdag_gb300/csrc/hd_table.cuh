@@ -33,6 +33,8 @@ HD_HD uint32_t append_position(uint32_t& size, uint32_t n, bool leaf)
 // end is given back at once, so poolTop never exceeds the pool (the
 // reference, unchecked in release builds, would write past its pool).
 // Free-list pops may run concurrently; pushes happen only inside a GC.
+// Returns the page's number, which is also where it lies unless the pool is
+// direct-mapped (place_page).
 HD_D uint32_t claim_page(const Table& t)
 {
     uint32_t* free_count = t.pool_top + 1;
@@ -48,6 +50,14 @@ HD_D uint32_t claim_page(const Table& t)
         return 0;
     }
     return p;
+}
+
+// Virtual page vp gets the claimed page p.
+HD_D void place_page(const Table& t, uint32_t vp, uint32_t p)
+{
+    if (t.direct)
+        __stcg(t.page_ids + vp, p);
+    __stcg(t.page_table + vp, t.direct ? vp + 1 : p);
 }
 
 // Maps every unmapped virtual page that [from, to) of the bucket touches.
@@ -66,7 +76,7 @@ HD_D bool map_pages(const Table& t, uint32_t level, uint32_t bucket, uint32_t fr
                 set_error(t.error, kErrPoolFull, level, bucket, __ldcg(t.pool_top + 2));
                 return false;
             }
-            __stcg(t.page_table + vp, p);
+            place_page(t, vp, p);
         }
     }
     return true;
@@ -75,7 +85,7 @@ HD_D bool map_pages(const Table& t, uint32_t level, uint32_t bucket, uint32_t fr
 // The filter of the physical page behind virtual word v
 HD_D uint32_t* bloom_of(const Table& t, uint32_t v)
 {
-    return t.bloom + uint64_t(__ldcg(t.page_table + (v >> kPageShift))) * kBloomWords;
+    return t.bloom + uint64_t(t.page_cg(v >> kPageShift)) * kBloomWords;
 }
 // Adds a node written at virtual word v to its page's filter
 HD_D void bloom_add(const Table& t, uint32_t v, uint32_t bits)

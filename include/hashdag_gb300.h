@@ -604,7 +604,8 @@ hd_status hd_import_table(hd_ctx* ctx, const uint32_t* h_bucket_sizes, const uin
                           const uint32_t* h_pool, uint64_t pool_words,
                           const uint32_t* h_full_nodes, uint32_t root);
 /* Device pointers of the table (for zero-copy consumers): pool, page
- * table, bucket sizes. */
+ * table, bucket sizes.  Virtual page p lies at pool page page_table[p] (0:
+ * unmapped); pages lie anywhere in the pool. */
 hd_status hd_device_table(hd_ctx* ctx, uint32_t** d_pool, uint32_t** d_page_table,
                           uint32_t** d_bucket_sizes);
 
