@@ -21,16 +21,23 @@
 
 namespace hd {
 
+// Bound by the atomics on the words of widely shared children: every parent
+// of a level's full node sets the same bit.  The bit is looked at first (a
+// cached read; one from L2 when that copy does not show it, as a stale line
+// may not), so that an atomic runs only for a bit not yet seen set: the 12
+// mark launches of a 2^14 scene go from 6,959 to 369 us.
 __global__ void k_gc_mark(Table t, const uint32_t* __restrict__ live, uint32_t n, uint32_t child_base,
-                          uint32_t* __restrict__ bitmap)
+                          uint32_t* bitmap)
 {
     HD_GRID_STRIDE(i, n)
     {
         const uint32_t* p = t.sys(live[i]);
         const uint32_t cnt = popc32(p[0] & 0xffu);
         for (uint32_t k = 0; k < cnt; k++) {
-            const uint32_t off = p[1 + k] - child_base;
-            atomicOr(bitmap + (off >> 5), 1u << (off & 31));
+            const uint32_t off = p[1 + k] - child_base, bit = 1u << (off & 31);
+            uint32_t* w = bitmap + (off >> 5);
+            if (!(__ldca(w) & bit) && !(__ldcg(w) & bit))
+                atomicOr(w, bit);
         }
     }
 }
@@ -68,39 +75,253 @@ HD_D uint32_t lower_bound(const uint32_t* v, uint32_t n, uint32_t x)
     return lo;
 }
 
-// Gathers the live nodes of a level (children remapped) before the level is
-// emptied; hashes and links them into the bucket lists.  A child's index in
-// the live list of the level below is its rank in that level's mark bitmap:
-// the live count of the bitmap words before it (child_pos) plus the bits
-// below it in its word.
-__global__ void k_gc_gather(Table t, uint32_t level, const uint32_t* __restrict__ live, uint32_t n,
-                            const uint32_t* __restrict__ child_bitmap, const uint32_t* __restrict__ child_pos,
-                            uint32_t child_base, const uint32_t* __restrict__ child_new,
-                            uint32_t* __restrict__ content,
-                            uint32_t* __restrict__ head, uint32_t* __restrict__ next, uint32_t* __restrict__ touched,
-                            uint32_t* __restrict__ n_touched)
+// A live node with its children remapped.  A child's index in the live list
+// of the level below is its rank in that level's mark bitmap: the live count
+// of the bitmap words before it (pos) plus the bits below it in its word.
+struct ChildMap {
+    const uint32_t* bitmap;
+    const uint32_t* pos;
+    const uint32_t* new_addr;
+    uint32_t base;
+};
+HD_D uint32_t remapped_node(const Table& t, uint32_t v, bool leaf, const ChildMap& m, uint32_t* c)
+{
+    const uint32_t* p = t.sys(v);
+    c[0] = p[0];
+    if (leaf) {
+        c[1] = p[1];
+        return 2;
+    }
+    const uint32_t cnt = popc32(c[0] & 0xffu);
+#pragma unroll
+    for (uint32_t k = 0; k < 8; k++)
+        if (k < cnt) {
+            const uint32_t off = p[1 + k] - m.base, w = off >> 5;
+            c[1 + k] = m.new_addr[m.pos[w] + popc32(m.bitmap[w] & ((1u << (off & 31)) - 1u))];
+        }
+    return cnt + 1;
+}
+
+// ---- dry run: every level's new addresses, before anything changes ----------
+// The rebuild of a level re-appends its live nodes with a different order
+// and so a different padding: a bucket can need a page it never had.  A
+// rebuild that runs out of pages half way cannot be undone, so the GC first
+// runs every level's rebuild on scratch bucket sizes (the full node first,
+// then the live nodes in increasing old address) and counts the pages it
+// would map, and the pages a releasing GC would free.  The addresses stay:
+// the rebuild itself then writes every node to its address, node by node in
+// parallel, with no order to keep.
+// A releasing GC frees a level's pages that lie wholly past their bucket's
+// final size before it rebuilds the level, so the same level's buckets can
+// take them: re-hashed parents (children remapped) move between buckets, and
+// one bucket's growth is met by another's shrinkage.
+
+// The level's full node at the head of its (empty) bucket, on dry sizes.
+__global__ void k_gc_dry_full(Table t, uint32_t level, uint32_t* dry_sizes, uint32_t* full_dry)
+{
+    uint32_t node[9];
+    uint32_t n, hash;
+    const bool leaf = level == t.g.leaf_level;
+    if (leaf) {
+        node[0] = node[1] = 0xFFFFFFFFu;
+        n = 2;
+        hash = hash_leaf(~0ull);
+    } else {
+        const uint32_t depth = t.g.depth - level;
+        const uint32_t voxels = level < t.g.T ? 0u : (1u << (3 * depth));
+        node[0] = (voxels << 8) | 0xffu;
+        for (int c = 0; c < 8; c++)
+            node[1 + c] = full_dry[level + 1];
+        n = 9;
+        hash = hash_interior(9, node);
+    }
+    const uint32_t bucket = hash & (t.g.buckets(level) - 1);
+    dry_sizes[bucket] = n;
+    full_dry[level] = t.g.make_ptr(level, bucket, 0);
+}
+
+// Bucket and size of every live node (bucket | words << 24; buckets stay
+// below 2^24) and its arrival rank in the bucket, in any order.
+__global__ void k_gc_keys(Table t, uint32_t level, const uint32_t* __restrict__ live, uint32_t n, ChildMap m,
+                          uint32_t* __restrict__ keys, uint32_t* __restrict__ rank, uint32_t* __restrict__ counts)
 {
     const bool leaf = level == t.g.leaf_level;
     HD_GRID_STRIDE(i, n)
     {
-        const uint32_t* p = t.sys(live[i]);
-        uint32_t* c = content + 9 * i;
-        uint32_t hash;
-        if (leaf) {
-            c[0] = p[0];
-            c[1] = p[1];
-            hash = hash_leaf(uint64_t(c[0]) | (uint64_t(c[1]) << 32));
-        } else {
-            const uint32_t cnt = popc32(p[0] & 0xffu);
-            c[0] = p[0];
-            for (uint32_t k = 0; k < cnt; k++) {
-                const uint32_t off = p[1 + k] - child_base, w = off >> 5;
-                c[1 + k] = child_new[child_pos[w] + popc32(child_bitmap[w] & ((1u << (off & 31)) - 1u))];
-            }
-            hash = hash_interior(cnt + 1, c);
-        }
+        uint32_t c[9];
+        const uint32_t words = remapped_node(t, live[i], leaf, m, c);
+        const uint32_t hash = leaf ? hash_leaf(uint64_t(c[0]) | (uint64_t(c[1]) << 32)) : hash_interior(words, c);
         const uint32_t bucket = hash & (t.g.buckets(level) - 1);
-        link_item(t.g.bucket_global(level, bucket), uint32_t(i), head, next, touched, n_touched);
+        keys[i] = bucket | (words << 24);
+        rank[i] = atomicAdd(counts + bucket, 1u);
+    }
+}
+
+__global__ void k_gc_group(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ rank,
+                           const uint32_t* __restrict__ first, uint32_t n, uint32_t* __restrict__ items)
+{
+    HD_GRID_STRIDE(i, n) items[first[keys[i] & 0xFFFFFFu] + rank[i]] = uint32_t(i);
+}
+
+// A warp per bucket: its items in increasing order, appended one after the
+// other to the dry size (append_position), 32 at a time: the sizes' prefix
+// sums place every node up to the first that would straddle a page, which
+// starts the next page.  Then the bucket's pages: those the rebuild maps
+// (unmapped, below the final size) and, releasing, frees (mapped, wholly
+// past it).
+// Bound by latency (a sort of a few dozen items, dependent shuffles).  When
+// the buckets were linked lists that one lane walked and then appended from,
+// the 13 dry and 13 real appends of a 2^14 scene took 892 and 2,313 us; the
+// groups and these assignments take 372 + 60 us, k_gc_write and k_gc_map 241.
+constexpr uint32_t kGcWarps = 2;
+__global__ void __launch_bounds__(32 * kGcWarps)
+    k_gc_assign(Table t, uint32_t level, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ counts,
+                const uint32_t* __restrict__ first, const uint32_t* __restrict__ list, uint32_t* __restrict__ dry_sizes,
+                uint32_t* __restrict__ out_addr, uint32_t* __restrict__ overflow, uint32_t release,
+                unsigned long long* need, unsigned long long* freed)
+{
+    __shared__ uint32_t items_s[kGcWarps][kMaxBucketItems];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t* items = items_s[warp];
+    const bool leaf = level == t.g.leaf_level;
+    const uint32_t nb = t.g.buckets(level), cap = t.g.capacity(level);
+    unsigned long long a = 0, f = 0;
+    for (uint32_t bucket = blockIdx.x * kGcWarps + warp; bucket < nb; bucket += gridDim.x * kGcWarps) {
+        uint32_t cnt = counts[bucket], size = dry_sizes[bucket];
+        if (cnt > kMaxBucketItems) {
+            if (lane == 0)
+                set_error(t.error, kErrBucketFull, 0xFFFFFFFFu, t.g.bucket_global(level, bucket), cnt);
+            cnt = 0;
+        }
+        if (cnt) {
+            const uint32_t* src = list + first[bucket];
+            if (cnt <= 32) {
+                // in registers: a bitonic network over the lanes
+                uint32_t x = lane < cnt ? src[lane] : kEmpty;
+                for (uint32_t k = 2; k <= 32; k <<= 1)
+                    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+                        x = ((lane & k) == 0) == ((lane & j) == 0) ? min(x, y) : max(x, y);
+                    }
+                items[lane] = x;
+            } else {
+                uint32_t n2 = 64;
+                while (n2 < cnt)
+                    n2 <<= 1;
+                for (uint32_t i = lane; i < n2; i += 32)
+                    items[i] = i < cnt ? src[i] : kEmpty;
+                __syncwarp();
+                sort_shared(items, n2);
+            }
+            __syncwarp();
+            for (uint32_t i0 = 0; i0 < cnt; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                const uint32_t r = i < cnt ? items[i] : 0u;
+                const uint32_t n = i < cnt ? (leaf ? 2u : keys[r] >> 24) : 0u;
+                const uint32_t inc = warp_incl_scan(n);
+                uint32_t done = 0, pos = 0; // words of the items placed so far, this lane's position
+                bool placed = n == 0;
+                for (;;) {
+                    // room in the page the size ends in (512 at a page start);
+                    // leaves pack pages exactly (even sizes), so they are
+                    // placed like nodes that never straddle
+                    const uint32_t room = kPage - (size & (kPage - 1));
+                    const bool fits = !placed && (leaf || inc - done <= room);
+                    const uint32_t fb = __ballot_sync(0xffffffffu, fits);
+                    if (fb) {
+                        if (fits) {
+                            pos = size + (inc - done) - n;
+                            placed = true;
+                        }
+                        const uint32_t all = __shfl_sync(0xffffffffu, inc, 31 - __clz(fb));
+                        size += all - done;
+                        done = all;
+                    }
+                    if (!__any_sync(0xffffffffu, !placed))
+                        break;
+                    size = (size + kPage - 1) & ~(kPage - 1); // the next node starts a page
+                }
+                if (i < cnt)
+                    out_addr[r] = t.g.make_ptr(level, bucket, pos);
+            }
+            if (lane == 0) {
+                if (size > cap)
+                    atomicExch(overflow, 1u);
+                dry_sizes[bucket] = size;
+            }
+        }
+        for (uint32_t off = lane * kPage; off < cap; off += 32 * kPage) {
+            const bool mapped = t.page_table[t.g.make_ptr(level, bucket, off) >> kPageShift] != 0;
+            if (off < size)
+                a += !mapped;
+            else if (release)
+                f += mapped;
+        }
+        __syncwarp();
+    }
+    for (int o = 16; o; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        f += __shfl_down_sync(0xffffffffu, f, o);
+    }
+    if (lane == 0 && a)
+        atomicAdd(need, a);
+    if (lane == 0 && f)
+        atomicAdd(freed, f);
+}
+
+// ---- rebuild of a level ---------------------------------------------------------
+// The live nodes, children remapped, staged before the level's pages are
+// written.
+__global__ void k_gc_gather(Table t, uint32_t level, const uint32_t* __restrict__ live, uint32_t n, ChildMap m,
+                            uint32_t* __restrict__ content)
+{
+    const bool leaf = level == t.g.leaf_level;
+    HD_GRID_STRIDE(i, n)
+    {
+        uint32_t c[9];
+        const uint32_t words = remapped_node(t, live[i], leaf, m, c);
+#pragma unroll
+        for (uint32_t k = 0; k < 9; k++)
+            if (k < words)
+                content[9 * i + k] = c[k];
+    }
+}
+
+// The buckets' final sizes, with every page below them mapped (after the
+// full node's).
+__global__ void k_gc_map(Table t, uint32_t level, const uint32_t* __restrict__ dry_sizes, uint32_t n)
+{
+    HD_GRID_STRIDE(b, uint64_t(t.g.buckets(level)))
+    {
+        const uint32_t size = dry_sizes[b];
+        if (map_pages(t, level, uint32_t(b), 0, size))
+            t.bucket_sizes[t.g.bucket_global(level, uint32_t(b))] = size;
+        if (b == 0)
+            t.level_nodes[level] += n;
+    }
+}
+
+// Every staged node to its address, and into its page's filter.
+__global__ void k_gc_write(Table t, uint32_t level, const uint32_t* __restrict__ content,
+                           const uint32_t* __restrict__ addr, uint32_t n)
+{
+    const bool leaf = level == t.g.leaf_level;
+    HD_GRID_STRIDE(i, n)
+    {
+        uint32_t c[9];
+        c[0] = content[9 * i];
+        const uint32_t words = leaf ? 2 : total_size(c[0]);
+#pragma unroll
+        for (uint32_t k = 1; k < 9; k++)
+            if (k < words)
+                c[k] = content[9 * i + k];
+        const uint32_t v = addr[i];
+        uint32_t* dst = t.sys_rw(v);
+#pragma unroll
+        for (uint32_t k = 0; k < 9; k++)
+            if (k < words)
+                dst[k] = c[k];
+        bloom_add(t, v, bloom_bits(c, words));
     }
 }
 
@@ -141,106 +362,6 @@ __global__ void k_zero_pages(Table t, uint32_t from, uint32_t to)
         t.pool[uint64_t(p) * kPage + (i % kPage)] = 0;
         if (i % kPage < kBloomWords)
             t.bloom[uint64_t(p) * kBloomWords + (i % kPage)] = 0;
-    }
-}
-
-// ---- dry run: the rebuild's page needs, computed before anything changes ----
-// The rebuild of a level re-appends its live nodes with a different order
-// and so a different padding: a bucket can need a page it never had.  A
-// rebuild that runs out of pages half way cannot be undone, so the GC first
-// runs every level's rebuild on scratch bucket sizes (the same full node
-// first, the same items in the same order, hence the same addresses) and
-// counts the pages it would map, and the pages a releasing GC would free.
-// A releasing GC frees a level's pages that lie wholly past their bucket's
-// final size (kept from the dry run) before it re-appends the level, so the
-// appends of the same level can take them: re-hashed parents (children
-// remapped) move between buckets, and one bucket's growth is met by
-// another's shrinkage.
-
-// The level's full node at the head of its (empty) bucket, on dry sizes.
-__global__ void k_gc_dry_full(Table t, uint32_t level, uint32_t* dry_sizes, uint32_t* full_dry)
-{
-    uint32_t node[9];
-    uint32_t n, hash;
-    const bool leaf = level == t.g.leaf_level;
-    if (leaf) {
-        node[0] = node[1] = 0xFFFFFFFFu;
-        n = 2;
-        hash = hash_leaf(~0ull);
-    } else {
-        const uint32_t depth = t.g.depth - level;
-        const uint32_t voxels = level < t.g.T ? 0u : (1u << (3 * depth));
-        node[0] = (voxels << 8) | 0xffu;
-        for (int c = 0; c < 8; c++)
-            node[1 + c] = full_dry[level + 1];
-        n = 9;
-        hash = hash_interior(9, node);
-    }
-    const uint32_t bucket = hash & (t.g.buckets(level) - 1);
-    dry_sizes[bucket] = n;
-    full_dry[level] = t.g.make_ptr(level, bucket, 0);
-}
-
-// The items' addresses and the buckets' final sizes, as k_append_items
-// places them, without writing the table.
-__global__ void __launch_bounds__(64)
-    k_gc_dry_append(Table t, uint32_t level, const uint32_t* __restrict__ content, uint32_t* __restrict__ head,
-                    const uint32_t* __restrict__ next, const uint32_t* __restrict__ touched,
-                    const uint32_t* __restrict__ n_touched, uint32_t* __restrict__ dry_sizes,
-                    uint32_t* __restrict__ out_addr, uint32_t* __restrict__ overflow)
-{
-    __shared__ uint32_t items_s[2][kMaxBucketItems];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t* items = items_s[warp];
-    const bool leaf = level == t.g.leaf_level;
-    const uint32_t nt = *n_touched;
-    const uint32_t first = t.g.level_first_bucket(level);
-    for (uint32_t ti = blockIdx.x * 2 + warp; ti < nt; ti += gridDim.x * 2) {
-        const uint32_t gb = touched[ti];
-        const uint32_t cnt = collect_sorted(gb, head, next, items, t.error);
-        if (cnt == 0)
-            continue;
-        const uint32_t bucket = gb - first;
-        if (lane == 0) {
-            uint32_t size = dry_sizes[bucket];
-            for (uint32_t i = 0; i < cnt; i++) {
-                const uint32_t r = items[i];
-                const uint32_t n = leaf ? 2 : total_size(content[9 * uint64_t(r)]);
-                out_addr[r] = t.g.make_ptr(level, bucket, append_position(size, n, leaf));
-            }
-            if (size > t.g.capacity(level))
-                atomicExch(overflow, 1u);
-            dry_sizes[bucket] = size;
-        }
-        __syncwarp();
-    }
-}
-
-// Pages the level's rebuild maps (unmapped pages below a bucket's final
-// size) and, releasing, frees (mapped pages wholly past it).
-__global__ void k_gc_dry_pages(Table t, uint32_t level, const uint32_t* __restrict__ dry_sizes, uint32_t release,
-                               unsigned long long* need, unsigned long long* freed)
-{
-    const uint32_t cap = t.g.capacity(level);
-    unsigned long long a = 0, f = 0;
-    HD_GRID_STRIDE(i, t.g.buckets(level))
-    {
-        const uint32_t bucket = uint32_t(i), size = dry_sizes[bucket];
-        for (uint32_t off = 0; off < cap; off += kPage) {
-            const bool mapped = t.page_table[t.g.make_ptr(level, bucket, off) >> kPageShift] != 0;
-            if (off < size)
-                a += !mapped;
-            else if (release)
-                f += mapped;
-        }
-    }
-    for (int o = 16; o; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        f += __shfl_down_sync(0xffffffffu, f, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(need, a);
-        atomicAdd(freed, f);
     }
 }
 
@@ -314,87 +435,81 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
         k_bitmap_to_list<<<grid_for(nwords, 256), 256, 0, st>>>(bitmap, pos, nwords, base, live[L + 1]);
         HD_LAUNCH_CHECK();
     }
-    uint32_t maxn = 1;
-    for (uint32_t L = 0; L <= leafl; L++)
+    uint32_t maxn = 1, max_buckets = 1;
+    for (uint32_t L = 0; L <= leafl; L++) {
         maxn = std::max(maxn, nlive[L]);
-    uint32_t* content = s.get<uint32_t>("gc_content", uint64_t(maxn) * 9);
-    uint32_t* next = s.get<uint32_t>("gc_next", maxn);
-    uint32_t* head = s.get<uint32_t>("gc_head", g.total_buckets);
-    uint32_t* touched = s.get<uint32_t>("gc_touched", g.total_buckets);
-    fill<uint32_t>(head, kEmpty, g.total_buckets, st);
-    // dry run, bottom-up: the pages every level's rebuild needs against the
-    // free pages (and those the levels below free when releasing)
+        max_buckets = std::max(max_buckets, g.buckets(L));
+    }
+    auto children = [&](int32_t L) {
+        return L < int32_t(leafl) ? ChildMap{bm[L + 1], bpos[L + 1], newaddr[L + 1], bbase[L + 1]} : ChildMap{};
+    };
+    uint32_t* dry_all = s.get<uint32_t>("gc_dry_sizes", g.total_buckets);
+    // dry run, bottom-up: every node's new address, and the pages every
+    // level's rebuild needs against the free pages (and those the levels
+    // below free when releasing)
     {
         uint32_t top[2];
         HD_CUDA(cudaMemcpyAsync(top, c->t.pool_top, 8, cudaMemcpyDeviceToHost, st));
-        uint32_t* dry_all = s.get<uint32_t>("gc_dry_sizes", g.total_buckets);
         uint32_t* full_dry = s.get<uint32_t>("gc_full_dry", HD_MAX_DEPTH);
-        uint32_t* dry_addr[2] = {s.get<uint32_t>("gc_dry_addr_a", uint64_t(maxn) + 1),
-                                 s.get<uint32_t>("gc_dry_addr_b", uint64_t(maxn) + 1)};
-        unsigned long long* cnt = s.get<unsigned long long>("gc_dry_cnt", 2);
-        uint32_t* overflow = s.get<uint32_t>("gc_dry_overflow", 1);
-        HD_CUDA(cudaMemsetAsync(overflow, 0, 4, st));
-        HD_CUDA(cudaStreamSynchronize(st));
-        int64_t avail = int64_t(g.pool_pages) - top[0] + top[1];
+        uint32_t* keys = s.get<uint32_t>("gc_keys", maxn);
+        uint32_t* rank = s.get<uint32_t>("gc_rank", maxn);
+        uint32_t* items = s.get<uint32_t>("gc_items", maxn);
+        uint32_t* counts = s.get<uint32_t>("gc_bucket_counts", max_buckets);
+        uint32_t* first = s.get<uint32_t>("gc_bucket_first", max_buckets);
+        unsigned long long* cnt = s.get<unsigned long long>("gc_dry_cnt", 2 * HD_MAX_DEPTH);
+        uint32_t* overflow = s.get<uint32_t>("gc_dry_overflow", HD_MAX_DEPTH);
+        HD_CUDA(cudaMemsetAsync(overflow, 0, HD_MAX_DEPTH * 4, st));
+        HD_CUDA(cudaMemsetAsync(cnt, 0, 2 * HD_MAX_DEPTH * 8, st));
+        HD_CUDA(cudaMemsetAsync(dry_all, 0, g.total_buckets * 4, st));
         for (int32_t L = int32_t(leafl); L >= 0; L--) {
-            const uint32_t n = nlive[L];
-            uint32_t* addr = dry_addr[L & 1];
-            const uint32_t* child_addr = dry_addr[(L + 1) & 1];
+            const uint32_t n = nlive[L], nb = g.buckets(uint32_t(L));
+            char nm[32];
+            snprintf(nm, sizeof(nm), "gc_new_%d", L);
+            newaddr[L] = s.get<uint32_t>(nm, uint64_t(n) + 1);
             uint32_t* dry_sizes = dry_all + g.level_first_bucket(uint32_t(L));
-            HD_CUDA(cudaMemsetAsync(dry_sizes, 0, uint64_t(g.buckets(uint32_t(L))) * 4, st));
-            HD_CUDA(cudaMemsetAsync(d_n, 0, 4, st));
+            HD_CUDA(cudaMemsetAsync(counts, 0, uint64_t(nb) * 4, st));
             k_gc_dry_full<<<1, 1, 0, st>>>(c->t, uint32_t(L), dry_sizes, full_dry);
             HD_LAUNCH_CHECK();
-            k_gc_gather<<<grid_for(n, 256), 256, 0, st>>>(c->t, uint32_t(L), live[L], n,
-                                                          L < int32_t(leafl) ? bm[L + 1] : nullptr,
-                                                          L < int32_t(leafl) ? bpos[L + 1] : nullptr,
-                                                          L < int32_t(leafl) ? bbase[L + 1] : 0u,
-                                                          L < int32_t(leafl) ? child_addr : nullptr, content, head,
-                                                          next, touched, d_n);
+            k_gc_keys<<<grid_for(n, 256), 256, 0, st>>>(c->t, uint32_t(L), live[L], n, children(L), keys, rank, counts);
             HD_LAUNCH_CHECK();
-            k_gc_dry_append<<<grid_for(uint64_t(n) * 32, 64, 152 * 16), 64, 0, st>>>(
-                c->t, uint32_t(L), content, head, next, touched, d_n, dry_sizes, addr, overflow);
+            exclusive_scan<uint32_t, uint32_t>(s, counts, first, nb, nullptr, st);
+            k_gc_group<<<grid_for(n, 256), 256, 0, st>>>(keys, rank, first, n, items);
             HD_LAUNCH_CHECK();
-            HD_CUDA(cudaMemsetAsync(cnt, 0, 16, st));
-            k_gc_dry_pages<<<grid_for(g.buckets(uint32_t(L)), 256), 256, 0, st>>>(
-                c->t, uint32_t(L), dry_sizes, release_pages ? 1u : 0u, cnt, cnt + 1);
+            k_gc_assign<<<grid_for(uint64_t(nb) * 32, 32 * kGcWarps, 152 * 12), 32 * kGcWarps, 0, st>>>(
+                c->t, uint32_t(L), keys, counts, first, items, dry_sizes, newaddr[L], overflow + L,
+                release_pages ? 1u : 0u, cnt + 2 * L, cnt + 2 * L + 1);
             HD_LAUNCH_CHECK();
-            unsigned long long h[2];
-            uint32_t ovf = 0;
-            HD_CUDA(cudaMemcpyAsync(h, cnt, 16, cudaMemcpyDeviceToHost, st));
-            HD_CUDA(cudaMemcpyAsync(&ovf, overflow, 4, cudaMemcpyDeviceToHost, st));
-            HD_CUDA(cudaStreamSynchronize(st));
-            if (ovf)
+        }
+        unsigned long long h[2 * HD_MAX_DEPTH];
+        uint32_t ovf[HD_MAX_DEPTH];
+        HD_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
+        HD_CUDA(cudaMemcpyAsync(ovf, overflow, sizeof(ovf), cudaMemcpyDeviceToHost, st));
+        HD_CUDA(cudaStreamSynchronize(st));
+        const uint32_t e = check_error(c); // a bucket of more than kMaxBucketItems
+        int64_t avail = int64_t(g.pool_pages) - top[0] + top[1];
+        for (int32_t L = int32_t(leafl); L >= 0; L--) {
+            if (ovf[L])
                 throw StatusError{HD_ERR_BUCKET_FULL, "GC: a rebuilt bucket of level " + std::to_string(L) +
                                                           " would exceed its capacity; the table is unchanged"};
             // releasing: the level's pages past the final sizes are freed
             // before its appends claim
-            avail += int64_t(h[1]);
-            if (int64_t(h[0]) > avail)
+            avail += int64_t(h[2 * L + 1]);
+            if (int64_t(h[2 * L]) > avail)
                 throw StatusError{HD_ERR_POOL_FULL, "GC: rebuilding level " + std::to_string(L) + " needs " +
-                                                        std::to_string(h[0]) + " new pages, " +
+                                                        std::to_string(h[2 * L]) + " new pages, " +
                                                         std::to_string(std::max<int64_t>(avail, 0)) +
                                                         " are free; the table is unchanged"};
-            avail -= int64_t(h[0]);
+            avail -= int64_t(h[2 * L]);
         }
-        const uint32_t e = check_error(c); // a bucket list over kMaxBucketItems in the dry run
         if (e)
             throw StatusError{hd_status(e), "GC: " + c->err_detail + "; the table is unchanged"};
     }
     // rebuild bottom-up
-    const uint32_t* dry_all = s.get<uint32_t>("gc_dry_sizes", g.total_buckets);
+    uint32_t* content = s.get<uint32_t>("gc_content", uint64_t(maxn) * 9);
     for (int32_t L = int32_t(leafl); L >= 0; L--) {
         const uint32_t n = nlive[L];
-        char nm[32];
-        snprintf(nm, sizeof(nm), "gc_new_%d", L);
-        newaddr[L] = s.get<uint32_t>(nm, uint64_t(n) + 1);
-        HD_CUDA(cudaMemsetAsync(d_n, 0, 4, st));
-        k_gc_gather<<<grid_for(n, 256), 256, 0, st>>>(c->t, uint32_t(L), live[L], n,
-                                                      L < int32_t(leafl) ? bm[L + 1] : nullptr,
-                                                      L < int32_t(leafl) ? bpos[L + 1] : nullptr,
-                                                      L < int32_t(leafl) ? bbase[L + 1] : 0u,
-                                                      L < int32_t(leafl) ? newaddr[L + 1] : nullptr, content, head,
-                                                      next, touched, d_n);
+        const uint32_t* dry_sizes = dry_all + g.level_first_bucket(uint32_t(L));
+        k_gc_gather<<<grid_for(n, 256), 256, 0, st>>>(c->t, uint32_t(L), live[L], n, children(L), content);
         HD_LAUNCH_CHECK();
         // empty the level's buckets and their pages' filters, then the
         // full node first
@@ -407,8 +522,7 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
             // zeroed, serve this level's appends and the levels above
             uint32_t before[2], after[2];
             HD_CUDA(cudaMemcpyAsync(before, c->t.pool_top, 8, cudaMemcpyDeviceToHost, st));
-            k_gc_release<<<grid_for(g.buckets(uint32_t(L)), 256), 256, 0, st>>>(
-                c->t, uint32_t(L), dry_all + g.level_first_bucket(uint32_t(L)));
+            k_gc_release<<<grid_for(g.buckets(uint32_t(L)), 256), 256, 0, st>>>(c->t, uint32_t(L), dry_sizes);
             HD_LAUNCH_CHECK();
             HD_CUDA(cudaMemcpyAsync(after, c->t.pool_top, 8, cudaMemcpyDeviceToHost, st));
             HD_CUDA(cudaStreamSynchronize(st));
@@ -419,7 +533,10 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
             }
         }
         add_full_nodes(c, uint32_t(L), uint32_t(L));
-        append_items(c, uint32_t(L), content, n, head, next, touched, d_n, newaddr[L]);
+        k_gc_map<<<grid_for(g.buckets(uint32_t(L)), 256), 256, 0, st>>>(c->t, uint32_t(L), dry_sizes, n);
+        HD_LAUNCH_CHECK();
+        k_gc_write<<<grid_for(n, 256), 256, 0, st>>>(c->t, uint32_t(L), content, newaddr[L], n);
+        HD_LAUNCH_CHECK();
     }
     uint32_t* d_roots = s.get<uint32_t>("gc_roots", roots.size());
     HD_CUDA(cudaMemcpyAsync(d_roots, roots.data(), roots.size() * 4, cudaMemcpyHostToDevice, st));

@@ -142,6 +142,28 @@ HD_D void link_item(uint32_t gb, uint32_t i, uint32_t* head, uint32_t* next, uin
         touched[atomicAdd(n_touched, 1u)] = gb;
 }
 
+// Warp-wide bitonic sort, ascending, of n2 (a power of two) shared words.
+HD_D void sort_shared(uint32_t* items, uint32_t n2)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t k = 2; k <= n2; k <<= 1) {
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t i = lane; i < n2; i += 32) {
+                const uint32_t ixj = i ^ j;
+                if (ixj > i) {
+                    const uint32_t a = items[i], b = items[ixj];
+                    const bool asc = (i & k) == 0;
+                    if ((a > b) == asc) {
+                        items[i] = b;
+                        items[ixj] = a;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
 // Warp-wide: gathers the items of bucket gb into `items` (shared), sorted
 // ascending, resets the list head; returns the count (0 on overflow, with
 // the error word set).
@@ -171,23 +193,7 @@ HD_D uint32_t collect_sorted(uint32_t gb, uint32_t* head, const uint32_t* next, 
     for (uint32_t i = cnt + lane; i < n2; i += 32)
         items[i] = kEmpty;
     __syncwarp();
-    // bitonic sort, ascending
-    for (uint32_t k = 2; k <= n2; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = lane; i < n2; i += 32) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const uint32_t a = items[i], b = items[ixj];
-                    const bool asc = (i & k) == 0;
-                    if ((a > b) == asc) {
-                        items[i] = b;
-                        items[ixj] = a;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
+    sort_shared(items, n2);
     return cnt;
 }
 
