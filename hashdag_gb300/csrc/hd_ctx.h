@@ -47,6 +47,10 @@ struct hd_ctx {
     hd_batch_tuning tuning{4, 4, 304, HD_BATCH_PERSISTENT};
     hd::BatchGraph* batch = nullptr;
     uint64_t batch_fallbacks = 0;
+    // launch shape of the persistent edit kernel per probe width (grid 0: it
+    // does not fit)
+    bool persist_known[3] = {false, false, false};
+    uint32_t persist_grid[3] = {0, 0, 0};
     uint32_t batch_applied = 0; // edits of the last batch call that were applied (also when it failed)
     // colours: the table, host mirror of its counters
     bool colors = false;

@@ -772,4 +772,27 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
     return !failed;
 }
 
+// ---- the persistent launch (hd_edit_persist.cu) and its buffers (hd_edit_batch.cu)
+// Level arrays sized by upper bounds of their entries, and the sort's arrays.
+struct PersistLevels {
+    std::vector<Level> lv;
+    std::vector<uint32_t> caps;
+    uint32_t *keys, *vals, *keys2, *vals2;
+};
+// The geometry of one edit as the persistent launch leaves it.
+struct EditGeometry {
+    EditCounters ctr;
+    uint32_t root, deepest;
+    std::vector<uint32_t> count; // entries per level (0 below the deepest)
+};
+// Buffers for one edit, or null when its levels may hold more entries than
+// the persistent launch is used for.
+const PersistLevels* one_edit_levels(hd_ctx* c, const Editor& ed);
+// Runs one edit's geometry in one persistent launch; false when it does not
+// apply (a level outgrew its bound, or the kernel does not fit on an SM): the
+// table is then untouched.  hold_root: the root is left for the caller to set.
+bool edit_geometry_persistent(hd_ctx* c, const Editor& ed, const PersistLevels& pl, bool hold_root, EditGeometry& out);
+// One edit, level by level from the host (hd_edit.cu).
+void edit_by_levels(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats);
+
 } // namespace hd

@@ -27,9 +27,7 @@ namespace hd {
 
 void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats); // hd_edit.cu
 // hd_edit_persist.cu
-void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const std::vector<Level>& lv,
-                           const std::vector<uint32_t>& caps, uint32_t* keys, uint32_t* vals, uint32_t* keys2,
-                           uint32_t* vals2, hd_edit* d_edits, EditCounters* d_ctr, uint32_t* d_roots,
+void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const PersistLevels& pl, hd_edit* d_edits,
                            std::vector<EditCounters>& ctr, std::vector<float>& dur_ms, std::vector<float>& end_ms,
                            float& device_ms, uint64_t& fallbacks);
 
@@ -380,25 +378,29 @@ __global__ void k_b_finish(BatchState* bs, const Level lv0, uint32_t* d_root, ui
 // Upper bound of the entries of every level for one edit: 8 per descended
 // entry of the level above.  Above C_colorTreeLevels every node the tool's
 // box overlaps descends; below, only nodes that cross the tool's surface,
-// which lie within 2 node sizes of it.
-static void edit_caps(const Geom& g, const hd_edit& e, std::vector<uint64_t>& cap)
+// which lie within 2 node sizes of it (every node the box overlaps for the
+// tools without is_full / is_empty).
+static void edit_caps(const Geom& g, const Editor& e, std::vector<uint64_t>& cap)
 {
     const uint32_t D = g.depth, leafl = g.leaf_level;
-    const double r = double(e.radius) + 1.0;
-    const bool sphere = e.tool == HD_TOOL_SPHERE_ADD || e.tool == HD_TOOL_SPHERE_REMOVE;
+    const double r = double(e.r) + 1.0;
+    // a voxel beyond the tool's box on either side
+    const double bmin[3] = {e.bminx - 1.0, e.bminy - 1.0, e.bminz - 1.0};
+    const double bmax[3] = {e.bmaxx + 1.0, e.bmaxy + 1.0, e.bmaxz + 1.0};
+    const bool sphere = e.sphere();
     cap[0] = std::max<uint64_t>(cap[0], 1);
     for (uint32_t L = 0; L < leafl; L++) {
         const double s = std::ldexp(1.0, int(D - L));
         const double side = std::ldexp(1.0, int(L));
         double box = 1.0;
         for (int a = 0; a < 3; a++) {
-            double lo = std::floor((double(e.center[a]) - r) / s), hi = std::floor((double(e.center[a]) + r) / s);
+            double lo = std::floor(bmin[a] / s), hi = std::floor(bmax[a] / s);
             lo = std::max(lo, 0.0);
             hi = std::min(hi, side - 1.0);
             box *= std::max(0.0, hi - lo + 1.0);
         }
         double desc = std::min(box, side * side * side);
-        if (L >= g.T) {
+        if (L >= g.T && e.shortcuts()) {
             double shell;
             if (sphere) {
                 const double ro = r + 2.0 * s, ri = std::max(0.0, r - 2.0 * s);
@@ -413,7 +415,28 @@ static void edit_caps(const Geom& g, const hd_edit& e, std::vector<uint64_t>& ca
     }
 }
 
+struct BatchBuffers : PersistLevels {
+    uint32_t *bsum, *hist, *rows, *roots;
+    hd_edit* edits;
+    EditCounters* ctr;
+    BatchState* bs;
+    uint32_t edit_cap;
+    std::vector<void*> ptrs() const
+    {
+        std::vector<void*> p{keys, vals, keys2, vals2, bsum, hist, rows, roots, edits, ctr, bs};
+        for (const Level& l : lv)
+            p.insert(p.end(), {l.x, l.y, l.z, l.old, l.state, l.res, l.cnt, l.flag, l.exp, l.leaf, l.cand});
+        return p;
+    }
+};
+
 struct BatchGraph {
+    // the buffers of the last call, while the scratch buffers stay where they
+    // are and fit
+    BatchBuffers buffers{};
+    uint64_t epoch = 0;
+    bool colors = false, have = false;
+    uint32_t blocks = 0;
     cudaGraphExec_t exec = nullptr;
     std::vector<void*> ptrs; // buffers the graph was captured with
     hd_batch_tuning tuning{};
@@ -429,24 +452,7 @@ struct BatchGraph {
     }
 };
 
-struct BatchBuffers {
-    std::vector<Level> lv;
-    std::vector<uint32_t> caps;
-    uint32_t *keys, *vals, *keys2, *vals2, *bsum, *hist, *rows, *roots;
-    hd_edit* edits;
-    EditCounters* ctr;
-    BatchState* bs;
-    uint32_t edit_cap;
-    std::vector<void*> ptrs() const
-    {
-        std::vector<void*> p{keys, vals, keys2, vals2, bsum, hist, rows, roots, edits, ctr, bs};
-        for (const Level& l : lv)
-            p.insert(p.end(), {l.x, l.y, l.z, l.old, l.state, l.res, l.cnt, l.flag, l.exp, l.leaf, l.cand});
-        return p;
-    }
-};
-
-static Level batch_level(Scratch& s, uint32_t L, uint64_t n, bool leaf)
+static Level batch_level(Scratch& s, uint32_t L, uint64_t n, bool leaf, bool colors)
 {
     char nm[48];
     auto buf = [&](const char* what, size_t bytes) {
@@ -465,6 +471,13 @@ static Level batch_level(Scratch& s, uint32_t L, uint64_t n, bool leaf)
     l.exp = static_cast<uint32_t*>(buf("exp", n * 4));
     l.leaf = leaf ? static_cast<uint64_t*>(buf("leaf", n * 8)) : nullptr;
     l.cand = static_cast<uint32_t*>(buf("cand", n * 36));
+    if (colors) {
+        l.ocnt = static_cast<uint32_t*>(buf("ocnt", n * 4));
+        l.cn = static_cast<uint32_t*>(buf("cn", n * 4));
+        l.noff = static_cast<uint32_t*>(buf("noff", n * 4));
+        l.ooff = static_cast<uint32_t*>(buf("ooff", n * 4));
+        l.task = static_cast<uint32_t*>(buf("task", n * 4));
+    }
     return l;
 }
 
@@ -484,7 +497,7 @@ static BatchBuffers batch_buffers(hd_ctx* c, const std::vector<uint64_t>& cap64,
     }
     b.lv.resize(levels);
     for (uint32_t L = 0; L < levels; L++)
-        b.lv[L] = batch_level(s, L, b.caps[L], L == g.leaf_level);
+        b.lv[L] = batch_level(s, L, b.caps[L], L == g.leaf_level, c->colors);
     b.keys = s.get<uint32_t>("eb_keys", maxn);
     b.vals = s.get<uint32_t>("eb_vals", maxn);
     b.keys2 = s.get<uint32_t>("eb_keys2", maxn);
@@ -500,6 +513,51 @@ static BatchBuffers batch_buffers(hd_ctx* c, const std::vector<uint64_t>& cap64,
     b.ctr = s.get<EditCounters>("eb_ctr", b.edit_cap);
     b.bs = s.get<BatchState>("eb_state", 1);
     return b;
+}
+
+// The buffers for level bounds `cap` and n edits.  Capacities only grow
+// (powers of two), so that one graph serves many batches; the graph's edit
+// count is the edits buffer's capacity.
+static const BatchBuffers& batch_levels(hd_ctx* c, std::vector<uint64_t>& cap, uint32_t n)
+{
+    if (!c->batch)
+        c->batch = new BatchGraph();
+    BatchGraph& bg = *c->batch;
+    bool fits = bg.have && bg.epoch == c->scratch.epoch() && bg.colors == c->colors &&
+                bg.blocks == c->tuning.grid_blocks && n <= bg.buffers.edit_cap;
+    for (size_t L = 0; L < cap.size(); L++) {
+        const uint64_t had = bg.have ? bg.buffers.caps[L] : 0;
+        fits = fits && cap[L] <= had;
+        uint64_t v = 256;
+        while (v < cap[L])
+            v <<= 1;
+        cap[L] = std::max(v, had);
+    }
+    if (!fits) {
+        bg.have = false;
+        bg.buffers = batch_buffers(c, cap, std::max<uint32_t>(n, bg.edit_cap));
+        bg.epoch = c->scratch.epoch();
+        bg.colors = c->colors;
+        bg.blocks = c->tuning.grid_blocks;
+        bg.have = true;
+    }
+    return bg.buffers;
+}
+
+// The persistent launch takes an edit whose levels hold at most this many
+// entries each (about 350 MB of level arrays); beyond, the level-by-level
+// path's arrays, sized by the entries there are, and its kernels over all of
+// them serve as well.
+constexpr uint64_t kOneEditEntries = 1ull << 22;
+
+const PersistLevels* one_edit_levels(hd_ctx* c, const Editor& ed)
+{
+    std::vector<uint64_t> cap(c->g.leaf_level + 1, 0);
+    edit_caps(c->g, ed, cap);
+    for (uint64_t n : cap)
+        if (n > kOneEditEntries)
+            return nullptr;
+    return &batch_levels(c, cap, 1);
 }
 
 constexpr uint32_t kFoaBatchWarps = 152 * 32;
@@ -642,21 +700,11 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
             *total = sum;
         return;
     }
-    if (!c->batch)
-        c->batch = new BatchGraph();
-    BatchGraph& bg = *c->batch;
     std::vector<uint64_t> cap(c->g.leaf_level + 1, 0);
     for (uint32_t i = 0; i < n; i++)
-        edit_caps(c->g, edits[i], cap);
-    // capacities only grow (powers of two), so that one graph serves many
-    // batches; the graph's edit count is the edits buffer's capacity
-    for (size_t L = 0; L < cap.size(); L++) {
-        uint64_t v = 256;
-        while (v < cap[L])
-            v <<= 1;
-        cap[L] = std::max<uint64_t>(v, L < bg.caps.size() ? bg.caps[L] : 0);
-    }
-    const BatchBuffers b = batch_buffers(c, cap, std::max<uint32_t>(n, bg.edit_cap));
+        edit_caps(c->g, make_editor(edits[i]), cap);
+    const BatchBuffers& b = batch_levels(c, cap, n);
+    BatchGraph& bg = *c->batch;
     if (c->tuning.mode == HD_BATCH_PERSISTENT) {
         std::vector<EditCounters> ctr(n);
         std::vector<float> end_ms(n, 0.0f), dur_ms(n, 0.0f);
@@ -664,8 +712,7 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
         bool failed = false;
         StatusError failure{HD_OK, ""};
         try {
-            edit_batch_persistent(c, edits, n, b.lv, b.caps, b.keys, b.vals, b.keys2, b.vals2, b.edits, b.ctr,
-                                  b.roots, ctr, dur_ms, end_ms, device_ms, c->batch_fallbacks);
+            edit_batch_persistent(c, edits, n, b, b.edits, ctr, dur_ms, end_ms, device_ms, c->batch_fallbacks);
         } catch (const StatusError& e) {
             failed = true;
             failure = e;
@@ -760,7 +807,7 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
         // capacity: this edit with the one-edit path, then resume
         c->root = read_scalar(c->d_root, st);
         hd_edit_stats s{};
-        edit_one(c, edits[done], &s);
+        edit_by_levels(c, edits[done], &s);
         ctr[done].num_voxels = s.num_voxels;
         ctr[done].num_nodes = s.num_nodes;
         ctr[done].foa = s.find_or_add_calls;

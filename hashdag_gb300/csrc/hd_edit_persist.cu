@@ -28,6 +28,7 @@
 //  * Nodes and pages that an edit appends are read by the following edits in
 //    the same launch: every table read uses L2-coherent loads.
 // The graph-per-edit form (hd_edit_batch.cu) stays as the other batch mode.
+#include <cstring>
 #include <vector>
 
 #include "hd_edit.cuh"
@@ -76,19 +77,27 @@ struct Ctl {
     Editor ed;
 };
 
+// What one edit of the launch gives back.
+struct EditOut {
+    EditCounters ctr;
+    uint32_t root, pad;
+    unsigned long long t_begin, t_end;
+};
+
+// The launch's arguments, read where they are needed (a __grid_constant__
+// parameter: the level arrays' pointers come from the constant bank).
 struct PArgs {
     Ctl* ctl;
-    const hd_edit* edits;
+    const hd_edit* edits; // the batch, or null: the one edit `one`
     uint32_t n_edits;
-    const Level* lv;     // device array: one Level per depth
+    uint32_t hold_root;   // the new root goes to the edit's EditOut only (its colours come first)
+    Editor one;
+    Level lv[HD_MAX_DEPTH];
     uint32_t cap[HD_MAX_DEPTH];
     uint32_t *keys, *vals, *keys2, *vals2;
     uint32_t* bsum;      // 3 x G: per-chunk descend-flag counts, by level parity
     uint32_t *hist, *hist2, *rows, *rows2; // kDigits x G, kDigits
-    EditCounters* ctr;
-    uint32_t* roots;
-    unsigned long long* t_begin;
-    unsigned long long* t_end;
+    EditOut* out;
     uint32_t* d_root;
 };
 
@@ -626,8 +635,7 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
             stop = kDone;
         ctl->stop = stop;
         if (stop == kRun) {
-            a.t_begin[idx] = now_ns();
-            *sm.ed = make_editor(a.edits[idx]);
+            *sm.ed = a.edits ? make_editor(a.edits[idx]) : a.one;
             ctl->ed = *sm.ed;
             for (uint32_t L = 0; L < HD_MAX_DEPTH; L++)
                 ctl->count[L] = 0;
@@ -637,7 +645,8 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
             l0.y[0] = 0;
             l0.z[0] = 0;
             l0.old[0] = __ldcg(a.d_root);
-            a.ctr[idx] = EditCounters{};
+            a.out[idx].ctr = EditCounters{};
+            a.out[idx].t_begin = now_ns();
         }
         sm.sm32[32] = stop;
     }
@@ -649,7 +658,7 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
     if (threadIdx.x == 0) {
         unsigned long long nn, vv;
         classify_entry<true>(t, *sm.ed, 0, a.lv[0], 0, nn, vv);
-        EditCounters* ctr = a.ctr + ctl->idx;
+        EditCounters* ctr = &a.out[ctl->idx].ctr;
         atomicAdd(&ctr->num_nodes, nn);
         atomicAdd(&ctr->num_voxels, vv);
     }
@@ -670,10 +679,11 @@ HD_D void finish_edit(const Table& t, const PArgs& a)
             if (r == kInvalid || r == kNotFound) {
                 ctl->stop = kEmptyScene;
             } else {
-                *a.d_root = r;
-                a.roots[idx] = r;
+                if (!a.hold_root)
+                    *a.d_root = r;
+                a.out[idx].root = r;
                 __threadfence();
-                a.t_end[idx] = now_ns();
+                a.out[idx].t_end = now_ns();
                 ctl->idx = idx + 1;
             }
         }
@@ -706,8 +716,7 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
             L = 0;
             ls = kLsTopDown;
         }
-        const uint32_t idx = ctl->idx;
-        EditCounters* ctr = a.ctr + idx;
+        EditCounters* ctr = &a.out[ctl->idx].ctr;
         if (ls == kLsTopDown) {
             __shared__ uint32_t tiny[2];
             while (L < leafl) {
@@ -816,7 +825,8 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
 }
 
 template <int PW>
-__global__ void __launch_bounds__(kPT, 1) k_edit_persistent(Table t, PArgs a)
+__global__ void __launch_bounds__(kPT, 1)
+    k_edit_persistent(__grid_constant__ const Table t, __grid_constant__ const PArgs a)
 {
     {
         const uint32_t skip = __ldcg(&a.ctl->skip_cta);
@@ -875,8 +885,7 @@ __global__ void __launch_bounds__(kPT, 1) k_edit_persistent(Table t, PArgs a)
         }
         L = cmd.level;
         uint32_t deepest = cmd.deepest;
-        const uint32_t idx = cmd.idx;
-        EditCounters* ctr = a.ctr + idx;
+        EditCounters* ctr = &a.out[cmd.idx].ctr;
         if (threadIdx.x == 0) {
             const uint32_t* src = reinterpret_cast<const uint32_t*>(&ctl->ed);
             uint32_t* dst = reinterpret_cast<uint32_t*>(&ed_s);
@@ -1009,13 +1018,6 @@ __global__ void __launch_bounds__(kPT, 1) k_edit_persistent(Table t, PArgs a)
 
 // ---- host side --------------------------------------------------------------------
 
-struct PersistBuffers {
-    Ctl* ctl = nullptr;
-    Level* d_lv = nullptr;
-    size_t smem = 0;
-    uint32_t grid = 0;
-};
-
 static size_t persist_smem() { return persist_smem_core() + size_t(kPT) * 4 * 2; }
 
 template <int PW>
@@ -1024,115 +1026,134 @@ static const void* persist_kernel()
     return reinterpret_cast<const void*>(k_edit_persistent<PW>);
 }
 
+namespace {
+
+// The launch shape of a context, found once: one CTA per SM.
+struct PersistShape {
+    const void* kern;
+    uint32_t grid; // 0: the kernel does not fit on an SM
+};
+
+PersistShape persist_shape(hd_ctx* c)
+{
+    const uint32_t pw = c->tuning.probe_words == 4 ? 2 : c->tuning.probe_words == 2 ? 1 : 0;
+    const void* kern = pw == 2 ? persist_kernel<4>() : pw == 1 ? persist_kernel<2>() : persist_kernel<1>();
+    if (!c->persist_known[pw]) {
+        int dev = 0, sms = 0, per_sm = 0;
+        HD_CUDA(cudaGetDevice(&dev));
+        HD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        HD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(persist_smem())));
+        HD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPT, persist_smem()));
+        c->persist_grid[pw] = per_sm < 1 ? 0u : uint32_t(sms);
+        c->persist_known[pw] = true;
+    }
+    return {kern, c->persist_grid[pw]};
+}
+
+// Device buffers of a launch of at most n edits; ctl and out lie in one
+// buffer, so that one copy brings the results back.
+PArgs persist_args(hd_ctx* c, const PersistLevels& pl, uint32_t grid, uint32_t n)
+{
+    Scratch& s = c->scratch;
+    PArgs a{};
+    a.ctl = reinterpret_cast<Ctl*>(s.get<unsigned char>("ep_ctl", sizeof(Ctl) + sizeof(EditOut) * n));
+    a.out = reinterpret_cast<EditOut*>(a.ctl + 1);
+    for (uint32_t L = 0; L <= c->g.leaf_level; L++) {
+        a.lv[L] = pl.lv[L];
+        a.cap[L] = pl.caps[L];
+    }
+    a.keys = pl.keys;
+    a.vals = pl.vals;
+    a.keys2 = pl.keys2;
+    a.vals2 = pl.vals2;
+    a.bsum = s.get<uint32_t>("ep_bsum", 3ull * grid);
+    a.hist = s.get<uint32_t>("ep_hist", uint64_t(kDigits) * grid);
+    a.hist2 = s.get<uint32_t>("ep_hist2", uint64_t(kDigits) * grid);
+    a.rows = s.get<uint32_t>("ep_rows", kDigits);
+    a.rows2 = s.get<uint32_t>("ep_rows2", kDigits);
+    a.d_root = c->d_root;
+    return a;
+}
+static_assert(sizeof(Ctl) % alignof(EditOut) == 0, "EditOut follows Ctl");
+
+void persist_launch(hd_ctx* c, const PersistShape& shape, PArgs& a)
+{
+    void* args[] = {&c->t, &a};
+    HD_CUDA(cudaLaunchCooperativeKernel(shape.kern, dim3(shape.grid), dim3(kPT), args, persist_smem(), c->stream));
+}
+
+[[noreturn]] void persist_timeout(hd_ctx* c, const Ctl& fin, uint32_t edit)
+{
+    check_error(c);
+    c->root = read_scalar(c->d_root, c->stream);
+    std::string where;
+    for (uint32_t k = 0; k < 8; k++)
+        where += (k ? " " : "") + std::to_string(fin.diag[k]);
+    throw StatusError{HD_ERR_TIMEOUT, "edit " + std::to_string(edit) +
+                                          ": a grid barrier of the persistent edit kernel ran out of time "
+                                          "(cta, barriers, arrivals, arrivals awaited, cta0 barriers, phase, level, edit: " +
+                                          where + ")"};
+}
+
+} // namespace
+
 // Applies edits[0..n) in one persistent launch per stretch of the batch (a
 // level that would outgrow its bound ends the stretch: that edit takes the
 // one-edit path and the next stretch starts after it).
-void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const std::vector<Level>& lv,
-                           const std::vector<uint32_t>& caps, uint32_t* keys, uint32_t* vals, uint32_t* keys2,
-                           uint32_t* vals2, hd_edit* d_edits, EditCounters* d_ctr, uint32_t* d_roots,
+void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const PersistLevels& pl, hd_edit* d_edits,
                            std::vector<EditCounters>& ctr, std::vector<float>& dur_ms, std::vector<float>& end_ms,
                            float& device_ms, uint64_t& fallbacks)
 {
     cudaStream_t st = c->stream;
-    Scratch& s = c->scratch;
-    const uint32_t levels = c->g.leaf_level + 1;
-    int dev = 0, sms = 0;
-    HD_CUDA(cudaGetDevice(&dev));
-    HD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const size_t smem = persist_smem();
-    const void* kern = c->tuning.probe_words == 4   ? persist_kernel<4>()
-                       : c->tuning.probe_words == 2 ? persist_kernel<2>()
-                                                    : persist_kernel<1>();
-    HD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int per_sm = 0;
-    HD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPT, smem));
-    if (per_sm < 1)
+    const PersistShape shape = persist_shape(c);
+    if (!shape.grid)
         throw StatusError{HD_ERR_STATE, "the persistent edit kernel does not fit on an SM"};
-    const uint32_t G = uint32_t(sms); // one CTA per SM
-    Ctl* ctl = s.get<Ctl>("ep_ctl", 1);
-    Level* d_lv = s.get<Level>("ep_lv", HD_MAX_DEPTH);
-    HD_CUDA(cudaMemcpyAsync(d_lv, lv.data(), sizeof(Level) * levels, cudaMemcpyHostToDevice, st));
-    PArgs a{};
-    a.ctl = ctl;
-    a.lv = d_lv;
-    for (uint32_t L = 0; L < levels; L++)
-        a.cap[L] = caps[L];
-    a.keys = keys;
-    a.vals = vals;
-    a.keys2 = keys2;
-    a.vals2 = vals2;
-    a.bsum = s.get<uint32_t>("ep_bsum", 3ull * G);
-    a.hist = s.get<uint32_t>("ep_hist", uint64_t(kDigits) * G);
-    a.hist2 = s.get<uint32_t>("ep_hist2", uint64_t(kDigits) * G);
-    a.rows = s.get<uint32_t>("ep_rows", kDigits);
-    a.rows2 = s.get<uint32_t>("ep_rows2", kDigits);
-    a.ctr = d_ctr;
-    a.roots = d_roots;
-    a.t_begin = s.get<unsigned long long>("ep_tbegin", n + 1);
-    a.t_end = s.get<unsigned long long>("ep_tend", n + 1);
-    a.d_root = c->d_root;
-    std::vector<unsigned long long> tb(n), te(n);
+    PArgs a = persist_args(c, pl, shape.grid, n);
+    std::vector<unsigned char> back(sizeof(Ctl) + sizeof(EditOut) * n);
     uint32_t done = 0;
     c->batch_applied = 0;
     float elapsed_before = 0.0f;
-    unsigned long long first_ns = 0;
     while (done < n) {
         const uint32_t m = n - done;
         a.edits = d_edits;
         a.n_edits = m;
         HD_CUDA(cudaMemcpyAsync(d_edits, edits + done, sizeof(hd_edit) * m, cudaMemcpyHostToDevice, st));
-        HD_CUDA(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
+        HD_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(Ctl), st));
         if (c->test_skip_cta) {
             // one launch only: the hook switches itself off
             const uint32_t skip = c->test_skip_cta;
             const unsigned long long wait = c->test_wait_ns;
-            HD_CUDA(cudaMemcpyAsync(&ctl->skip_cta, &skip, 4, cudaMemcpyHostToDevice, st));
-            HD_CUDA(cudaMemcpyAsync(&ctl->wait_ns, &wait, 8, cudaMemcpyHostToDevice, st));
+            HD_CUDA(cudaMemcpyAsync(&a.ctl->skip_cta, &skip, 4, cudaMemcpyHostToDevice, st));
+            HD_CUDA(cudaMemcpyAsync(&a.ctl->wait_ns, &wait, 8, cudaMemcpyHostToDevice, st));
             HD_CUDA(cudaStreamSynchronize(st));
             c->test_skip_cta = 0;
             c->test_wait_ns = 0;
         }
         HD_CUDA(cudaEventRecord(c->ev0, st));
-        void* args[] = {&c->t, &a};
-        HD_CUDA(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(kPT), args, smem, st));
+        persist_launch(c, shape, a);
         HD_CUDA(cudaEventRecord(c->ev1, st));
-        Ctl fin{};
-        HD_CUDA(cudaMemcpyAsync(&fin, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+        HD_CUDA(cudaMemcpyAsync(back.data(), a.ctl, sizeof(Ctl) + sizeof(EditOut) * m, cudaMemcpyDeviceToHost, st));
         HD_CUDA(cudaStreamSynchronize(st));
+        Ctl fin;
+        std::memcpy(&fin, back.data(), sizeof(Ctl));
+        const EditOut* out = reinterpret_cast<const EditOut*>(back.data() + sizeof(Ctl));
         float launch_ms = 0;
         HD_CUDA(cudaEventElapsedTime(&launch_ms, c->ev0, c->ev1));
         const uint32_t ok = fin.idx;
-        if (ok) {
-            HD_CUDA(cudaMemcpy(ctr.data() + done, d_ctr, sizeof(EditCounters) * ok, cudaMemcpyDeviceToHost));
-            std::vector<uint32_t> roots(ok);
-            HD_CUDA(cudaMemcpy(roots.data(), d_roots, 4ull * ok, cudaMemcpyDeviceToHost));
-            HD_CUDA(cudaMemcpy(tb.data() + done, a.t_begin, 8ull * ok, cudaMemcpyDeviceToHost));
-            HD_CUDA(cudaMemcpy(te.data() + done, a.t_end, 8ull * ok, cudaMemcpyDeviceToHost));
-            if (!first_ns)
-                first_ns = tb[done];
-            for (uint32_t k = 0; k < ok; k++) {
-                UndoFrame f;
-                f.root = c->root;
-                push_undo(c, std::move(f));
-                c->root = roots[k];
-                dur_ms[done + k] = float(double(te[done + k] - tb[done + k]) * 1e-6);
-                end_ms[done + k] = elapsed_before + float(double(te[done + k] - tb[done]) * 1e-6);
-            }
+        for (uint32_t k = 0; k < ok; k++) {
+            UndoFrame f;
+            f.root = c->root;
+            push_undo(c, std::move(f));
+            c->root = out[k].root;
+            ctr[done + k] = out[k].ctr;
+            dur_ms[done + k] = float(double(out[k].t_end - out[k].t_begin) * 1e-6);
+            end_ms[done + k] = elapsed_before + float(double(out[k].t_end - out[0].t_begin) * 1e-6);
         }
         elapsed_before += launch_ms;
         done += ok;
         c->batch_applied = done;
-        if (fin.abort) {
-            check_error(c);
-            c->root = read_scalar(c->d_root, st);
-            std::string where;
-            for (uint32_t k = 0; k < 8; k++)
-                where += (k ? " " : "") + std::to_string(fin.diag[k]);
-            throw StatusError{HD_ERR_TIMEOUT, "edit " + std::to_string(done) +
-                                                  ": a grid barrier of the persistent edit kernel ran out of time "
-                                                  "(cta, barriers, arrivals, arrivals awaited, cta0 barriers, phase, level, edit: " +
-                                                  where + ")"};
-        }
+        if (fin.abort)
+            persist_timeout(c, fin, done);
         if (fin.stop == kDone)
             break;
         if (fin.stop == kTableError || fin.stop == kEmptyScene) {
@@ -1143,10 +1164,10 @@ void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const st
             throw StatusError{hd_status(err ? err : HD_ERR_CUDA),
                               "edit " + std::to_string(done) + " failed on the device (" + c->err_detail + ")"};
         }
-        // capacity: this edit with the one-edit path, then resume
+        // capacity: this edit with the level-by-level path, then resume
         c->root = read_scalar(c->d_root, st);
         hd_edit_stats es{};
-        edit_one(c, edits[done], &es);
+        edit_by_levels(c, edits[done], &es);
         ctr[done].num_voxels = es.num_voxels;
         ctr[done].num_nodes = es.num_nodes;
         ctr[done].foa = es.find_or_add_calls;
@@ -1160,6 +1181,44 @@ void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const st
         fallbacks++;
     }
     device_ms = elapsed_before;
+}
+
+bool edit_geometry_persistent(hd_ctx* c, const Editor& ed, const PersistLevels& pl, bool hold_root, EditGeometry& out)
+{
+    cudaStream_t st = c->stream;
+    const PersistShape shape = persist_shape(c);
+    if (!shape.grid)
+        return false;
+    PArgs a = persist_args(c, pl, shape.grid, 1);
+    a.n_edits = 1;
+    a.hold_root = hold_root;
+    a.one = ed;
+    HD_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(Ctl), st));
+    persist_launch(c, shape, a);
+    if (!hold_root)
+        HD_CUDA(cudaEventRecord(c->ev1, st)); // with colours the edit goes on
+    struct {
+        Ctl ctl;
+        EditOut edit;
+    } back;
+    HD_CUDA(cudaMemcpyAsync(&back, a.ctl, sizeof(back), cudaMemcpyDeviceToHost, st));
+    HD_CUDA(cudaStreamSynchronize(st));
+    const Ctl& fin = back.ctl;
+    if (fin.abort)
+        persist_timeout(c, fin, 0);
+    if (fin.stop == kCapacity)
+        return false;
+    if (fin.stop == kEmptyScene)
+        throw StatusError{HD_ERR_STATE, "edit would empty the whole scene"};
+    if (fin.idx != 1) {
+        const uint32_t err = check_error(c);
+        throw StatusError{hd_status(err ? err : HD_ERR_CUDA), "edit failed on the device (" + c->err_detail + ")"};
+    }
+    out.ctr = back.edit.ctr;
+    out.root = back.edit.root;
+    out.deepest = fin.deepest;
+    out.count.assign(fin.count, fin.count + c->g.leaf_level + 1);
+    return true;
 }
 
 } // namespace hd

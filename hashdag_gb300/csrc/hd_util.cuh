@@ -45,6 +45,7 @@ public:
                 cudaFree(b.ptr);
             b.ptr = nullptr;
             b.bytes = 0;
+            epoch_++;
             size_t want = bytes + bytes / 4 + 256;
             if (cudaMalloc(&b.ptr, want) != cudaSuccess) {
                 cudaGetLastError();
@@ -70,7 +71,11 @@ public:
         if (it->second.ptr)
             cudaFree(it->second.ptr);
         bufs_.erase(it);
+        epoch_++;
     }
+    // changes whenever a buffer moves or goes: pointers kept from get() hold
+    // while it stays
+    uint64_t epoch() const { return epoch_; }
     size_t peak() const { return peak_; }
     void note_peak()
     {
@@ -83,6 +88,7 @@ public:
             if (kv.second.ptr)
                 cudaFree(kv.second.ptr);
         bufs_.clear();
+        epoch_++;
     }
     size_t total() const
     {
@@ -99,6 +105,7 @@ private:
     };
     std::unordered_map<std::string, Buf> bufs_;
     size_t peak_ = 0;
+    uint64_t epoch_ = 0;
 };
 
 // ----------------------------------------------------------------- scan ---
