@@ -94,7 +94,7 @@ hd_status hd_create(const hd_config* cfg, hd_ctx** out)
         // 64 bytes past the last page: a node read at its physical offset
         // stays inside the allocation even in a corrupt table
         HD_CUDA(cudaMalloc(&t.pool, size_t(conf.pool_pages) * HD_PAGE_SIZE * 4 + 64));
-        HD_CUDA(cudaMalloc(&t.bloom, size_t(conf.pool_pages) * kBloomWords * 4));
+        HD_CUDA(cudaMalloc(&t.meta, size_t(conf.pool_pages) * kPageMeta * 4));
         HD_CUDA(cudaMalloc(&t.page_table, kPageTableEntries * 4));
         HD_CUDA(cudaMalloc(&t.bucket_sizes, c->g.total_buckets * 4));
         HD_CUDA(cudaMalloc(&t.full_nodes, HD_MAX_DEPTH * 4));
@@ -136,7 +136,7 @@ hd_status hd_destroy(hd_ctx* c)
         cudaFree(c->t.page_ids);
     }
     cudaFree(c->t.pool);
-    cudaFree(c->t.bloom);
+    cudaFree(c->t.meta);
     cudaFree(c->t.page_table);
     cudaFree(c->t.bucket_sizes);
     cudaFree(c->t.full_nodes);
@@ -525,7 +525,7 @@ hd_status hd_memory_stats(hd_ctx* c, uint64_t* out)
     if (!c || !out)
         return HD_ERR_INVALID;
     out[0] = uint64_t(c->cfg.pool_pages) * HD_PAGE_SIZE * 4 + kPageTableEntries * 4 + c->g.total_buckets * 4 +
-             uint64_t(c->cfg.pool_pages) * kBloomWords * 4 + (c->t.direct ? c->g.total_vpages * 4 : 0);
+             uint64_t(c->cfg.pool_pages) * kPageMeta * 4 + (c->t.direct ? c->g.total_vpages * 4 : 0);
     const ColorTable& ct = c->ct;
     out[1] = ct.cap_nodes * 4 + ct.cap_leaves * sizeof(LeafDesc) + ct.cap_blocks * 8 + ct.cap_macros * 8 +
              ct.cap_weights * 4;

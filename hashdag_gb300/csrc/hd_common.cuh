@@ -97,7 +97,7 @@ inline Geom make_geom(const hd_config& c)
 // reference's tracer does, tracer.cu:146).
 struct Table {
     uint32_t* pool;
-    uint32_t* bloom;        // kBloomWords per physical page (see bloom_*)
+    uint32_t* meta;         // kPageMeta words per physical page (see bloom_*)
     uint32_t* page_table;
     uint32_t* bucket_sizes;
     uint32_t* full_nodes;   // [depth]
@@ -209,6 +209,26 @@ HD_HD uint32_t hash_interior(uint32_t n, const uint32_t* node)
     return murmur32(h);
 }
 
+// hash_interior of a row of 9 words (n of them used), unrolled: the words
+// stay in registers.
+HD_HD uint32_t hash_interior_words(uint32_t n, const uint32_t (&node)[9])
+{
+    uint32_t h = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 9; ++i) {
+        uint32_t k = node[i];
+        k *= 0xcc9e2d51u;
+        k = (k << 15) | (k >> 17);
+        k *= 0x1b873593u;
+        uint32_t g = h ^ k;
+        g = (g << 13) | (g >> 19);
+        g = g * 5u + 0xe6546b64u;
+        h = i < n ? g : h;
+    }
+    h ^= n;
+    return murmur32(h);
+}
+
 HD_HD uint32_t popc32(uint32_t v)
 {
 #ifdef __CUDA_ARCH__
@@ -237,23 +257,38 @@ HD_HD uint64_t mix64(uint64_t z)
 }
 
 // ---- per-page Bloom filters (hash_table.h:564-659, USE_BLOOM_FILTER) --------
-// Every physical page has a 512-bit filter holding 3 bits of every node
-// ever written into it; a bucket scan skips a page whose filter lacks a bit
-// of the node it looks for.  The filter can only say "maybe": a page that
-// holds the node always passes, so results never change, only the pages
-// read.  Bits come from a hash of the node's words independent of the
-// bucket hash.
-constexpr uint32_t kBloomWords = 16;
+// Every physical page has a 128-byte line that bucket scans read before the
+// page itself.
+//  * A filter holding 3 bits of every node ever written into the page: a scan
+//    skips a page whose filter lacks a bit of the node it looks for.  It can
+//    only say "maybe": a page that holds the node always passes, so results
+//    never change, only the pages read.  1024 bits in a leaf page (up to 256
+//    nodes), 512 in an interior page.
+//  * In an interior page, a bit for every word a node starts at: whether a
+//    match lies on the scan's walk (node to node from the page's start) is
+//    then one bit instead of the walk, a chain of some 50 dependent
+//    shared-memory reads.  Every start is on the walk; the few words a node
+//    that did not fit leaves at a page's end can be on it too (a match there
+//    is walked to).
+// Bits come from a multilinear hash of the node's words (independent products)
+// apart from the bucket hash.
+constexpr uint32_t kPageMeta = 32;   // words of a page's line
+constexpr uint32_t kPageStarts = 16; // the first of an interior page's start bits
 constexpr uint32_t kBloomHashes = 3;
 HD_HD uint32_t bloom_bits(const uint32_t* q, uint32_t n)
 {
-    uint64_t h = 0x51ED2701F3A5C9B7ull ^ n;
-    for (uint32_t k = 0; k < n; k++)
-        h = mix64(h ^ q[k]);
-    // three 9-bit positions, packed
-    return uint32_t(h & 0x7FFFFFFu);
+    constexpr uint64_t mul[9] = {0x9E3779B97F4A7C15ull, 0xC2B2AE3D27D4EB4Full, 0x165667B19E3779F9ull,
+                                 0xD6E8FEB86659FD93ull, 0xA0761D6478BD642Full, 0xE7037ED1A0B428DBull,
+                                 0x8EBC6AF09C88C6E3ull, 0x589965CC75374CC3ull, 0x1D8E4E27C47D124Full};
+    uint64_t h = n;
+#pragma unroll
+    for (uint32_t k = 0; k < 9; k++)
+        if (k < n)
+            h += uint64_t(q[k]) * mul[k];
+    // three positions of 10 bits, packed
+    return uint32_t(mix64(h)) & 0x3FFFFFFFu;
 }
-HD_HD uint32_t bloom_pos(uint32_t bits, uint32_t i) { return (bits >> (9 * i)) & 511u; }
+HD_HD uint32_t bloom_pos(uint32_t bits, uint32_t i, bool leaf) { return (bits >> (10 * i)) & (leaf ? 1023u : 511u); }
 
 // Leaf bit of voxel (x, y, z) inside its 4x4x4 block (dag_utils.h:160-167).
 HD_HD uint32_t leaf_bit(uint32_t x, uint32_t y, uint32_t z)

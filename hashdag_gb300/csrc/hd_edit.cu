@@ -75,8 +75,8 @@ __global__ void __launch_bounds__(32 * kFoaWarps)
                        const uint32_t* __restrict__ vals, const uint32_t* __restrict__ starts,
                        const uint32_t* __restrict__ n_seg, const uint32_t* __restrict__ n_cand, EditCounters* ctr)
 {
-    __shared__ uint32_t page_s[kFoaWarps][kPage];
-    __shared__ uint32_t q_s[kFoaWarps][9];
+    __shared__ __align__(16) uint32_t page_s[kFoaWarps][kPage];
+    __shared__ __align__(16) uint32_t q_s[kFoaWarps][kFoaQuery];
     __shared__ FoaCache cache_s[kFoaWarps];
     if (__ldcg(t.error) != 0)
         return; // a level below failed (see k_edit_candidates)
@@ -132,7 +132,7 @@ static Level alloc_level(Scratch& s, uint32_t L, uint64_t n, bool leaf, bool col
     l.flag = static_cast<uint32_t*>(buf("flag", n * 4));
     l.exp = static_cast<uint32_t*>(buf("exp", n * 4));
     l.leaf = leaf ? static_cast<uint64_t*>(buf("leaf", n * 8)) : nullptr;
-    l.cand = static_cast<uint32_t*>(buf("cand", n * 36));
+    l.cand = static_cast<uint32_t*>(buf("cand", n * 4 * kRow));
     if (colors) {
         l.ocnt = static_cast<uint32_t*>(buf("ocnt", n * 4));
         l.cn = static_cast<uint32_t*>(buf("cn", n * 4));

@@ -196,6 +196,10 @@ HD_D bool inside_tool(const Editor& e, float mnx, float mny, float mnz, float mx
     return e.bminx <= mnx && e.bminy <= mny && e.bminz <= mnz && e.bmaxx >= mxx && e.bmaxy >= mxy && e.bmaxz >= mxz;
 }
 
+// A candidate's row: its words (zeros past the last), then at kRowBloom its
+// filter bits and at kRowSize its word count; 16-byte aligned.
+constexpr uint32_t kRow = 12, kRowBloom = 9, kRowSize = 10;
+
 // ---- per-level entry state ---------------------------------------------------
 enum : uint8_t {
     kSkip = 0,      // level-C_colorTreeLevels child the parent never hands to edit_leaf
@@ -217,7 +221,7 @@ struct Level {
     uint32_t* flag;  // 1 = descends
     uint32_t* exp;   // exclusive scan of flag
     uint64_t* leaf;  // new leaf masks (leaf level only)
-    uint32_t* cand;  // candidate content, 9 words per entry
+    uint32_t* cand;  // candidate rows, kRow words per entry
     // colours (allocated only when the context has colours)
     uint32_t* ocnt;  // voxel count of the old node (levels >= T)
     uint32_t* cn;    // levels < T: colour node; level T: the slot's leaf reference
@@ -398,7 +402,7 @@ HD_D uint32_t candidate_entry(const Table& t, uint32_t level, const Level& lv, c
 {
     const uint32_t T = t.g.T;
     const uint8_t state = lv.state[i];
-    uint32_t* c = lv.cand + 9 * i;
+    uint4* row = reinterpret_cast<uint4*>(lv.cand + uint64_t(kRow) * i);
     uint32_t hash;
     if (state == kLeafEval) {
         const uint64_t leaf = lv.leaf[i];
@@ -418,27 +422,40 @@ HD_D uint32_t candidate_entry(const Table& t, uint32_t level, const Level& lv, c
             lv.cnt[i] = 0;
             return kNoBucket;
         }
-        c[0] = uint32_t(leaf);
-        c[1] = uint32_t(leaf >> 32);
+        const uint32_t w[9] = {uint32_t(leaf), uint32_t(leaf >> 32)};
+        row[0] = make_uint4(w[0], w[1], 0, 0);
+        row[1] = make_uint4(0, 0, 0, 0);
+        row[2] = make_uint4(0, bloom_bits(w, 2), 2, 0);
         hash = hash_leaf(leaf);
     } else if (state == kDescend) {
+        // the 8 children in three independent reads of each array (all were
+        // spawned; old: the spawned child's old node, kInvalid where the old
+        // node had none, so the old node itself is not read again), the
+        // words hashed as they come: no chain of reads
         const uint32_t base = 8 * lv.exp[i];
         const uint32_t old = lv.old[i];
-        uint32_t mask = 0, k = 1, total = 0;
+        uint32_t oc[8], nc[8], cc[8];
+        const uint4* po = reinterpret_cast<const uint4*>(child.old + base);
+        const uint4* pr = reinterpret_cast<const uint4*>(child.res + base);
+        const uint4* pc = reinterpret_cast<const uint4*>(child.cnt + base);
+        const uint2 st = *reinterpret_cast<const uint2*>(child.state + base);
+#pragma unroll
+        for (uint32_t h = 0; h < 2; h++) {
+            const uint4 o = po[h], r = pr[h], n = level >= T ? pc[h] : make_uint4(0, 0, 0, 0);
+            oc[4 * h] = o.x, oc[4 * h + 1] = o.y, oc[4 * h + 2] = o.z, oc[4 * h + 3] = o.w;
+            nc[4 * h] = r.x, nc[4 * h + 1] = r.y, nc[4 * h + 2] = r.z, nc[4 * h + 3] = r.w;
+            cc[4 * h] = n.x, cc[4 * h + 1] = n.y, cc[4 * h + 2] = n.z, cc[4 * h + 3] = n.w;
+        }
+        uint32_t mask = 0, total = 0;
         bool changed = false;
+#pragma unroll
         for (uint32_t s = 0; s < 8; s++) {
-            // the old child in slot s: the spawned child's old node (all 8
-            // children were spawned; kInvalid where the old node had none),
-            // so the old node itself is not read again
-            const uint32_t oc = child.old[base + s];
-            const uint8_t cs = child.state[base + s];
-            const uint32_t nc = cs == kSkip ? oc : child.res[base + s];
-            changed |= nc != oc;
-            if (nc != kInvalid) {
+            const uint32_t cs = ((s < 4 ? st.x : st.y) >> (8 * (s & 3))) & 0xffu;
+            nc[s] = cs == kSkip ? oc[s] : nc[s];
+            changed |= nc[s] != oc[s];
+            if (nc[s] != kInvalid) {
                 mask |= 1u << s;
-                c[k++] = nc;
-                if (level >= T)
-                    total += child.cnt[base + s];
+                total += cc[s];
             }
         }
         lv.cnt[i] = total;
@@ -451,14 +468,41 @@ HD_D uint32_t candidate_entry(const Table& t, uint32_t level, const Level& lv, c
             lv.cnt[i] = 0;
             return kNoBucket;
         }
-        c[0] = (level >= T ? (total << 8) : 0u) | mask;
-        hash = hash_interior(k, c);
+        // the children packed to the front: a stable compaction by moves of
+        // 4, 2 and 1 slots (a child moves left by the empty slots before it)
+        uint32_t w[9], gap[8];
+        w[0] = (level >= T ? (total << 8) : 0u) | mask;
+#pragma unroll
+        for (uint32_t s = 0; s < 8; s++)
+            gap[s] = (mask >> s & 1u) ? popc32(~mask & ((1u << s) - 1u)) : 0u;
+#pragma unroll
+        for (uint32_t m = 1; m <= 4; m <<= 1)
+#pragma unroll
+            for (uint32_t s = m; s < 8; s++)
+                if (gap[s] & m) {
+                    nc[s - m] = nc[s];
+                    gap[s - m] = gap[s] - m;
+                    gap[s] = 0;
+                }
+        const uint32_t n = 1 + popc32(mask);
+#pragma unroll
+        for (uint32_t s = 0; s < 8; s++)
+            w[1 + s] = s + 1 < n ? nc[s] : 0u;
+        row[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        row[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        row[2] = make_uint4(w[8], bloom_bits(w, n), n, 0);
+        hash = hash_interior_words(n, w);
     } else {
         return kNoBucket;
     }
     const uint32_t bucket = hash & (t.g.buckets(level) - 1);
     lv.res[i] = kNotFound; // resolved by find-or-add
     return bucket;
+}
+
+HD_D bool same_words(const uint4& a, const uint4& b)
+{
+    return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
 }
 
 // One warp per bucket: the bucket's candidates, in depth-first order, each
@@ -489,126 +533,219 @@ HD_D bool visible(uint32_t p, uint32_t n, uint32_t S, bool leaf)
     return p + n < (S < pe ? S : pe);
 }
 
-// Copies words [0, used) of a page (used <= kPage) into the warp's shared
-// buffer, PW words per lane and load (the probe width: 1, 2 or 4).  L2-
-// coherent loads: the same kernel appends nodes and maps pages.  Up to PW-1
-// words past `used`, still inside the page, are copied too.
+// A page's words in the warp's registers and in its shared buffer: load r of
+// lane l holds words (32 r + l) PW .. + PW - 1 (PW, the probe width: 1, 2 or
+// 4), every load issued before the first is used.  L2-coherent loads: the
+// same kernel appends nodes and maps pages.  Words past `used`: whatever the
+// page holds there, or zeros.
 template <int PW>
-HD_D void stage_page(const uint32_t* src, uint32_t used, uint32_t* page, uint32_t lane)
+HD_D void load_page(const uint32_t* src, uint32_t used, uint32_t (&v)[kPage / 32], uint32_t* page, uint32_t lane)
 {
-    if constexpr (PW == 4) {
-        for (uint32_t w = lane * 4; w < used; w += 128) {
-            const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + w));
-            page[w] = v.x;
-            page[w + 1] = v.y;
-            page[w + 2] = v.z;
-            page[w + 3] = v.w;
+    constexpr uint32_t R = kPage / 32 / PW;
+#pragma unroll
+    for (uint32_t r = 0; r < R; r++) {
+        const uint32_t w = (r * 32 + lane) * PW;
+        const bool in = w < used;
+        if constexpr (PW == 4) {
+            const uint4 x = in ? __ldcg(reinterpret_cast<const uint4*>(src + w)) : make_uint4(0, 0, 0, 0);
+            v[4 * r] = x.x, v[4 * r + 1] = x.y, v[4 * r + 2] = x.z, v[4 * r + 3] = x.w;
+        } else if constexpr (PW == 2) {
+            const uint2 x = in ? __ldcg(reinterpret_cast<const uint2*>(src + w)) : make_uint2(0, 0);
+            v[2 * r] = x.x, v[2 * r + 1] = x.y;
+        } else {
+            v[r] = in ? __ldcg(src + w) : 0u;
         }
-    } else if constexpr (PW == 2) {
-        for (uint32_t w = lane * 2; w < used; w += 64) {
-            const uint2 v = __ldcg(reinterpret_cast<const uint2*>(src + w));
-            page[w] = v.x;
-            page[w + 1] = v.y;
-        }
-    } else {
-        for (uint32_t w = lane; w < used; w += 32)
-            page[w] = __ldcg(src + w);
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < R; r++) {
+        const uint32_t w = (r * 32 + lane) * PW;
+        if constexpr (PW == 4)
+            *reinterpret_cast<uint4*>(page + w) = make_uint4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
+        else if constexpr (PW == 2)
+            *reinterpret_cast<uint2*>(page + w) = make_uint2(v[2 * r], v[2 * r + 1]);
+        else
+            page[w] = v[r];
     }
 }
+
+// The walk from the page's start meets word `at` (lane 0 walks).
+HD_D bool walk_meets(const uint32_t* page, uint32_t at)
+{
+    uint32_t on = 0;
+    if ((threadIdx.x & 31) == 0) {
+        uint32_t p = 0;
+        while (p < at)
+            p += total_size(page[p]);
+        on = p == at;
+    }
+    return __shfl_sync(0xffffffffu, on, 0) != 0;
+}
+
+// The first word below `lim` of the staged page at which the n words of q lie,
+// on the walk (warp-wide); kNotFound when there is none.  Leaves: at even
+// words.  Interiors: `starts`, the page's start bits, says at once that a
+// match is on the walk; a match that is no start is walked to.
+template <int PW>
+HD_D uint32_t match_page(const uint32_t (&v)[kPage / 32], const uint32_t* page, const uint32_t* starts,
+                         const uint32_t* q, uint32_t n, uint32_t lim, bool leaf)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t m = 0; // the lane's words equal to q[0]
+#pragma unroll
+    for (uint32_t k = 0; k < kPage / 32; k++)
+        m |= (v[k] == q[0] ? 1u : 0u) << k;
+    uint32_t best = kNotFound, odd = kNotFound; // the lowest match that is a start, that is not
+    while (m) {
+        const uint32_t k = __ffs(m) - 1;
+        m &= m - 1;
+        const uint32_t w = ((k / PW) * 32 + lane) * PW + k % PW;
+        if (w >= lim || (leaf && (w & 1)))
+            continue;
+        bool eq = page[w + 1] == q[1];
+        for (uint32_t j = 2; eq && j < n; j++)
+            eq = page[w + j] == q[j];
+        if (!eq)
+            continue;
+        if (leaf || ((starts[w >> 5] >> (w & 31)) & 1u))
+            best = min(best, w);
+        else
+            odd = min(odd, w);
+    }
+    best = __reduce_min_sync(0xffffffffu, best);
+    // (no loop over further odd matches: past the first that the walk misses,
+    // each is looked at in turn)
+    uint32_t first = __reduce_min_sync(0xffffffffu, odd);
+    while (first < best) {
+        if (walk_meets(page, first))
+            return first;
+        // the next odd match of any lane, found again from the staged words
+        uint32_t next = kNotFound;
+        for (uint32_t w = lane; w < lim; w += 32) {
+            if (w <= first || ((starts[w >> 5] >> (w & 31)) & 1u))
+                continue;
+            bool eq = true;
+            for (uint32_t j = 0; eq && j < n; j++)
+                eq = page[w + j] == q[j];
+            if (eq) {
+                next = w;
+                break;
+            }
+        }
+        first = __reduce_min_sync(0xffffffffu, next);
+    }
+    return best;
+}
+
+// Words of a warp's query buffer: the candidate's row, then the start bits of
+// the page being scanned.
+constexpr uint32_t kFoaQuery = kRow + 16;
 
 // Warp-wide scan of the bucket for the first compared position holding q
 // (find_leaf_node_in_bucket / find_interior_node_in_bucket); returns the
 // bucket position or kNotFound.  *last_match: for interiors, the bucket's
 // last node when it holds q (compared by no scan until something follows).
+// Three dependent waits at most per scanned page: the size (the caller's)
+// and the filters together, then a page with its start bits.  (With the
+// pages' lines of 512 filter bits alone, a walk per match and words compared
+// from shared memory 32 at a time, 53 buckets of a small level took 25 us;
+// with runs dealt out to the warps as well, 7.6.)
 template <int PW>
-HD_D uint32_t scan_bucket(const Table& t, uint32_t vbase, uint32_t S, const uint32_t* q, uint32_t n, bool leaf,
+HD_D uint32_t scan_bucket(const Table& t, uint32_t vbase, uint32_t S, uint32_t* q, uint32_t n, bool leaf, uint32_t may,
                           uint32_t bloom, uint32_t pt_lane, uint32_t* page, uint32_t* last_match,
                           unsigned long long& scanned)
 {
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t found = kNotFound;
+    uint32_t* starts = q + kRow;
+    uint32_t found = kNotFound, staged = kNotFound;
     *last_match = kNotFound;
-    // the filters of the bucket's first 32 pages at once, a lane per page
-    // (pt_lane: the physical page behind the bucket's page `lane`, read
-    // once per bucket run)
-    const uint32_t npages = (S + kPage - 1) / kPage;
-    const uint32_t may = __ballot_sync(0xffffffffu, lane < npages && bloom_may_phys(t, pt_lane, bloom));
+    // page pi's physical page and whether its filter admits q: the first 32
+    // pages' from pt_lane / may (a lane per page)
+    auto page_of = [&](uint32_t pi) {
+        const uint32_t near = __shfl_sync(0xffffffffu, pt_lane, pi & 31);
+        return pi < 32 ? near : t.page_cg((vbase >> kPageShift) + pi);
+    };
+    auto admits = [&](uint32_t pi) {
+        return pi < 32 ? ((may >> pi) & 1u) != 0 : bloom_may_phys(t, page_of(pi), bloom, leaf);
+    };
+    uint32_t v[kPage / 32];
+    auto stage = [&](uint32_t pi, uint32_t used) {
+        const uint32_t phys = page_of(pi);
+        uint32_t sb = 0;
+        if (!leaf && lane < 16)
+            sb = __ldcg(t.meta + uint64_t(phys) * kPageMeta + kPageStarts + lane);
+        __syncwarp();
+        load_page<PW>(t.pool + (uint64_t(phys) << kPageShift), used, v, page, lane);
+        if (!leaf && lane < 16)
+            starts[lane] = sb;
+        __syncwarp();
+        staged = pi;
+    };
     for (uint32_t pindex = 0; pindex < S && found == kNotFound; pindex += kPage) {
         const uint32_t page_end = S < pindex + kPage ? S : pindex + kPage;
         if (!leaf && pindex + n >= page_end)
             break; // "return 0xFFFFFFFF" of the reference scan
         const uint32_t pi = pindex / kPage;
-        if (pi < 32 ? !((may >> pi) & 1u) : !bloom_may(t, vbase + pindex, bloom))
+        if (!admits(pi))
             continue; // the page cannot hold q
         const uint32_t used = page_end - pindex;
-        const uint32_t phys = __shfl_sync(0xffffffffu, pt_lane, pi & 31);
-        stage_page<PW>(pi < 32 ? t.pool + (uint64_t(phys) << kPageShift) : t.sys_cg(vbase + pindex), used, page, lane);
-        __syncwarp();
-        if (leaf) {
-            for (uint32_t w0 = 0; w0 < used && found == kNotFound; w0 += 64) {
-                const uint32_t w = w0 + 2 * lane;
-                const bool m = w < used && page[w] == q[0] && page[w + 1] == q[1];
-                const uint32_t b = __ballot_sync(0xffffffffu, m);
-                if (b)
-                    found = pindex + w0 + 2 * (__ffs(b) - 1);
-            }
-        } else {
-            const uint32_t lim = used - n;
-            for (uint32_t w0 = 0; w0 < lim && found == kNotFound; w0 += 32) {
-                const uint32_t w = w0 + lane;
-                bool m = w < lim && page[w] == q[0];
-                if (m)
-                    for (uint32_t k = 1; k < n; k++)
-                        m &= page[w + k] == q[k];
-                uint32_t b = __ballot_sync(0xffffffffu, m);
-                while (b && found == kNotFound) {
-                    const uint32_t cand = w0 + __ffs(b) - 1;
-                    b &= b - 1;
-                    uint32_t on_walk = 0;
-                    if (lane == 0) {
-                        uint32_t p = 0;
-                        while (p < cand)
-                            p += total_size(page[p]);
-                        on_walk = p == cand;
-                    }
-                    on_walk = __shfl_sync(0xffffffffu, on_walk, 0);
-                    if (on_walk)
-                        found = pindex + cand;
-                }
-            }
-        }
+        stage(pi, used);
+        const uint32_t w = match_page<PW>(v, page, starts, q, n, leaf ? used : used - n, leaf);
+        if (w != kNotFound)
+            found = pindex + w;
         scanned += found == kNotFound ? used : (found - pindex + n);
-        __syncwarp();
     }
-    const uint32_t tail_pi = (S - n) / kPage;
-    if (!leaf && found == kNotFound && S >= n && ((S - n) & ~(kPage - 1)) == ((S - 1) & ~(kPage - 1)) &&
-        (tail_pi < 32 ? ((may >> tail_pi) & 1u) != 0 : bloom_may(t, vbase + ((S - n) & ~(kPage - 1)), bloom))) {
+    if (!leaf && found == kNotFound && S >= n && ((S - n) & ~(kPage - 1)) == ((S - 1) & ~(kPage - 1))) {
         // the bucket's last node ends at S; it holds q iff it starts at S - n
-        // (nodes never straddle a page, so S - n lies in the tail's page)
-        const uint32_t p = S - n;
-        const uint32_t pindex = p & ~(kPage - 1);
-        const uint32_t phys = __shfl_sync(0xffffffffu, pt_lane, tail_pi & 31);
-        stage_page<PW>(tail_pi < 32 ? t.pool + (uint64_t(phys) << kPageShift) : t.sys_cg(vbase + pindex), S - pindex,
-                       page, lane); // S - pindex <= kPage
-        __syncwarp();
-        uint32_t ok = 0;
-        if (lane == 0) {
-            bool m = true;
-            for (uint32_t k = 0; k < n; k++)
-                m &= page[p - pindex + k] == q[k];
-            if (m) {
-                uint32_t w = 0;
-                while (w < p - pindex)
-                    w += total_size(page[w]);
-                ok = w == p - pindex;
-            }
+        // (nodes never straddle a page, so S - n lies in the tail's page,
+        // whose used words hold nodes only)
+        const uint32_t p = S - n, pi = p / kPage, at = p & (kPage - 1);
+        if (admits(pi)) {
+            if (staged != pi)
+                stage(pi, ((S - 1) & (kPage - 1)) + 1);
+            bool ok = lane >= n || page[at + lane] == q[lane];
+            ok = __all_sync(0xffffffffu, ok) && ((starts[at >> 5] >> (at & 31)) & 1u);
+            if (ok)
+                *last_match = p;
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (ok)
-            *last_match = p;
-        __syncwarp();
     }
     return found;
+}
+
+// A run of followers whose results are written after the find-or-add phase
+// (hd_edit_persist.cu): positions [begin, end) of the sorted candidates take
+// `result`.
+struct FollowerRun {
+    uint32_t begin, end, result, pad;
+};
+// The repeats of a level's sorted candidates: bit j set when candidate j has
+// the bucket and the words of candidate j - 1; runs longer than kLongRun go
+// to the list.
+struct Repeats {
+    const uint32_t* same; // null: not known
+    uint32_t words;
+    FollowerRun* runs;
+    uint32_t* n_runs;
+};
+constexpr uint32_t kLongRun = 64;
+
+// The end of the run of set bits from bit j on (warp-wide).
+HD_D uint32_t end_of_repeats(const Repeats& rep, uint32_t j)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t w0 = j >> 5, below = (1u << (j & 31)) - 1u;
+    for (;;) {
+        uint32_t word = w0 + lane < rep.words ? __ldcg(rep.same + w0 + lane) : 0u;
+        if (lane == 0)
+            word |= below;
+        below = 0;
+        const uint32_t open = __ballot_sync(0xffffffffu, word != 0xffffffffu);
+        if (open) {
+            const uint32_t l = __ffs(open) - 1;
+            const uint32_t at = __shfl_sync(0xffffffffu, word, l);
+            return (w0 + l) * 32 + __ffs(~at) - 1;
+        }
+        w0 += 32;
+    }
 }
 
 // Resolves the candidates vals[j0..j1) of one bucket (all lanes of a warp):
@@ -618,60 +755,66 @@ HD_D uint32_t scan_bucket(const Table& t, uint32_t vbase, uint32_t S, const uint
 template <int PW>
 HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uint32_t* __restrict__ vals, uint32_t j0,
                       uint32_t j1, uint32_t bucket, uint32_t* page, uint32_t* q, FoaCache& cache,
-                      unsigned long long& foa, unsigned long long& added, unsigned long long& scanned)
+                      unsigned long long& foa, unsigned long long& added, unsigned long long& scanned,
+                      const Repeats& rep = Repeats{})
 {
     const uint32_t lane = threadIdx.x & 31;
     const bool leaf = level == t.g.leaf_level;
     const uint32_t gb = t.g.bucket_global(level, bucket);
     const uint32_t vbase = t.g.make_ptr(level, bucket, 0);
-    uint32_t S = __ldcg(t.bucket_sizes + gb);
     // the bucket's page-table entries, lane p holding page p's (the warp owns
     // the bucket for the run: only its own appends map pages here)
     const uint32_t vpage0 = vbase >> kPageShift, cap_pages = t.g.capacity(level) >> kPageShift;
+    uint32_t S = __ldcg(t.bucket_sizes + gb);
     uint32_t pt_lane = lane < cap_pages ? t.page_cg(vpage0 + lane) : 0u;
     uint32_t used_entries = 0, next_slot = 0;
     bool failed = false;
     uint32_t j = j0;
     // the run's entry indices 32 at a time (lane k: entry of position vb + k)
-    // and the next candidate's words loaded while the current one resolves
+    // and the next candidate's row loaded while the current one resolves
     uint32_t vb = j0, vreg = j0 + lane < j1 ? vals[j0 + lane] : 0u;
     const uint32_t c0 = __shfl_sync(0xffffffffu, vreg, 0); // every lane: a full-warp shuffle
-    uint32_t qj = j0, qw = lane < 9 ? lv.cand[9 * uint64_t(c0) + lane] : 0u;
+    uint32_t qj = j0, qw = lane < kRow ? lv.cand[kRow * uint64_t(c0) + lane] : 0u;
     while (j < j1 && !failed) {
         if (j - vb >= 32) {
             vb = j;
             vreg = j + lane < j1 ? vals[j + lane] : 0u;
         }
         const uint32_t ci = __shfl_sync(0xffffffffu, vreg, j - vb);
-        if (qj != j && lane < 9)
-            qw = lv.cand[9 * uint64_t(ci) + lane];
-        if (lane < 9)
+        if (qj != j && lane < kRow)
+            qw = lv.cand[kRow * uint64_t(ci) + lane];
+        if (lane < kRow)
             q[lane] = qw;
         __syncwarp();
+        const uint32_t n = q[kRowSize], bloom = q[kRowBloom];
+        // the filters of the bucket's first 32 pages, a lane per page, beside
+        // the bucket size (they do not wait for it)
+        const uint32_t maybe = __ballot_sync(0xffffffffu, lane < cap_pages && bloom_may_phys(t, pt_lane, bloom, leaf));
         // prefetch candidate j + 1 (its entry index is in vreg unless it
         // starts the next group of 32)
         qj = j + 1;
         if (qj < j1 && qj - vb < 32) {
             const uint32_t cn = __shfl_sync(0xffffffffu, vreg, qj - vb);
-            if (lane < 9)
-                qw = lv.cand[9 * uint64_t(cn) + lane];
+            if (lane < kRow)
+                qw = lv.cand[kRow * uint64_t(cn) + lane];
         } else {
             qj = kNotFound;
         }
-        const uint32_t n = leaf ? 2 : total_size(q[0]);
         // cache lookup: lane e checks entry e
         bool hit = lane < used_entries && cache.n[lane] == n;
         if (hit)
             for (uint32_t k = 0; k < n; k++)
                 hit &= cache.words[lane][k] == q[k];
         const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-        const uint32_t bloom = bloom_bits(q, n);
         uint32_t e;
         if (hb) {
             e = __ffs(hb) - 1;
         } else {
             uint32_t last_match;
-            const uint32_t f = scan_bucket<PW>(t, vbase, S, q, n, leaf, bloom, pt_lane, page, &last_match, scanned);
+            const uint32_t npages = (S + kPage - 1) / kPage;
+            const uint32_t may = npages < 32 ? maybe & ((1u << npages) - 1u) : maybe;
+            const uint32_t f =
+                scan_bucket<PW>(t, vbase, S, q, n, leaf, may, bloom, pt_lane, page, &last_match, scanned);
             e = next_slot;
             next_slot = (next_slot + 1) % kCache;
             used_entries = used_entries < kCache ? used_entries + 1 : kCache;
@@ -687,73 +830,81 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
             }
             __syncwarp();
         }
-        // the first visible copy, else append (lane 0)
-        uint32_t result = kNotFound, appended = 0, ok = 1;
-        const uint32_t S_scan = S;
-        // where an append would go, on every lane (S and n are the warp's),
-        // and the physical page there when it is already mapped: the pages
-        // below the size are, so an append that stays in the size's last
-        // page reads no page-table entry
-        uint32_t a_size = S;
-        const uint32_t a_pos = append_position(a_size, n, leaf);
-        const bool a_mapped = S > 0 && a_size <= ((S + kPage - 1) & ~(kPage - 1));
-        const uint32_t a_phys = __shfl_sync(0xffffffffu, pt_lane, (a_pos >> kPageShift) & 31);
-        if (lane == 0) {
-            for (uint32_t k = 0; k < cache.npos[e] && result == kNotFound; k++)
-                if (visible(cache.pos[e][k], n, S, leaf))
-                    result = cache.pos[e][k];
-            if (result == kNotFound) {
-                uint32_t size = a_size;
-                const uint32_t pos = a_pos;
-                if (size > t.g.capacity(level)) {
+        // the first visible copy, else append (the same on every lane)
+        uint32_t result = kNotFound;
+        const uint32_t np = cache.npos[e];
+        for (uint32_t k = 0; k < np && result == kNotFound; k++)
+            if (visible(cache.pos[e][k], n, S, leaf))
+                result = cache.pos[e][k];
+        const bool appended = result == kNotFound;
+        if (appended) {
+            uint32_t size = S;
+            const uint32_t pos = append_position(size, n, leaf);
+            // the pages below the size are mapped: an append that stays in
+            // the size's last page reads no page-table entry
+            const bool mapped = S > 0 && size <= ((S + kPage - 1) & ~(kPage - 1));
+            uint32_t ok = 1;
+            if (size > t.g.capacity(level)) {
+                if (lane == 0)
                     set_error(t.error, kErrBucketFull, level, bucket, size);
-                    ok = 0;
-                } else if (!a_mapped && !map_pages(t, level, bucket, pos, size)) {
-                    ok = 0;
-                } else {
-                    const uint32_t phys =
-                        a_mapped && (pos >> kPageShift) < 32 ? a_phys : t.page_cg(vpage0 + (pos >> kPageShift));
-                    uint32_t* dst = t.pool + (uint64_t(phys) << kPageShift) + (pos & (kPage - 1));
-                    for (uint32_t k = 0; k < n; k++)
-                        __stcg(dst + k, q[k]);
-                    bloom_add_phys(t, phys, bloom);
-                    result = pos;
-                    S = size;
-                    appended = 1;
-                    if (cache.npos[e] == kCachePos) { // keep the newest copies
-                        for (uint32_t k = 1; k < kCachePos; k++)
-                            cache.pos[e][k - 1] = cache.pos[e][k];
-                        cache.npos[e]--;
-                    }
-                    cache.pos[e][cache.npos[e]++] = pos;
-                }
+                ok = 0;
+            } else if (!mapped) {
+                if (lane == 0)
+                    ok = map_pages(t, level, bucket, pos, size);
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                // refresh the entries of the pages the append reached
+                if (ok && lane < cap_pages && lane * kPage < size && lane * kPage + kPage > S)
+                    pt_lane = t.page_cg(vpage0 + lane);
             }
+            if (ok) {
+                const uint32_t near = __shfl_sync(0xffffffffu, pt_lane, (pos >> kPageShift) & 31);
+                const uint32_t phys = (pos >> kPageShift) < 32 ? near : t.page_cg(vpage0 + (pos >> kPageShift));
+                if (lane < n)
+                    __stcg(t.pool + (uint64_t(phys) << kPageShift) + (pos & (kPage - 1)) + lane, q[lane]);
+                if (lane == 0)
+                    bloom_add_phys(t, phys, pos & (kPage - 1), bloom, leaf);
+                result = pos;
+                S = size;
+                added++;
+            } else {
+                failed = true;
+            }
+            __syncwarp(); // the positions were read by every lane
+            if (lane == 0 && ok) {
+                if (cache.npos[e] == kCachePos) { // keep the newest copies
+                    for (uint32_t k = 1; k < kCachePos; k++)
+                        cache.pos[e][k - 1] = cache.pos[e][k];
+                    cache.npos[e]--;
+                }
+                cache.pos[e][cache.npos[e]++] = pos;
+            }
+        }
+        if (lane == 0)
             lv.res[ci] = vbase + result;
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        result = __shfl_sync(0xffffffffu, result, 0);
-        appended = __shfl_sync(0xffffffffu, appended, 0);
-        const uint32_t S_before = __shfl_sync(0xffffffffu, S_scan, 0);
-        S = __shfl_sync(0xffffffffu, S, 0);
-        // an append that reached a new page mapped it: refresh that lane
-        if (appended && lane < cap_pages && lane * kPage < S && lane * kPage + kPage > S_before)
-            pt_lane = t.page_cg(vpage0 + lane);
         foa++;
-        added += appended;
-        if (!ok) {
-            failed = true;
+        if (failed)
             break;
-        }
         j++;
         // a found result holds for the identical candidates that follow
-        if (!appended) {
+        if (!appended && rep.same) {
+            const uint32_t e1 = min(end_of_repeats(rep, j), j1);
+            if (e1 - j > kLongRun) {
+                if (lane == 0)
+                    rep.runs[atomicAdd(rep.n_runs, 1u)] = FollowerRun{j, e1, vbase + result, 0};
+            } else {
+                for (uint32_t k = j + lane; k < e1; k += 32)
+                    lv.res[vals[k]] = vbase + result;
+            }
+            foa += e1 - j;
+            j = e1;
+        } else if (!appended) {
             for (;;) {
                 const uint32_t jj = j + lane;
                 bool same = jj < j1;
                 if (same) {
-                    const uint32_t* c = lv.cand + 9 * uint64_t(vals[jj]);
-                    for (uint32_t k = 0; k < n; k++)
-                        same &= c[k] == q[k];
+                    const uint4* c = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(vals[jj]));
+                    const uint4* p = reinterpret_cast<const uint4*>(q);
+                    same = same_words(c[0], p[0]) && same_words(c[1], p[1]) && c[2].x == p[2].x;
                 }
                 const uint32_t b = __ballot_sync(0xffffffffu, same);
                 const uint32_t run = b == 0xffffffffu ? 32u : __ffs(~b) - 1;

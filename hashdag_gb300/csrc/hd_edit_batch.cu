@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(32 * WARPS)
 {
     if (bs->skip || __ldcg(t.error) != 0)
         return;
-    __shared__ uint32_t page_s[WARPS][kPage];
-    __shared__ uint32_t q_s[WARPS][9];
+    __shared__ __align__(16) uint32_t page_s[WARPS][kPage];
+    __shared__ __align__(16) uint32_t q_s[WARPS][kFoaQuery];
     __shared__ FoaCache cache_s[WARPS];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = bs->count[level];
@@ -470,7 +470,7 @@ static Level batch_level(Scratch& s, uint32_t L, uint64_t n, bool leaf, bool col
     l.flag = static_cast<uint32_t*>(buf("flag", n * 4));
     l.exp = static_cast<uint32_t*>(buf("exp", n * 4));
     l.leaf = leaf ? static_cast<uint64_t*>(buf("leaf", n * 8)) : nullptr;
-    l.cand = static_cast<uint32_t*>(buf("cand", n * 36));
+    l.cand = static_cast<uint32_t*>(buf("cand", n * 4 * kRow));
     if (colors) {
         l.ocnt = static_cast<uint32_t*>(buf("ocnt", n * 4));
         l.cn = static_cast<uint32_t*>(buf("cn", n * 4));
@@ -491,7 +491,7 @@ static BatchBuffers batch_buffers(hd_ctx* c, const std::vector<uint64_t>& cap64,
     b.caps.resize(levels);
     uint64_t maxn = 1;
     for (uint32_t L = 0; L < levels; L++) {
-        const uint64_t v = std::min<uint64_t>(std::max<uint64_t>(cap64[L], 256), 0xFFFFFFF0ull / 9);
+        const uint64_t v = std::min<uint64_t>(std::max<uint64_t>(cap64[L], 256), 0xFFFFFFF0ull / kRow);
         b.caps[L] = uint32_t(v);
         maxn = std::max(maxn, v);
     }
@@ -895,7 +895,7 @@ void copy_table(hd_ctx* to, hd_ctx* from)
         // pages lie anywhere in a direct-mapped pool: all of it
         HD_CUDA(cudaMemcpyAsync(to->t.pool, from->t.pool, uint64_t(from->g.pool_pages) * kPage * 4,
                                 cudaMemcpyDeviceToDevice, st));
-        HD_CUDA(cudaMemcpyAsync(to->t.bloom, from->t.bloom, uint64_t(from->g.pool_pages) * kBloomWords * 4,
+        HD_CUDA(cudaMemcpyAsync(to->t.meta, from->t.meta, uint64_t(from->g.pool_pages) * kPageMeta * 4,
                                 cudaMemcpyDeviceToDevice, st));
         HD_CUDA(cudaMemcpyAsync(to->t.page_ids, from->t.page_ids, from->g.total_vpages * 4, cudaMemcpyDeviceToDevice,
                                 st));
@@ -908,9 +908,9 @@ void copy_table(hd_ctx* to, hd_ctx* from)
         HD_CUDA(
             cudaMemcpyAsync(to->t.pool, from->t.pool, uint64_t(top_from) * kPage * 4, cudaMemcpyDeviceToDevice, st));
         if (top_to > top_from)
-            HD_CUDA(cudaMemsetAsync(to->t.bloom + uint64_t(top_from) * kBloomWords, 0,
-                                    uint64_t(top_to - top_from) * kBloomWords * 4, st));
-        HD_CUDA(cudaMemcpyAsync(to->t.bloom, from->t.bloom, uint64_t(top_from) * kBloomWords * 4,
+            HD_CUDA(cudaMemsetAsync(to->t.meta + uint64_t(top_from) * kPageMeta, 0,
+                                    uint64_t(top_to - top_from) * kPageMeta * 4, st));
+        HD_CUDA(cudaMemcpyAsync(to->t.meta, from->t.meta, uint64_t(top_from) * kPageMeta * 4,
                                 cudaMemcpyDeviceToDevice, st));
     }
     HD_CUDA(cudaMemcpyAsync(to->t.page_table, from->t.page_table, from->g.total_vpages * 4, cudaMemcpyDeviceToDevice,

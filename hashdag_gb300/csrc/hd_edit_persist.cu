@@ -28,6 +28,7 @@
 //  * Nodes and pages that an edit appends are read by the following edits in
 //    the same launch: every table read uses L2-coherent loads.
 // The graph-per-edit form (hd_edit_batch.cu) stays as the other batch mode.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -41,6 +42,11 @@ constexpr uint32_t kPT = 1024;             // threads per CTA (one CTA per SM)
 constexpr uint32_t kPWarps = kPT / 32;
 constexpr uint32_t kSmall = kPT;           // entries of a level CTA 0 handles alone
 constexpr uint32_t kDigits = 512;          // radix digits per pass at most (9 bits)
+// Bucket runs of a small level that CTA 0's warps resolve themselves (four
+// each, about 1.5 us a run); more are worth the two barriers of a grid step.
+constexpr uint32_t kLocalRuns = 4 * kPWarps;
+// Candidates of a big level from which repeats are looked for (a grid step).
+constexpr uint32_t kRepeatLevel = 4096;
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
 enum : uint32_t { kRun = 0, kDone = 1, kCapacity = 2, kTableError = 3, kEmptyScene = 4, kAborted = 5 };
@@ -58,12 +64,18 @@ struct Cmd {
 // read: it writes the slot of the next barrier, which no CTA reads until
 // every CTA has left this one.
 struct Ctl {
-    uint32_t arrived, abort, stop; // arrived: grid barrier arrivals of the launch
+    // grid barrier arrivals of the launch, and the flag of a CTA that gave up
+    // (read together, as one word)
+    uint32_t arrived, abort;
+    uint32_t stop;
     uint32_t idx;       // edit being applied
     uint32_t phase;     // the grid step CTA 0 asks for (kPh*)
     uint32_t level;     // its level
     uint32_t deepest;   // deepest level of the current edit
+    uint32_t n_small_runs; // bucket runs of the small level handed to the grid
     Cmd cmd[2];
+    uint32_t ncand[HD_MAX_DEPTH]; // big levels: candidates for find-or-add
+    uint32_t nruns[HD_MAX_DEPTH]; // big levels: long runs of repeats
     uint32_t count[HD_MAX_DEPTH];
     // where a wait ran out: the CTA, its barrier count, the arrivals then and
     // the count it waited for, CTA 0's barrier count, phase, level and edit
@@ -97,6 +109,8 @@ struct PArgs {
     uint32_t *keys, *vals, *keys2, *vals2;
     uint32_t* bsum;      // 3 x G: per-chunk descend-flag counts, by level parity
     uint32_t *hist, *hist2, *rows, *rows2; // kDigits x G, kDigits
+    uint32_t* same;      // a big level's repeats, a bit per sorted candidate
+    FollowerRun* runs;   // its long runs of repeats
     EditOut* out;
     uint32_t* d_root;
 };
@@ -113,12 +127,22 @@ HD_D uint32_t ld_acquire(const uint32_t* p)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+HD_D unsigned long long ld_acquire64(const void* p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // Grid barrier of the cooperative launch with a bounded wait; false when a
 // wait ran out or another CTA gave up (the caller returns).  The arrival
 // count only grows (the control block starts at zero every launch), so the
 // k-th barrier is passed once k x CTAs have arrived: no reset, and no
-// generation word for the last CTA to publish after its arrival.
+// generation word for the last CTA to publish after its arrival.  Bound by
+// L2 round trips: a poll is one acquire of the arrivals and the abort flag
+// together, without a pause until it has waited long (with two reads and a
+// pause a poll, and a fence after, a grid step of almost no work took 2.7-4.3
+// us, now 2.4-3.5).
 HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
 {
     __shared__ uint32_t ok;
@@ -130,35 +154,44 @@ HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
             __stcg(&ctl->bars0, nbar);
         const uint32_t target = nbar * gridDim.x;
         __threadfence();
-        if (atomicAdd(&ctl->arrived, 1u) + 1u != target) {
-            const unsigned long long t0 = now_ns();
-            const unsigned long long set_ns = __ldcg(&ctl->wait_ns);
-            const unsigned long long limit = set_ns ? set_ns : kWaitNs;
+        if (atomicAdd(&ctl->arrived, 1u) + 1u == target) {
+            __threadfence(); // the last to arrive acquires here
+        } else {
+            unsigned long long t0 = 0;
             uint32_t spins = 0;
-            while (int32_t(ld_acquire(&ctl->arrived) - target) < 0) {
-                if (ld_acquire(&ctl->abort)) {
+            for (;;) {
+                const unsigned long long both = ld_acquire64(&ctl->arrived);
+                if (int32_t(uint32_t(both) - target) >= 0)
+                    break;
+                if (uint32_t(both >> 32)) {
                     ok = 0;
                     break;
                 }
-                if ((++spins & 255u) == 0 && now_ns() - t0 > limit) {
-                    if (atomicExch(&ctl->abort, 1u) == 0) {
-                        ctl->diag[0] = blockIdx.x;
-                        ctl->diag[1] = nbar;
-                        ctl->diag[2] = ld_acquire(&ctl->arrived);
-                        ctl->diag[3] = target;
-                        ctl->diag[4] = ld_acquire(&ctl->bars0);
-                        ctl->diag[5] = ld_acquire(&ctl->phase);
-                        ctl->diag[6] = ld_acquire(&ctl->level);
-                        ctl->diag[7] = ld_acquire(&ctl->idx);
+                if ((++spins & 255u) == 0) {
+                    if (!t0)
+                        t0 = now_ns();
+                    const unsigned long long set_ns = __ldcg(&ctl->wait_ns);
+                    const unsigned long long limit = set_ns ? set_ns : kWaitNs;
+                    if (now_ns() - t0 > limit) {
+                        if (atomicExch(&ctl->abort, 1u) == 0) {
+                            ctl->diag[0] = blockIdx.x;
+                            ctl->diag[1] = nbar;
+                            ctl->diag[2] = ld_acquire(&ctl->arrived);
+                            ctl->diag[3] = target;
+                            ctl->diag[4] = ld_acquire(&ctl->bars0);
+                            ctl->diag[5] = ld_acquire(&ctl->phase);
+                            ctl->diag[6] = ld_acquire(&ctl->level);
+                            ctl->diag[7] = ld_acquire(&ctl->idx);
+                        }
+                        set_error(err, kErrTimeout, 0xFFFFFFFEu, blockIdx.x, 0);
+                        ok = 0;
+                        break;
                     }
-                    set_error(err, kErrTimeout, 0xFFFFFFFEu, blockIdx.x, 0);
-                    ok = 0;
-                    break;
                 }
-                __nanosleep(64);
+                if (spins > 64)
+                    __nanosleep(64);
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return ok != 0;
@@ -401,16 +434,41 @@ HD_D void candidates_range(const Table& t, const Level* lvs, uint32_t L, uint32_
     }
 }
 
-// Find-or-add over sorted keys [0, n) (runs of one bucket in entry order):
-// the positions are split into one chunk per warp (ceil(n / nw), at least
-// one) and warp w of nw resolves every run that starts in its chunk, so that
-// short runs spread over all the warps.
-// SH: keys / vals in the CTA's shared memory (CTA 0's small levels), read
-// with plain loads; else global arrays another phase wrote, read from L2.
-template <int PW, bool SH = false>
+HD_D void foa_counts(const Table& t, uint32_t L, EditCounters* ctr, unsigned long long foa, unsigned long long added,
+                     unsigned long long scanned)
+{
+    if ((threadIdx.x & 31) == 0 && (foa | added | scanned)) {
+        atomicAdd(&ctr->foa, foa);
+        atomicAdd(&ctr->added, added);
+        atomicAdd(&ctr->scanned, scanned);
+        atomicAdd(reinterpret_cast<unsigned long long*>(t.level_nodes + L), added);
+    }
+}
+
+// Find-or-add of a small level: its bucket runs (starts[r] .. starts[r + 1] of
+// the sorted candidates) dealt out to the nw warps in turn.
+template <int PW>
+HD_D void foa_runs(const Table& t, uint32_t L, const Level& lv, const uint32_t* keys, const uint32_t* vals,
+                   const uint32_t* starts, uint32_t runs, uint32_t w, uint32_t nw, uint32_t* page, uint32_t* q,
+                   FoaCache& cache, EditCounters* ctr)
+{
+    unsigned long long foa = 0, added = 0, scanned = 0;
+    for (uint32_t r = w; r < runs; r += nw) {
+        const uint32_t j0 = starts[r], j1 = starts[r + 1];
+        foa_segment<PW>(t, L, lv, vals, j0, j1, keys[j0], page, q, cache, foa, added, scanned);
+    }
+    foa_counts(t, L, ctr, foa, added, scanned);
+}
+
+// Find-or-add over the sorted keys [0, n) of a big level (runs of one bucket
+// in entry order; n: its candidates): the positions are split into one chunk
+// per warp (ceil(n / nw), at least one) and warp w of nw resolves every run
+// that starts in its chunk, so that short runs spread over all the warps.
+// The arrays were written in another phase: read from L2.
+template <int PW>
 HD_D void foa_sorted(const Table& t, uint32_t L, const Level& lv, const uint32_t* keys, const uint32_t* vals,
                      uint32_t n, uint32_t w, uint32_t nw, uint32_t* page, uint32_t* q, FoaCache& cache,
-                     EditCounters* ctr)
+                     EditCounters* ctr, const Repeats& rep)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t empty = t.g.buckets(L);
@@ -421,101 +479,142 @@ HD_D void foa_sorted(const Table& t, uint32_t L, const Level& lv, const uint32_t
     for (uint32_t c0 = cbeg; c0 < cend; c0 += 32) {
         const uint32_t j = c0 + lane;
         const bool in = j < cend;
-        const uint32_t key = in ? (SH ? keys[j] : __ldcg(keys + j)) : empty;
-        const uint32_t prev = (in && j > 0) ? (SH ? keys[j - 1] : __ldcg(keys + j - 1)) : kNoBucket;
+        const uint32_t key = in ? __ldcg(keys + j) : empty;
+        const uint32_t prev = (in && j > 0) ? __ldcg(keys + j - 1) : kNoBucket;
         uint32_t starts = __ballot_sync(0xffffffffu, in && key < empty && key != prev);
         while (starts) {
             const uint32_t s = __ffs(starts) - 1;
             starts &= starts - 1;
             const uint32_t j0 = c0 + s;
             const uint32_t bucket = __shfl_sync(0xffffffffu, key, s);
+            // the run's end: 128 keys at a time
             uint32_t j1 = j0 + 1;
             for (;;) {
-                const uint32_t jj = j1 + lane;
-                const uint32_t k = jj < n ? (SH ? keys[jj] : __ldcg(keys + jj)) : kNoBucket;
-                const uint32_t diff = __ballot_sync(0xffffffffu, k != bucket);
-                if (diff) {
-                    j1 += __ffs(diff) - 1;
-                    break;
+                uint32_t k[4];
+#pragma unroll
+                for (uint32_t m = 0; m < 4; m++)
+                    k[m] = j1 + 32 * m + lane < n ? __ldcg(keys + j1 + 32 * m + lane) : kNoBucket;
+                uint32_t same = 128; // keys before the first other one
+#pragma unroll
+                for (int m = 3; m >= 0; m--) {
+                    const uint32_t diff = __ballot_sync(0xffffffffu, k[m] != bucket);
+                    same = diff ? 32 * m + __ffs(diff) - 1 : same;
                 }
-                j1 += 32;
+                j1 += same;
+                if (same < 128)
+                    break;
             }
-            foa_segment<PW>(t, L, lv, vals, j0, j1, bucket, page, q, cache, foa, added, scanned);
+            foa_segment<PW>(t, L, lv, vals, j0, j1, bucket, page, q, cache, foa, added, scanned, rep);
         }
     }
-    if (lane == 0 && (foa | added | scanned)) {
-        atomicAdd(&ctr->foa, foa);
-        atomicAdd(&ctr->added, added);
-        atomicAdd(&ctr->scanned, scanned);
-        atomicAdd(reinterpret_cast<unsigned long long*>(t.level_nodes + L), added);
+    foa_counts(t, L, ctr, foa, added, scanned);
+}
+
+// Bit j of `same`: sorted candidate j has the bucket and the words of
+// candidate j - 1 (positions [j0, j1), j0 a multiple of 32; n: candidates).
+// A flat face of a box gives tens of thousands of equal candidates in one
+// bucket; the warp that resolves them then steps over them by these bits, 1,024
+// at a time, and leaves their results to the whole grid (fill_runs), where
+// it compared and wrote them 32 at a time: the leaf level of a box of radius
+// 250 (55,640 candidates) went from 1,063 to 94 us, the edit from 1.96 to 0.53
+// ms.
+HD_D void mark_repeats(const Level& lv, const uint32_t* keys, const uint32_t* vals, uint32_t n, uint32_t j0,
+                       uint32_t j1, uint32_t* same)
+{
+    for (uint32_t j = j0 + threadIdx.x; j - threadIdx.x < j1; j += kPT) {
+        bool eq = false;
+        if (j < j1 && j > 0 && j < n && __ldcg(keys + j) == __ldcg(keys + j - 1)) {
+            const uint4* a = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(__ldcg(vals + j)));
+            const uint4* b = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(__ldcg(vals + j - 1)));
+            eq = same_words(a[0], b[0]) && same_words(a[1], b[1]) && a[2].x == b[2].x;
+        }
+        const uint32_t bits = __ballot_sync(0xffffffffu, eq);
+        if ((threadIdx.x & 31) == 0 && j < j1)
+            same[j >> 5] = bits;
+    }
+}
+
+// The results of the long runs of repeats, by every thread of the grid.
+HD_D void fill_runs(const Level& lv, const uint32_t* vals, const FollowerRun* runs, uint32_t n)
+{
+    for (uint32_t r = 0; r < n; r++) {
+        const uint4 x = __ldcg(reinterpret_cast<const uint4*>(runs + r));
+        for (uint32_t j = x.x + blockIdx.x * kPT + threadIdx.x; j < x.y; j += gridDim.x * kPT)
+            lv.res[__ldcg(vals + j)] = x.z;
     }
 }
 
 // CTA 0 alone: stable sort of the n (<= kPT) candidates of a small level by
-// (bucket, entry) in shared memory, written back to keys / vals (visible to
-// the CTA after its barriers, to the grid after the next grid barrier);
-// returns the number of bucket runs.
-HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, uint32_t* keys, uint32_t* vals,
-                         unsigned long long* s64, uint32_t* sm32, uint32_t* sk, uint32_t* sv)
+// (bucket, entry) in registers, one a thread: a bitonic network with lane
+// shuffles, and shared memory for the steps across warps (two buffers, so
+// one barrier a step; a rank sort, n reads a thread, took 15.6 us at n = 784).
+// The sorted buckets and entries go to sk / sv, the starts of the bucket runs
+// to rs (one more: their end); returns the number of runs.
+HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, const uint32_t* keys, const uint32_t* vals,
+                         unsigned long long* s64, uint32_t* sm32, uint32_t* sk, uint32_t* sv, uint32_t* rs)
 {
     const uint32_t empty = t.g.buckets(L);
+    const uint32_t i = threadIdx.x, lane = i & 31;
+    unsigned long long x = i < n ? (uint64_t(keys[i]) << 32) | vals[i] : ~0ull;
+    auto keep = [&](unsigned long long y, uint32_t k, uint32_t j) {
+        const bool up = (i & k) == 0, low = (i & j) == 0;
+        x = (low == up) == (x < y) ? x : y;
+    };
+    const bool mine = (i & ~31u) < n; // the other warps hold no candidate
+    if (mine)
+        for (uint32_t k = 2; k <= 32; k <<= 1)
+            for (uint32_t j = k >> 1; j > 0; j >>= 1)
+                keep(__shfl_xor_sync(0xffffffffu, x, j), k, j);
+    uint32_t n2 = 32, step = 0;
+    while (n2 < n)
+        n2 <<= 1;
+    for (uint32_t k = 64; k <= n2; k <<= 1) {
+        for (uint32_t j = k >> 1; j >= 32; j >>= 1) {
+            unsigned long long* buf = s64 + (step++ & 1) * kPT;
+            if (i < n2)
+                buf[i] = x;
+            __syncthreads();
+            if (i < n2)
+                keep(buf[i ^ j], k, j);
+        }
+        if (i < n2)
+            for (uint32_t j = 16; j > 0; j >>= 1)
+                keep(__shfl_xor_sync(0xffffffffu, x, j), k, j);
+    }
+    const uint32_t key = uint32_t(x >> 32);
+    const bool cand = i < n && key < empty;
+    if (i < n) {
+        sk[i] = key;
+        sv[i] = uint32_t(x);
+    }
     if (n <= 32) {
-        // one warp, in registers: a bitonic network over the lanes on the
-        // (bucket, entry) pairs (entries are distinct: the order is total)
-        if (threadIdx.x < 32) {
-            const uint32_t lane = threadIdx.x;
-            unsigned long long x = lane < n ? (uint64_t(keys[lane]) << 32) | vals[lane] : ~0ull;
-            for (uint32_t k = 2; k <= 32; k <<= 1)
-                for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                    const unsigned long long y = __shfl_xor_sync(0xffffffffu, x, j);
-                    const bool up = (lane & k) == 0, low = (lane & j) == 0;
-                    x = (low == up) ? (x < y ? x : y) : (x < y ? y : x);
-                }
-            const uint32_t key = uint32_t(x >> 32);
+        // one warp holds them all
+        if (i < 32) {
             const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-            if (lane < n) {
-                keys[lane] = key;
-                vals[lane] = uint32_t(x);
-                sk[lane] = key;
-                sv[lane] = uint32_t(x);
+            const bool start = cand && (lane == 0 || prev != key);
+            const uint32_t sb = __ballot_sync(0xffffffffu, start), cb = __ballot_sync(0xffffffffu, cand);
+            if (start)
+                rs[__popc(sb & ((1u << lane) - 1u))] = i;
+            if (lane == 0) {
+                rs[__popc(sb)] = __popc(cb);
+                sm32[0] = __popc(sb);
             }
-            const uint32_t runs = __popc(__ballot_sync(0xffffffffu, lane < n && key < empty && (lane == 0 || prev != key)));
-            if (lane == 0)
-                sm32[0] = runs;
         }
         __syncthreads();
         const uint32_t runs = sm32[0];
         __syncthreads();
         return runs;
     }
-    // n <= kPT: a rank sort, one element per thread: the (bucket, entry)
-    // pairs are distinct, so an element's rank is the count of smaller ones
-    // (every thread reads the same shared word at a time: a broadcast)
-    unsigned long long* in = s64;
-    unsigned long long* out = s64 + kPT;
-    const uint32_t i = threadIdx.x;
-    const unsigned long long x = i < n ? (uint64_t(keys[i]) << 32) | vals[i] : ~0ull;
-    in[i] = x;
+    const uint32_t ncand = __syncthreads_count(cand); // also: sk is written
+    const bool start = cand && (i == 0 || sk[i - 1] != key);
+    uint32_t runs;
+    const uint32_t at = cta_scan(start, &runs, sm32);
+    if (start)
+        rs[at] = i;
+    if (i == 0)
+        rs[runs] = ncand;
     __syncthreads();
-    if (i < n) {
-        uint32_t rank = 0;
-        for (uint32_t k = 0; k < n; k++)
-            rank += in[k] < x;
-        out[rank] = x;
-    }
-    __syncthreads();
-    uint32_t runs = 0;
-    if (i < n) {
-        const uint32_t key = uint32_t(out[i] >> 32);
-        keys[i] = key;
-        vals[i] = uint32_t(out[i]);
-        sk[i] = key;
-        sv[i] = uint32_t(out[i]);
-        runs = key < empty && (i == 0 || uint32_t(out[i - 1] >> 32) != key);
-    }
-    uint32_t total;
-    cta_scan(runs, &total, sm32);
-    return total;
+    return runs;
 }
 
 // Per digit row of a [kDigits][nb] count table: exclusive scan over the
@@ -601,16 +700,17 @@ enum : uint32_t { kPhNone = 0, kPhTopDown = 1, kPhBottomUp = 2, kPhGridFoa = 3 }
 // follow.
 HD_HD constexpr size_t persist_smem_core()
 {
-    return (size_t(kPWarps) * kPage * 4 + size_t(kPWarps) * 12 * 4 + size_t(kPWarps) * sizeof(FoaCache) >
+    return (size_t(kPWarps) * kPage * 4 + size_t(kPWarps) * kFoaQuery * 4 + size_t(kPWarps) * sizeof(FoaCache) >
                     size_t(kPT) * 8 * 2
-                ? size_t(kPWarps) * kPage * 4 + size_t(kPWarps) * 12 * 4 + size_t(kPWarps) * sizeof(FoaCache)
+                ? size_t(kPWarps) * kPage * 4 + size_t(kPWarps) * kFoaQuery * 4 + size_t(kPWarps) * sizeof(FoaCache)
                 : size_t(kPT) * 8 * 2) +
            15 & ~size_t(15);
 }
 
 struct Smem {
-    uint32_t* sk; // a small level's sorted keys and entries (kPT each), past
-    uint32_t* sv; // the buffers below (which the find-or-add overwrites)
+    uint32_t* sk; // a small level's sorted keys and entries (kPT each) and
+    uint32_t* sv; // run starts (kPT + 1), past the buffers below (which the
+    uint32_t* rs; // find-or-add overwrites)
     uint32_t* page;
     uint32_t* q;
     FoaCache* cache;
@@ -638,7 +738,7 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
             *sm.ed = a.edits ? make_editor(a.edits[idx]) : a.one;
             ctl->ed = *sm.ed;
             for (uint32_t L = 0; L < HD_MAX_DEPTH; L++)
-                ctl->count[L] = 0;
+                ctl->count[L] = ctl->ncand[L] = ctl->nruns[L] = 0;
             ctl->count[0] = 1;
             const Level l0 = a.lv[0];
             l0.x[0] = 0;
@@ -695,20 +795,31 @@ HD_D void finish_edit(const Table& t, const PArgs& a)
 // the end of an edit, the start of the next) until the grid is needed
 // (ctl->phase / ctl->level) or the batch stops (ctl->stop).
 template <int PW>
-HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L, const Smem& sm)
+HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L, const Smem& sm, const uint32_t& nbar)
 {
     Ctl* ctl = a.ctl;
     const uint32_t G = gridDim.x, leafl = t.g.leaf_level;
     const uint32_t warp = threadIdx.x >> 5;
+    __shared__ bool meet;
+    const unsigned long long t_in = now_ns();
     for (;;) {
         if (ls == kLsFinish) {
-            // the edit ends; the grid meets once per edit, so that no wait at
-            // a barrier spans more than one edit of CTA 0's work
+            // the edit ends; the next one begins at once when every other CTA
+            // already waits at the coming barrier (it reads no more of this
+            // edit's state) and has not waited a good part of its bound
             finish_edit(t, a);
-            if (threadIdx.x == 0)
+            if (threadIdx.x == 0) {
+                const unsigned long long set_ns = __ldcg(&ctl->wait_ns);
                 ctl->phase = kPhNone;
+                meet = int32_t(ld_acquire(&ctl->arrived) - (nbar * G + G - 1)) < 0 ||
+                       now_ns() - t_in > (set_ns ? set_ns : kWaitNs) / 16;
+            }
             __syncthreads();
-            return;
+            const bool m = meet;
+            __syncthreads();
+            if (m)
+                return;
+            ls = kLsBegin;
         }
         if (ls == kLsBegin) {
             if (!begin_edit(t, a, sm))
@@ -799,18 +910,25 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
                 }
                 candidates_range(t, a.lv, L, deepest, 0, n, a.keys, a.vals);
                 __syncthreads();
-                const uint32_t runs = small_sort(t, L, n, a.keys, a.vals, sm.s64, sm.sm32, sm.sk, sm.sv);
-                if (runs > 2 * kPWarps) {
+                const uint32_t runs = small_sort(t, L, n, a.keys, a.vals, sm.s64, sm.sm32, sm.sk, sm.sv, sm.rs);
+                if (runs > kLocalRuns) {
                     // many buckets: the grid resolves them
+                    if (threadIdx.x < n) {
+                        a.keys[threadIdx.x] = sm.sk[threadIdx.x];
+                        a.vals[threadIdx.x] = sm.sv[threadIdx.x];
+                    }
+                    for (uint32_t r = threadIdx.x; r <= runs; r += kPT)
+                        a.keys2[r] = sm.rs[r];
                     if (threadIdx.x == 0) {
                         ctl->phase = kPhGridFoa;
                         ctl->level = L;
+                        ctl->n_small_runs = runs;
                     }
                     __syncthreads();
                     return;
                 }
-                foa_sorted<PW, true>(t, L, a.lv[L], sm.sk, sm.sv, n, warp, kPWarps, sm.page + warp * kPage,
-                               sm.q + warp * 12, sm.cache[warp], ctr);
+                foa_runs<PW>(t, L, a.lv[L], sm.sk, sm.sv, sm.rs, runs, warp, kPWarps, sm.page + warp * kPage,
+                             sm.q + warp * kFoaQuery, sm.cache[warp], ctr);
                 // the CTA barrier makes this level's results (lv.res, appended
                 // nodes) visible to CTA 0's next level; the grid barrier
                 // (a CTA barrier, then a fence by its thread 0) to the grid
@@ -842,10 +960,11 @@ __global__ void __launch_bounds__(kPT, 1)
     Smem sm;
     sm.page = reinterpret_cast<uint32_t*>(smem_raw);
     sm.q = sm.page + kPWarps * kPage;
-    sm.cache = reinterpret_cast<FoaCache*>(sm.q + kPWarps * 12);
+    sm.cache = reinterpret_cast<FoaCache*>(sm.q + kPWarps * kFoaQuery);
     sm.s64 = reinterpret_cast<unsigned long long*>(smem_raw);
     sm.sk = reinterpret_cast<uint32_t*>(smem_raw + persist_smem_core());
     sm.sv = sm.sk + kPT;
+    sm.rs = sm.sv + kPT;
     sm.list = sm.page;
     sm.sm32 = sm32;
     sm.ed = &ed_s;
@@ -861,7 +980,7 @@ __global__ void __launch_bounds__(kPT, 1)
     __syncthreads();
     for (;;) {
         if (cta == 0) {
-            local_advance<PW>(t, a, ls, L, sm);
+            local_advance<PW>(t, a, ls, L, sm, nbar);
             if (threadIdx.x == 0) // the command of the coming barrier
                 ctl->cmd[(nbar + 1) & 1] = Cmd{ctl->stop, ctl->phase, ctl->level, ctl->deepest, ctl->idx, {0, 0, 0}};
         }
@@ -943,9 +1062,8 @@ __global__ void __launch_bounds__(kPT, 1)
         }
         if (phase == kPhGridFoa) {
             // a small level's sorted candidates in many buckets
-            const uint32_t n = __ldcg(&ctl->count[L]);
-            foa_sorted<PW>(t, L, a.lv[L], a.keys, a.vals, n, cta * kPWarps + warp, G * kPWarps,
-                           sm.page + warp * kPage, sm.q + warp * 12, sm.cache[warp], ctr);
+            foa_runs<PW>(t, L, a.lv[L], a.keys, a.vals, a.keys2, __ldcg(&ctl->n_small_runs), warp * G + cta,
+                         G * kPWarps, sm.page + warp * kPage, sm.q + warp * kFoaQuery, sm.cache[warp], ctr);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             if (L == 0) {
@@ -973,8 +1091,15 @@ __global__ void __launch_bounds__(kPT, 1)
                 __syncthreads();
                 const uint32_t i0 = cta * chunk, i1 = min(n, i0 + chunk);
                 candidates_range(t, a.lv, L, deepest, i0, i1, a.keys, a.vals);
-                for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPT)
-                    atomicAdd(&cnt[a.keys[i] & (nd - 1)], 1u);
+                uint32_t mine = 0;
+                for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPT) {
+                    const uint32_t key = a.keys[i];
+                    atomicAdd(&cnt[key & (nd - 1)], 1u);
+                    mine += key < t.g.buckets(L);
+                }
+                mine = __reduce_add_sync(0xffffffffu, mine);
+                if ((threadIdx.x & 31) == 0 && mine)
+                    atomicAdd(&ctl->ncand[L], mine);
                 __syncthreads();
                 for (uint32_t d = threadIdx.x; d < nd; d += kPT)
                     a.hist[d * nb + cta] = cnt[d];
@@ -1002,10 +1127,25 @@ __global__ void __launch_bounds__(kPT, 1)
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             // 6. find-or-add, one warp per bucket run
-            foa_sorted<PW>(t, L, a.lv[L], a.keys, a.vals, n, cta * kPWarps + warp, G * kPWarps,
-                           sm.page + warp * kPage, sm.q + warp * 12, sm.cache[warp], ctr);
+            const uint32_t ncand = __ldcg(&ctl->ncand[L]);
+            Repeats rep{};
+            if (ncand >= kRepeatLevel) {
+                const uint32_t part = chunk_len(ncand, G, 32);
+                const uint32_t p0 = min(ncand, cta * part), p1 = min(ncand, p0 + part);
+                mark_repeats(a.lv[L], a.keys, a.vals, ncand, p0, p1, a.same);
+                if (!grid_sync(ctl, t.error, nbar))
+                    return;
+                rep = Repeats{a.same, (ncand + 31) / 32, a.runs, &ctl->nruns[L]};
+            }
+            foa_sorted<PW>(t, L, a.lv[L], a.keys, a.vals, ncand, cta * kPWarps + warp, G * kPWarps,
+                           sm.page + warp * kPage, sm.q + warp * kFoaQuery, sm.cache[warp], ctr, rep);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
+            if (const uint32_t nr = __ldcg(&ctl->nruns[L])) {
+                fill_runs(a.lv[L], a.vals, a.runs, nr);
+                if (!grid_sync(ctl, t.error, nbar))
+                    return;
+            }
             if (L == 0)
                 break; // (level 0 holds one entry: never big)
             L--;
@@ -1018,7 +1158,7 @@ __global__ void __launch_bounds__(kPT, 1)
 
 // ---- host side --------------------------------------------------------------------
 
-static size_t persist_smem() { return persist_smem_core() + size_t(kPT) * 4 * 2; }
+static size_t persist_smem() { return persist_smem_core() + size_t(kPT) * 4 * 3 + 16; }
 
 template <int PW>
 static const void* persist_kernel()
@@ -1071,6 +1211,11 @@ PArgs persist_args(hd_ctx* c, const PersistLevels& pl, uint32_t grid, uint32_t n
     a.hist2 = s.get<uint32_t>("ep_hist2", uint64_t(kDigits) * grid);
     a.rows = s.get<uint32_t>("ep_rows", kDigits);
     a.rows2 = s.get<uint32_t>("ep_rows2", kDigits);
+    uint64_t most = 1;
+    for (uint32_t L = 0; L <= c->g.leaf_level; L++)
+        most = std::max<uint64_t>(most, pl.caps[L]);
+    a.same = s.get<uint32_t>("ep_same", most / 32 + 1);
+    a.runs = s.get<FollowerRun>("ep_runs", most / kLongRun + 1);
     a.d_root = c->d_root;
     return a;
 }

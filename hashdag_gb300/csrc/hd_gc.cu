@@ -321,7 +321,7 @@ __global__ void k_gc_write(Table t, uint32_t level, const uint32_t* __restrict__
         for (uint32_t k = 0; k < 9; k++)
             if (k < words)
                 dst[k] = c[k];
-        bloom_add(t, v, bloom_bits(c, words));
+        bloom_add(t, v, bloom_bits(c, words), leaf);
     }
 }
 
@@ -360,8 +360,8 @@ __global__ void k_zero_pages(Table t, uint32_t from, uint32_t to)
     {
         const uint32_t p = t.free_phys[from + uint32_t(i / kPage)];
         t.pool[uint64_t(p) * kPage + (i % kPage)] = 0;
-        if (i % kPage < kBloomWords)
-            t.bloom[uint64_t(p) * kBloomWords + (i % kPage)] = 0;
+        if (i % kPage < kPageMeta)
+            t.meta[uint64_t(p) * kPageMeta + (i % kPage)] = 0;
     }
 }
 

@@ -50,7 +50,7 @@ __global__ void k_add_full_nodes(Table t, uint32_t first_level, uint32_t last_le
         uint32_t* dst = t.sys_rw(v);
         for (uint32_t i = 0; i < n; i++)
             dst[i] = node[i];
-        bloom_add(t, v, bloom_bits(node, n));
+        bloom_add(t, v, bloom_bits(node, n), leaf);
         *size_ptr = size;
         t.level_nodes[level] += 1;
         t.full_nodes[level] = v;
@@ -109,7 +109,7 @@ void table_reset(hd_ctx* c)
 {
     const Geom& g = c->g;
     HD_CUDA(cudaMemsetAsync(c->t.pool, 0, size_t(g.pool_pages) * kPage * 4 + 64, c->stream));
-    HD_CUDA(cudaMemsetAsync(c->t.bloom, 0, size_t(g.pool_pages) * kBloomWords * 4, c->stream));
+    HD_CUDA(cudaMemsetAsync(c->t.meta, 0, size_t(g.pool_pages) * kPageMeta * 4, c->stream));
     HD_CUDA(cudaMemsetAsync(c->t.page_table, 0, kPageTableEntries * 4, c->stream));
     if (c->t.direct)
         HD_CUDA(cudaMemsetAsync(c->t.page_ids, 0, g.total_vpages * 4, c->stream));
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(32 * kAppendWarps)
             uint32_t* dst = t.sys_rw(v);
             for (uint32_t k = 0; k < n; k++)
                 dst[k] = src[k];
-            bloom_add(t, v, bloom_bits(src, n));
+            bloom_add(t, v, bloom_bits(src, n), leaf);
             out_addr[r] = v;
         }
         __syncwarp();
@@ -457,7 +457,8 @@ void import_basic_dag(hd_ctx* c, const uint32_t* d_words, uint64_t n_words)
 // by walking every bucket the way the scans do: leaves two words apart,
 // interior nodes by their sizes from each page's start.  Words past a page's
 // last node (the gap a node that did not fit leaves) are walked as nodes too,
-// which only adds bits, so a filter never misses a node it holds.
+// which only adds bits, so a filter never misses a node it holds (and starts
+// only words on the scans' walk).
 __global__ void k_bloom_rebuild(Table t, uint32_t level)
 {
     const Geom& g = t.g;
@@ -473,7 +474,7 @@ __global__ void k_bloom_rebuild(Table t, uint32_t level)
                 const uint32_t n = leaf ? 2 : total_size(page[w]);
                 if (w + n > used)
                     break;
-                bloom_add(t, vbase + pindex + w, bloom_bits(page + w, n));
+                bloom_add(t, vbase + pindex + w, bloom_bits(page + w, n), leaf);
                 w += n;
             }
         }
@@ -506,7 +507,7 @@ void check_table(const Geom& g, const uint32_t* pt, const uint32_t* bs, uint32_t
 void bloom_rebuild(hd_ctx* c)
 {
     const Geom& g = c->g;
-    HD_CUDA(cudaMemsetAsync(c->t.bloom, 0, size_t(g.pool_pages) * kBloomWords * 4, c->stream));
+    HD_CUDA(cudaMemsetAsync(c->t.meta, 0, size_t(g.pool_pages) * kPageMeta * 4, c->stream));
     for (uint32_t L = 0; L <= g.leaf_level; L++) {
         k_bloom_rebuild<<<grid_for(g.buckets(L), 128), 128, 0, c->stream>>>(c->t, L);
         HD_LAUNCH_CHECK();
@@ -518,9 +519,11 @@ __global__ void k_bloom_clear_level(Table t, uint32_t vp0, uint32_t vp1)
     HD_GRID_STRIDE(i, uint64_t(vp1 - vp0))
     {
         const uint32_t p = t.page_table[vp0 + i];
-        if (p)
-            for (uint32_t k = 0; k < kBloomWords; k++)
-                t.bloom[uint64_t(p) * kBloomWords + k] = 0;
+        if (p) {
+            uint4* line = reinterpret_cast<uint4*>(t.meta + uint64_t(p) * kPageMeta);
+            for (uint32_t k = 0; k < kPageMeta / 4; k++)
+                line[k] = make_uint4(0, 0, 0, 0);
+        }
     }
 }
 

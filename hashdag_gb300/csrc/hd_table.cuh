@@ -82,54 +82,34 @@ HD_D bool map_pages(const Table& t, uint32_t level, uint32_t bucket, uint32_t fr
     return true;
 }
 
-// The filter of the physical page behind virtual word v
-HD_D uint32_t* bloom_of(const Table& t, uint32_t v)
+// Adds a node written at word `word` of physical page p to the page's line.
+HD_D void bloom_add_phys(const Table& t, uint32_t p, uint32_t word, uint32_t bits, bool leaf)
 {
-    return t.bloom + uint64_t(t.page_cg(v >> kPageShift)) * kBloomWords;
-}
-// Adds a node written at virtual word v to its page's filter
-HD_D void bloom_add(const Table& t, uint32_t v, uint32_t bits)
-{
-    uint32_t* f = bloom_of(t, v);
+    uint32_t* f = t.meta + uint64_t(p) * kPageMeta;
 #pragma unroll
     for (uint32_t i = 0; i < kBloomHashes; i++) {
-        const uint32_t b = bloom_pos(bits, i);
+        const uint32_t b = bloom_pos(bits, i, leaf);
         atomicOr(f + (b >> 5), 1u << (b & 31));
     }
+    if (!leaf)
+        atomicOr(f + kPageStarts + (word >> 5), 1u << (word & 31));
 }
-// Adds a node written into physical page p to the page's filter
-HD_D void bloom_add_phys(const Table& t, uint32_t p, uint32_t bits)
+// Adds a node written at virtual word v to its page's line
+HD_D void bloom_add(const Table& t, uint32_t v, uint32_t bits, bool leaf)
 {
-    uint32_t* f = t.bloom + uint64_t(p) * kBloomWords;
-#pragma unroll
-    for (uint32_t i = 0; i < kBloomHashes; i++) {
-        const uint32_t b = bloom_pos(bits, i);
-        atomicOr(f + (b >> 5), 1u << (b & 31));
-    }
+    bloom_add_phys(t, t.page_cg(v >> kPageShift), v & (kPage - 1), bits, leaf);
 }
 // False when physical page p's filter rules the node out
-HD_D bool bloom_may_phys(const Table& t, uint32_t p, uint32_t bits)
+HD_D bool bloom_may_phys(const Table& t, uint32_t p, uint32_t bits, bool leaf)
 {
-    const uint32_t* f = t.bloom + uint64_t(p) * kBloomWords;
-    bool may = true;
+    const uint32_t* f = t.meta + uint64_t(p) * kPageMeta;
+    uint32_t may = 1;
 #pragma unroll
     for (uint32_t i = 0; i < kBloomHashes; i++) {
-        const uint32_t b = bloom_pos(bits, i);
-        may &= ((__ldcg(f + (b >> 5)) >> (b & 31)) & 1u) != 0;
+        const uint32_t b = bloom_pos(bits, i, leaf);
+        may &= __ldcg(f + (b >> 5)) >> (b & 31);
     }
-    return may;
-}
-// False when the page behind virtual word v cannot hold the node
-HD_D bool bloom_may(const Table& t, uint32_t v, uint32_t bits)
-{
-    const uint32_t* f = bloom_of(t, v);
-    bool may = true;
-#pragma unroll
-    for (uint32_t i = 0; i < kBloomHashes; i++) {
-        const uint32_t b = bloom_pos(bits, i);
-        may &= ((__ldcg(f + (b >> 5)) >> (b & 31)) & 1u) != 0;
-    }
-    return may;
+    return may & 1u;
 }
 
 // Pushes item i onto the list of bucket gb; the first item of a bucket also
