@@ -200,6 +200,78 @@ HD_D bool inside_tool(const Editor& e, float mnx, float mny, float mnz, float mx
 // filter bits and at kRowSize its word count; 16-byte aligned.
 constexpr uint32_t kRow = 12, kRowBloom = 9, kRowSize = 10;
 
+// The voxels of the 4^3 leaf at (x0, y0, z0) whose cubes should_edit_impl
+// takes, as leaf bits.  Its terms are per axis, so they are made for the 4
+// voxel slabs of each axis: a box is an and of three slab masks, and a sphere
+// 64 sums of three squares in should_edit_impl's order (a slab the centre
+// lies in takes nothing away).  The leaf level's evaluation, a thread a leaf,
+// was bound by 64 whole tests: the children of a level (spawned, classified,
+// leaves evaluated) went from 12.4 to 7.9 us for 4,816 of them, from 28 to 10
+// us for 184,528.
+HD_D uint64_t leaf_edit_mask(const Editor& e, uint32_t x0, uint32_t y0, uint32_t z0)
+{
+    if (e.sphere()) {
+        float sx[4], sy[4], sz[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const float mnx = float(x0 + k), mny = float(y0 + k), mnz = float(z0 + k);
+            const float mxx = mnx + 1.0f, mxy = mny + 1.0f, mxz = mnz + 1.0f;
+            sx[k] = e.cx < mnx ? sqr(e.cx - mnx) : e.cx > mxx ? sqr(e.cx - mxx) : 0.0f;
+            sy[k] = e.cy < mny ? sqr(e.cy - mny) : e.cy > mxy ? sqr(e.cy - mxy) : 0.0f;
+            sz[k] = e.cz < mnz ? sqr(e.cz - mnz) : e.cz > mxz ? sqr(e.cz - mxz) : 0.0f;
+        }
+        uint32_t half[2] = {0, 0};
+#pragma unroll
+        for (uint32_t b = 0; b < 64; b++) {
+            const uint32_t c1 = b >> 3, c2 = b & 7;
+            const float d = ((e.r2 - sx[((c1 >> 2) & 1) * 2 + ((c2 >> 2) & 1)]) -
+                             sy[((c1 >> 1) & 1) * 2 + ((c2 >> 1) & 1)]) -
+                            sz[(c1 & 1) * 2 + (c2 & 1)];
+            half[b >> 5] |= (d > 0 ? 1u : 0u) << (b & 31);
+        }
+        return uint64_t(half[0]) | (uint64_t(half[1]) << 32);
+    }
+    auto taken = [](float lo, float hi, float mn) {
+        const float mx = mn + 1.0f;
+        return !(lo >= mx || hi <= mn || mn >= hi || mx <= lo);
+    };
+    uint64_t mx = 0, my = 0, mz = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+        // slab k of an axis: the half of the 2^3 blocks (bytes) and of the
+        // voxels in a block (bits of a byte)
+        mx |= taken(e.bminx, e.bmaxx, float(x0 + k)) ? ((k & 2) ? 0xFFFFFFFF00000000ull : 0x00000000FFFFFFFFull) &
+                                                           ((k & 1) ? 0xF0F0F0F0F0F0F0F0ull : 0x0F0F0F0F0F0F0F0Full)
+                                                     : 0ull;
+        my |= taken(e.bminy, e.bmaxy, float(y0 + k)) ? ((k & 2) ? 0xFFFF0000FFFF0000ull : 0x0000FFFF0000FFFFull) &
+                                                           ((k & 1) ? 0xCCCCCCCCCCCCCCCCull : 0x3333333333333333ull)
+                                                     : 0ull;
+        mz |= taken(e.bminz, e.bmaxz, float(z0 + k)) ? ((k & 2) ? 0xFF00FF00FF00FF00ull : 0x00FF00FF00FF00FFull) &
+                                                           ((k & 1) ? 0xAAAAAAAAAAAAAAAAull : 0x5555555555555555ull)
+                                                     : 0ull;
+    }
+    return mx & my & mz;
+}
+
+// The leaf after the tool: get_new_value of its edited voxels.
+HD_D uint64_t edited_leaf(const Editor& e, uint32_t x0, uint32_t y0, uint32_t z0, uint64_t leaf, uint64_t edited)
+{
+    if (e.shortcuts()) // sphere and box carve / fill: the same value everywhere
+        return e.adding() ? (leaf | edited) : (leaf & ~edited);
+    if (e.tool == HD_TOOL_SPHERE_PAINT)
+        return leaf;
+    uint64_t out = leaf;
+    for (uint64_t todo = edited; todo; todo &= todo - 1) {
+        const uint32_t b = __ffsll((long long)todo) - 1, c1 = b >> 3, c2 = b & 7;
+        const float px = float(x0 + ((c1 >> 2) & 1) * 2 + ((c2 >> 2) & 1));
+        const float py = float(y0 + ((c1 >> 1) & 1) * 2 + ((c2 >> 1) & 1));
+        const float pz = float(z0 + (c1 & 1) * 2 + (c2 & 1));
+        const uint64_t bit = 1ull << b;
+        out = new_value(e, px, py, pz, (leaf & bit) != 0) ? (out | bit) : (out & ~bit);
+    }
+    return out;
+}
+
 // ---- per-level entry state ---------------------------------------------------
 enum : uint8_t {
     kSkip = 0,      // level-C_colorTreeLevels child the parent never hands to edit_leaf
@@ -307,20 +379,9 @@ HD_D void classify_values(const Table& t, const Editor& ed, uint32_t level, cons
                     const NodeRead<CG> p(t, old);
                     leaf = uint64_t(p[0]) | (uint64_t(p[1]) << 32);
                 }
-                const uint32_t x0 = x << 2, y0 = y << 2, z0 = z << 2;
-                uint32_t edited = 0;
-                for (uint32_t c1 = 0; c1 < 8; c1++)
-                    for (uint32_t c2 = 0; c2 < 8; c2++) {
-                        const float px = float(x0 + ((c1 >> 2) & 1) * 2 + ((c2 >> 2) & 1));
-                        const float py = float(y0 + ((c1 >> 1) & 1) * 2 + ((c2 >> 1) & 1));
-                        const float pz = float(z0 + (c1 & 1) * 2 + (c2 & 1));
-                        if (should_edit_impl(ed, px, py, pz, px + 1.0f, py + 1.0f, pz + 1.0f)) {
-                            edited++;
-                            const uint64_t bit = 1ull << (c1 * 8 + c2);
-                            leaf = new_value(ed, px, py, pz, (leaf & bit) != 0) ? (leaf | bit) : (leaf & ~bit);
-                        }
-                    }
-                voxels = edited;
+                const uint64_t edited = leaf_edit_mask(ed, x << 2, y << 2, z << 2);
+                voxels = popc64(edited);
+                leaf = edited_leaf(ed, x << 2, y << 2, z << 2, leaf, edited);
                 lv.leaf[i] = leaf;
             } else {
                 state = kDescend;
@@ -897,22 +958,38 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
             }
             foa += e1 - j;
             j = e1;
-        } else if (!appended) {
+        } else if (!appended && j < j1) {
+            // 128 candidates at a time, their reads independent
+            const uint4* p = reinterpret_cast<const uint4*>(q);
             for (;;) {
-                const uint32_t jj = j + lane;
-                bool same = jj < j1;
-                if (same) {
-                    const uint4* c = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(vals[jj]));
-                    const uint4* p = reinterpret_cast<const uint4*>(q);
-                    same = same_words(c[0], p[0]) && same_words(c[1], p[1]) && c[2].x == p[2].x;
+                uint32_t entry[4];
+                bool same[4];
+#pragma unroll
+                for (uint32_t m = 0; m < 4; m++) {
+                    const uint32_t jj = j + 32 * m + lane;
+                    entry[m] = jj < j1 ? vals[jj] : kNotFound;
                 }
-                const uint32_t b = __ballot_sync(0xffffffffu, same);
-                const uint32_t run = b == 0xffffffffu ? 32u : __ffs(~b) - 1;
-                if (lane < run)
-                    lv.res[vals[jj]] = vbase + result;
+#pragma unroll
+                for (uint32_t m = 0; m < 4; m++) {
+                    same[m] = entry[m] != kNotFound;
+                    if (same[m]) {
+                        const uint4* c = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(entry[m]));
+                        same[m] = same_words(c[0], p[0]) && same_words(c[1], p[1]) && c[2].x == p[2].x;
+                    }
+                }
+                uint32_t run = 128;
+#pragma unroll
+                for (int m = 3; m >= 0; m--) {
+                    const uint32_t diff = __ballot_sync(0xffffffffu, !same[m]);
+                    run = diff ? 32 * m + __ffs(diff) - 1 : run;
+                }
+#pragma unroll
+                for (uint32_t m = 0; m < 4; m++)
+                    if (32 * m + lane < run)
+                        lv.res[entry[m]] = vbase + result;
                 foa += run;
                 j += run;
-                if (run < 32)
+                if (run < 128)
                     break;
             }
         }

@@ -534,13 +534,31 @@ HD_D void mark_repeats(const Level& lv, const uint32_t* keys, const uint32_t* va
     }
 }
 
-// The results of the long runs of repeats, by every thread of the grid.
+// The results of the long runs of repeats, by every warp of the grid: pieces
+// of kPiece positions dealt out over all the runs (32 runs at a time: a lane
+// holds one, its pieces counted by a prefix sum).
 HD_D void fill_runs(const Level& lv, const uint32_t* vals, const FollowerRun* runs, uint32_t n)
 {
-    for (uint32_t r = 0; r < n; r++) {
-        const uint4 x = __ldcg(reinterpret_cast<const uint4*>(runs + r));
-        for (uint32_t j = x.x + blockIdx.x * kPT + threadIdx.x; j < x.y; j += gridDim.x * kPT)
-            lv.res[__ldcg(vals + j)] = x.z;
+    constexpr uint32_t kPiece = 256;
+    const uint32_t lane = threadIdx.x & 31, nw = gridDim.x * kPWarps;
+    const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (uint32_t r0 = 0; r0 < n; r0 += 32) {
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (r0 + lane < n)
+            x = __ldcg(reinterpret_cast<const uint4*>(runs + r0 + lane));
+        const uint32_t end = warp_incl_scan((x.y - x.x + kPiece - 1) / kPiece); // pieces up to this run's last
+        const uint32_t all = __shfl_sync(0xffffffffu, end, 31);
+        for (uint32_t p = gw; p < all; p += nw) {
+            const uint32_t r = __popc(__ballot_sync(0xffffffffu, end <= p)); // the run of piece p
+            const uint32_t before = r ? __shfl_sync(0xffffffffu, end, r - 1) : 0u;
+            const uint32_t b = __shfl_sync(0xffffffffu, x.x, r) + (p - before) * kPiece;
+            const uint32_t e = min(b + kPiece, __shfl_sync(0xffffffffu, x.y, r));
+            const uint32_t result = __shfl_sync(0xffffffffu, x.z, r);
+#pragma unroll
+            for (uint32_t k = 0; k < kPiece; k += 32)
+                if (b + k + lane < e)
+                    lv.res[__ldcg(vals + b + k + lane)] = result;
+        }
     }
 }
 
@@ -640,12 +658,15 @@ HD_D void scan_rows(uint32_t* hist, uint32_t nb, uint32_t nd, uint32_t* rows)
 
 // Stable scatter of chunk `cb` of (keys, vals) by digit (key >> shift) & (nd
 // - 1): bases from the row totals and this chunk's row offsets; warps of a
-// tile take their turn in order.  With hist_next, counts each element's next
-// digit in the chunk its output position falls in.
+// tile take their turn in order.  Keys of `empty` and above are left out.
+// With hist_next, counts each element's next digit in the chunk (of chunk_next
+// positions, nb_next of them) its output position falls in, equal ones of a
+// warp with one atomic.  (Entries resolved at once, keyed `empty`, were sorted
+// along and met in one counter: 55 us of a level of 184,528 entries, now 24.)
 HD_D void scatter_chunk(const uint32_t* keys, const uint32_t* vals, uint32_t n, uint32_t nb, uint32_t cb,
-                        uint32_t shift, uint32_t nd, const uint32_t* hist, const uint32_t* rows,
+                        uint32_t shift, uint32_t nd, uint32_t empty, const uint32_t* hist, const uint32_t* rows,
                         uint32_t* keys_out, uint32_t* vals_out, uint32_t* hist_next, uint32_t next_shift,
-                        uint32_t* run, uint32_t* sm32)
+                        uint32_t nb_next, uint32_t chunk_next, uint32_t* run, uint32_t* sm32)
 {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
@@ -663,13 +684,14 @@ HD_D void scatter_chunk(const uint32_t* keys, const uint32_t* vals, uint32_t n, 
     const uint32_t i0 = cb * chunk, i1 = min(n, i0 + chunk);
     for (uint32_t base = i0; base < i1; base += kPT) {
         const uint32_t i = base + threadIdx.x;
-        const bool valid = i < i1;
-        const uint32_t key = valid ? __ldcg(keys + i) : 0u;
-        const uint32_t val = valid ? __ldcg(vals + i) : 0u;
+        const uint32_t key = i < i1 ? __ldcg(keys + i) : empty;
+        const uint32_t val = i < i1 ? __ldcg(vals + i) : 0u;
+        const bool valid = key < empty;
         const uint32_t digit = valid ? (key >> shift) & (nd - 1) : kDigits + lane;
         const uint32_t peers = __match_any_sync(0xffffffffu, digit);
         const uint32_t leader = __ffs(peers) - 1;
-        for (uint32_t w = 0; w < kPWarps; w++) {
+        const uint32_t turns = min(kPWarps, (i1 - base + 31) / 32);
+        for (uint32_t w = 0; w < turns; w++) {
             if (warp == w) {
                 uint32_t b = 0;
                 if (valid && lane == leader) {
@@ -677,12 +699,17 @@ HD_D void scatter_chunk(const uint32_t* keys, const uint32_t* vals, uint32_t n, 
                     run[digit] = b + __popc(peers);
                 }
                 b = __shfl_sync(0xffffffffu, b, leader);
+                const uint32_t pos = b + __popc(peers & lt);
                 if (valid) {
-                    const uint32_t pos = b + __popc(peers & lt);
                     keys_out[pos] = key;
                     vals_out[pos] = val;
-                    if (hist_next)
-                        atomicAdd(hist_next + ((key >> next_shift) & (nd - 1)) * nb + pos / chunk, 1u);
+                }
+                if (hist_next) {
+                    const uint32_t at = valid ? ((key >> next_shift) & (nd - 1)) * nb_next + pos / chunk_next
+                                              : 0x80000000u + lane;
+                    const uint32_t same = __match_any_sync(0xffffffffu, at);
+                    if (valid && lane == uint32_t(__ffs(same) - 1))
+                        atomicAdd(hist_next + at, uint32_t(__popc(same)));
                 }
             }
             __syncthreads();
@@ -1082,6 +1109,7 @@ __global__ void __launch_bounds__(kPT, 1)
             while ((1u << key_bits) <= t.g.buckets(L))
                 key_bits++;
             const uint32_t dbits = (key_bits + 1) / 2, nd = 1u << dbits;
+            const uint32_t empty = t.g.buckets(L);
             // 1. candidates and their pass-1 digit counts
             if (cta < nb) {
                 for (uint32_t d = threadIdx.x; d < nd; d += kPT) {
@@ -1094,8 +1122,10 @@ __global__ void __launch_bounds__(kPT, 1)
                 uint32_t mine = 0;
                 for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPT) {
                     const uint32_t key = a.keys[i];
-                    atomicAdd(&cnt[key & (nd - 1)], 1u);
-                    mine += key < t.g.buckets(L);
+                    if (key < empty) {
+                        atomicAdd(&cnt[key & (nd - 1)], 1u);
+                        mine++;
+                    }
                 }
                 mine = __reduce_add_sync(0xffffffffu, mine);
                 if ((threadIdx.x & 31) == 0 && mine)
@@ -1106,28 +1136,31 @@ __global__ void __launch_bounds__(kPT, 1)
             }
             if (!grid_sync(ctl, t.error, nbar))
                 return;
+            // the second pass and the find-or-add: candidates only
+            const uint32_t ncand = __ldcg(&ctl->ncand[L]);
+            const uint32_t nb2 = max(1u, min(G, (ncand + kChunkAlign - 1) / kChunkAlign));
+            const uint32_t chunk2 = max(kChunkAlign, chunk_len(ncand, nb2, kChunkAlign));
             // 2. pass-1 rows
             scan_rows(a.hist, nb, nd, a.rows);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             // 3. pass-1 scatter, pass-2 counts
             if (cta < nb)
-                scatter_chunk(a.keys, a.vals, n, nb, cta, 0, nd, a.hist, a.rows, a.keys2, a.vals2, a.hist2, dbits,
-                              run, sm32);
+                scatter_chunk(a.keys, a.vals, n, nb, cta, 0, nd, empty, a.hist, a.rows, a.keys2, a.vals2, a.hist2,
+                              dbits, nb2, chunk2, run, sm32);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             // 4. pass-2 rows
-            scan_rows(a.hist2, nb, nd, a.rows2);
+            scan_rows(a.hist2, nb2, nd, a.rows2);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             // 5. pass-2 scatter
-            if (cta < nb)
-                scatter_chunk(a.keys2, a.vals2, n, nb, cta, dbits, nd, a.hist2, a.rows2, a.keys, a.vals, nullptr, 0,
-                              run, sm32);
+            if (cta < nb2)
+                scatter_chunk(a.keys2, a.vals2, ncand, nb2, cta, dbits, nd, empty, a.hist2, a.rows2, a.keys, a.vals,
+                              nullptr, 0, 0, 0, run, sm32);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             // 6. find-or-add, one warp per bucket run
-            const uint32_t ncand = __ldcg(&ctl->ncand[L]);
             Repeats rep{};
             if (ncand >= kRepeatLevel) {
                 const uint32_t part = chunk_len(ncand, G, 32);
