@@ -565,6 +565,16 @@ HD_D bool same_words(const uint4& a, const uint4& b)
 {
     return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
 }
+// The same words in two candidates' rows of a level
+HD_D bool same_row(const uint32_t* a, const uint32_t* b, bool leaf)
+{
+    if (leaf) {
+        const uint2 x = *reinterpret_cast<const uint2*>(a), y = *reinterpret_cast<const uint2*>(b);
+        return x.x == y.x && x.y == y.y;
+    }
+    const uint4 *p = reinterpret_cast<const uint4*>(a), *q = reinterpret_cast<const uint4*>(b);
+    return same_words(p[0], q[0]) && same_words(p[1], q[1]) && p[2].x == q[2].x;
+}
 
 // One warp per bucket: the bucket's candidates, in depth-first order, each
 // resolved against the bucket as it stands (earlier candidates' appends
@@ -579,7 +589,7 @@ constexpr uint32_t kCachePos = 3;
 
 struct FoaCache {
     uint32_t words[kCache][9];
-    uint32_t n[kCache];
+    uint32_t bloom[kCache]; // the words' filter bits: looked at first
     uint32_t npos[kCache];
     uint32_t pos[kCache][kCachePos];
 };
@@ -697,9 +707,10 @@ HD_D uint32_t match_page(const uint32_t (&v)[kPage / 32], const uint32_t* page, 
     return best;
 }
 
-// Words of a warp's query buffer: the candidate's row, then the start bits of
-// the page being scanned.
-constexpr uint32_t kFoaQuery = kRow + 16;
+// Words of a warp's query buffer: the rows of kRowsAhead candidates, then the
+// start bits of the page being scanned.
+constexpr uint32_t kRowsAhead = 8;
+constexpr uint32_t kFoaQuery = kRow * kRowsAhead + 16;
 
 // Warp-wide scan of the bucket for the first compared position holding q
 // (find_leaf_node_in_bucket / find_interior_node_in_bucket); returns the
@@ -711,12 +722,11 @@ constexpr uint32_t kFoaQuery = kRow + 16;
 // from shared memory 32 at a time, 53 buckets of a small level took 25 us;
 // with runs dealt out to the warps as well, 7.6.)
 template <int PW>
-HD_D uint32_t scan_bucket(const Table& t, uint32_t vbase, uint32_t S, uint32_t* q, uint32_t n, bool leaf, uint32_t may,
-                          uint32_t bloom, uint32_t pt_lane, uint32_t* page, uint32_t* last_match,
-                          unsigned long long& scanned)
+HD_D uint32_t scan_bucket(const Table& t, uint32_t vbase, uint32_t S, const uint32_t* q, uint32_t n, bool leaf,
+                          uint32_t may, uint32_t bloom, uint32_t pt_lane, uint32_t* page, uint32_t* starts,
+                          uint32_t* last_match, unsigned long long& scanned)
 {
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t* starts = q + kRow;
     uint32_t found = kNotFound, staged = kNotFound;
     *last_match = kNotFound;
     // page pi's physical page and whether its filter admits q: the first 32
@@ -831,58 +841,71 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
     uint32_t used_entries = 0, next_slot = 0;
     bool failed = false;
     uint32_t j = j0;
-    // the run's entry indices 32 at a time (lane k: entry of position vb + k)
-    // and the next candidate's row loaded while the current one resolves
-    uint32_t vb = j0, vreg = j0 + lane < j1 ? vals[j0 + lane] : 0u;
-    const uint32_t c0 = __shfl_sync(0xffffffffu, vreg, 0); // every lane: a full-warp shuffle
-    uint32_t qj = j0, qw = lane < kRow ? lv.cand[kRow * uint64_t(c0) + lane] : 0u;
+    // The rows of kRowsAhead candidates lie in shared memory (with the entry's
+    // index in a row's last word), the next kRowsAhead on their way in
+    // registers, so that the reads of a row wait for no candidate before it.
+    constexpr uint32_t kLoads = kRow * kRowsAhead / 32;
+    uint32_t ahead[kLoads], jb = j0, ja = j0;
+    uint32_t* starts = q + kRow * kRowsAhead;
+    auto load_rows = [&](uint32_t from) {
+#pragma unroll
+        for (uint32_t m = 0; m < kLoads; m++) {
+            const uint32_t k = lane + 32 * m, jj = from + k / kRow, w = k % kRow;
+            ahead[m] = 0;
+            if (jj < j1) {
+                const uint32_t entry = vals[jj];
+                ahead[m] = w == kRow - 1 ? entry : lv.cand[kRow * uint64_t(entry) + w];
+            }
+        }
+    };
+    load_rows(j0);
+    bool staged = false;
     while (j < j1 && !failed) {
-        if (j - vb >= 32) {
-            vb = j;
-            vreg = j + lane < j1 ? vals[j + lane] : 0u;
+        if (!staged || j >= jb + kRowsAhead) {
+            if (staged && j - ja >= kRowsAhead) { // a run of repeats was passed over
+                ja = j;
+                load_rows(ja);
+            }
+            __syncwarp();
+#pragma unroll
+            for (uint32_t m = 0; m < kLoads; m++)
+                q[lane + 32 * m] = ahead[m];
+            __syncwarp();
+            staged = true;
+            jb = ja;
+            ja = jb + kRowsAhead;
+            if (ja < j1)
+                load_rows(ja);
         }
-        const uint32_t ci = __shfl_sync(0xffffffffu, vreg, j - vb);
-        if (qj != j && lane < kRow)
-            qw = lv.cand[kRow * uint64_t(ci) + lane];
-        if (lane < kRow)
-            q[lane] = qw;
-        __syncwarp();
-        const uint32_t n = q[kRowSize], bloom = q[kRowBloom];
-        // the filters of the bucket's first 32 pages, a lane per page, beside
-        // the bucket size (they do not wait for it)
-        const uint32_t maybe = __ballot_sync(0xffffffffu, lane < cap_pages && bloom_may_phys(t, pt_lane, bloom, leaf));
-        // prefetch candidate j + 1 (its entry index is in vreg unless it
-        // starts the next group of 32)
-        qj = j + 1;
-        if (qj < j1 && qj - vb < 32) {
-            const uint32_t cn = __shfl_sync(0xffffffffu, vreg, qj - vb);
-            if (lane < kRow)
-                qw = lv.cand[kRow * uint64_t(cn) + lane];
-        } else {
-            qj = kNotFound;
+        const uint32_t* qj = q + kRow * (j - jb);
+        const uint32_t n = qj[kRowSize], bloom = qj[kRowBloom], ci = qj[kRow - 1];
+        // cache lookup: lane e compares entry e's filter bits, then the lanes
+        // a word each of an entry that has them
+        uint32_t hb = __ballot_sync(0xffffffffu, lane < used_entries && cache.bloom[lane] == bloom);
+        uint32_t e = kCache;
+        while (hb && e == kCache) {
+            const uint32_t k = __ffs(hb) - 1;
+            hb &= hb - 1;
+            if (__all_sync(0xffffffffu, lane >= 9 || cache.words[k][lane] == qj[lane]))
+                e = k;
         }
-        // cache lookup: lane e checks entry e
-        bool hit = lane < used_entries && cache.n[lane] == n;
-        if (hit)
-            for (uint32_t k = 0; k < n; k++)
-                hit &= cache.words[lane][k] == q[k];
-        const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-        uint32_t e;
-        if (hb) {
-            e = __ffs(hb) - 1;
-        } else {
+        if (e == kCache) {
+            // the filters of the bucket's first 32 pages, a lane per page,
+            // beside the bucket size (they do not wait for it)
+            const uint32_t maybe =
+                __ballot_sync(0xffffffffu, lane < cap_pages && bloom_may_phys(t, pt_lane, bloom, leaf));
             uint32_t last_match;
             const uint32_t npages = (S + kPage - 1) / kPage;
             const uint32_t may = npages < 32 ? maybe & ((1u << npages) - 1u) : maybe;
             const uint32_t f =
-                scan_bucket<PW>(t, vbase, S, q, n, leaf, may, bloom, pt_lane, page, &last_match, scanned);
+                scan_bucket<PW>(t, vbase, S, qj, n, leaf, may, bloom, pt_lane, page, starts, &last_match, scanned);
             e = next_slot;
             next_slot = (next_slot + 1) % kCache;
             used_entries = used_entries < kCache ? used_entries + 1 : kCache;
             if (lane < 9)
-                cache.words[e][lane] = q[lane];
+                cache.words[e][lane] = qj[lane];
             if (lane == 0) {
-                cache.n[e] = n;
+                cache.bloom[e] = bloom;
                 cache.npos[e] = 0;
                 if (f != kNotFound)
                     cache.pos[e][cache.npos[e]++] = f;
@@ -921,7 +944,7 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
                 const uint32_t near = __shfl_sync(0xffffffffu, pt_lane, (pos >> kPageShift) & 31);
                 const uint32_t phys = (pos >> kPageShift) < 32 ? near : t.page_cg(vpage0 + (pos >> kPageShift));
                 if (lane < n)
-                    __stcg(t.pool + (uint64_t(phys) << kPageShift) + (pos & (kPage - 1)) + lane, q[lane]);
+                    __stcg(t.pool + (uint64_t(phys) << kPageShift) + (pos & (kPage - 1)) + lane, qj[lane]);
                 if (lane == 0)
                     bloom_add_phys(t, phys, pos & (kPage - 1), bloom, leaf);
                 result = pos;
@@ -958,9 +981,10 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
             }
             foa += e1 - j;
             j = e1;
-        } else if (!appended && j < j1) {
-            // 128 candidates at a time, their reads independent
-            const uint4* p = reinterpret_cast<const uint4*>(q);
+        } else if (!appended && j < j1 &&
+                   (j - jb >= kRowsAhead || __all_sync(0xffffffffu, lane >= 9 || qj[kRow + lane] == qj[lane]))) {
+            // the next candidate is equal (or not staged): 128 candidates at
+            // a time, their reads independent
             for (;;) {
                 uint32_t entry[4];
                 bool same[4];
@@ -972,10 +996,8 @@ HD_D bool foa_segment(const Table& t, uint32_t level, const Level& lv, const uin
 #pragma unroll
                 for (uint32_t m = 0; m < 4; m++) {
                     same[m] = entry[m] != kNotFound;
-                    if (same[m]) {
-                        const uint4* c = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(entry[m]));
-                        same[m] = same_words(c[0], p[0]) && same_words(c[1], p[1]) && c[2].x == p[2].x;
-                    }
+                    if (same[m])
+                        same[m] = same_row(lv.cand + kRow * uint64_t(entry[m]), qj, leaf);
                 }
                 uint32_t run = 128;
 #pragma unroll

@@ -12,17 +12,18 @@
 //  * Levels are small near the root.  A level of at most kSmall entries is
 //    processed by CTA 0 alone while the other CTAs wait at the next grid
 //    barrier: consecutive small levels, the end of one edit and the start of
-//    the next cost one barrier in all.  A bottom-up small level whose
-//    candidates fall in more buckets than CTA 0 has warps hands its
-//    find-or-add to the whole grid.
-//  * A big level top-down is one grid phase: each CTA scans the descend
-//    flags of its chunk (offsets of the chunks before it: sums of per-chunk
-//    flag counts gathered while the level was classified), spawns the
-//    children of its descended entries and classifies them.
-//  * A big level bottom-up is six phases: candidates with their pass-1 digit
-//    counts, two stable radix passes on the level-local bucket (digit rows
-//    scanned across the grid between them; pass-2 counts gathered while
-//    pass 1 scatters), then find-or-add, one warp per bucket run.
+//    the next cost one barrier in all, or none when no grid step came
+//    between.  A bottom-up small level whose candidates fall in more than
+//    kLocalRuns buckets hands its find-or-add to the whole grid.
+//  * A big level top-down is one grid phase: each CTA finds the descended
+//    entries of its share of the children (per-chunk counts of descend flags
+//    were gathered while the level was classified), spawns and classifies
+//    them.
+//  * A big level bottom-up is four phases: candidates with their pass-1 digit
+//    counts, two stable radix passes on the level-local bucket (each CTA sums
+//    the digit counts itself; pass-2 counts gathered while pass 1 scatters),
+//    then find-or-add, one warp per bucket run; from kRepeatLevel candidates
+//    on, the repeats and the runs' starts are marked before it.
 //  * Grid barriers are bounded waits: a wait longer than kWaitNs sets
 //    HD_ERR_TIMEOUT and every CTA returns; the host reports the error.
 //  * Nodes and pages that an edit appends are read by the following edits in
@@ -76,6 +77,7 @@ struct Ctl {
     Cmd cmd[2];
     uint32_t ncand[HD_MAX_DEPTH]; // big levels: candidates for find-or-add
     uint32_t nruns[HD_MAX_DEPTH]; // big levels: long runs of repeats
+    uint32_t nstarts[HD_MAX_DEPTH]; // big levels: listed bucket runs
     uint32_t count[HD_MAX_DEPTH];
     // where a wait ran out: the CTA, its barrier count, the arrivals then and
     // the count it waited for, CTA 0's barrier count, phase, level and edit
@@ -108,7 +110,8 @@ struct PArgs {
     uint32_t cap[HD_MAX_DEPTH];
     uint32_t *keys, *vals, *keys2, *vals2;
     uint32_t* bsum;      // 3 x G: per-chunk descend-flag counts, by level parity
-    uint32_t *hist, *hist2, *rows, *rows2; // kDigits x G, kDigits
+    uint32_t *hist, *hist2; // G x kDigits: a big level's digit counts per chunk
+    uint32_t *rows, *rows2; // kDigits: their totals
     uint32_t* same;      // a big level's repeats, a bit per sorted candidate
     FollowerRun* runs;   // its long runs of repeats
     EditOut* out;
@@ -290,59 +293,86 @@ HD_D void td_range(const Table& t, const Editor& ed, const Level* lvs, uint32_t 
     warp_add(&ctr->num_voxels, voxels);
 }
 
-// The grid's top-down step of a big level, in two phases so that the
-// children (8 per descended entry, and the work of classifying them) spread
-// evenly over the CTAs whatever chunks the descended entries fall in.
-// Phase 1: entries [i0, i1) get their positions (prefix: the descended
-// entries before i0) and are listed by position in dlist.
-HD_D void td_positions(const Level& lv, uint32_t i0, uint32_t i1, uint32_t prefix, uint32_t* dlist, uint32_t* sm32)
-{
-    uint32_t run = prefix;
-    for (uint32_t base = i0; base < i1; base += kPT) {
-        const uint32_t i = base + threadIdx.x;
-        const uint32_t f = i < i1 ? lv.flag[i] : 0u;
-        uint32_t total;
-        const uint32_t off = cta_scan(f, &total, sm32);
-        if (f) {
-            lv.exp[i] = run + off;
-            dlist[run + off] = i;
-        }
-        run += total;
-    }
-}
-
-// Phase 2: children [k0, k1) of the level (child k of descended entry
-// dlist[k / 8], slot k % 8) spawned and classified; their descend flags
-// counted per top-down chunk of the next level into cnt_next.  k0 is a
-// multiple of 32, so each warp's 32 consecutive children fall in at most two
-// chunks.
-HD_D void td_children(const Table& t, const Editor& ed, const Level* lvs, uint32_t L, uint32_t k0, uint32_t k1,
-                      uint32_t n_next, uint32_t G, const uint32_t* dlist, uint32_t* cnt_next, EditCounters* ctr)
+// The grid's top-down step of a big level: children [k0, k1) of the level
+// (child k: slot k % 8 of the descended entry of rank k / 8) spawned and
+// classified, so that the children (and the work of classifying them) spread
+// evenly over the CTAs whatever chunks the descended entries fall in.  A CTA
+// finds its ranks' entries itself, kListRanks at a time: cnt holds the
+// descended entries per chunk of the level, and only the flags of the chunks
+// that hold its ranks are scanned (a phase of its own for the ranks, listed in
+// global memory, cost 4-5 us a level).  k0 is a multiple of 32, so each warp's
+// 32 consecutive children fall in at most two chunks of the next level, whose
+// descend flags are counted into cnt_next.
+constexpr uint32_t kListRanks = 4096;
+HD_D void td_children(const Table& t, const Editor& ed, const Level* lvs, uint32_t L, uint32_t n, uint32_t k0,
+                      uint32_t k1, uint32_t n_next, uint32_t G, const uint32_t* cnt, uint32_t* cnt_next,
+                      EditCounters* ctr, uint32_t* sm32, uint32_t* list, uint32_t* chunk_end)
 {
     const Level lv = lvs[L], nx = lvs[L + 1];
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long nodes = 0, voxels = 0;
-    for (uint32_t kb = k0 + (threadIdx.x & ~31u); kb < k1; kb += kPT) {
-        const uint32_t k = kb + lane;
-        const bool act = k < k1;
-        uint32_t fl = 0, ch = 0xFFFFFFFFu;
-        if (act) {
-            uint32_t x, y, z, old;
-            spawn_child(t, lv, nx, __ldcg(dlist + (k >> 3)), k & 7, k, x, y, z, old);
-            unsigned long long nn, vv;
-            classify_values<true>(t, ed, L + 1, nx, k, x, y, z, old, nn, vv);
-            nodes += nn;
-            voxels += vv;
-            fl = nx.flag[k];
-            ch = td_chunk(k, n_next, G);
+    const uint32_t chunk = chunk_len(n, G, kChunkAlign);
+    // chunk_end[b]: descended entries in chunks 0 .. b
+    for (uint32_t b0 = 0, run = 0; b0 < G; b0 += kPT) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint32_t c = b < G ? __ldcg(cnt + b) : 0u;
+        uint32_t total;
+        const uint32_t before = cta_scan(c, &total, sm32);
+        if (b < G)
+            chunk_end[b] = run + before + c;
+        run += total;
+    }
+    __syncthreads();
+    for (uint32_t r0 = k0 / 8; r0 < k1 / 8; r0 += kListRanks) {
+        const uint32_t r1 = min(k1 / 8, r0 + kListRanks);
+        // the chunks that hold ranks [r0, r1)
+        uint32_t b0 = 0, b1 = 0;
+        for (uint32_t base = 0; base < G; base += kPT) {
+            const uint32_t b = base + threadIdx.x;
+            b0 += __syncthreads_count(b < G && chunk_end[b] <= r0);
+            b1 += __syncthreads_count(b < G && (b ? chunk_end[b - 1] : 0u) < r1);
         }
-        const uint32_t ch0 = __shfl_sync(0xffffffffu, ch, 0);
-        const uint32_t b0 = __ballot_sync(0xffffffffu, act && fl && ch == ch0);
-        const uint32_t b1 = __ballot_sync(0xffffffffu, act && fl && ch != ch0);
-        if (lane == 0 && b0)
-            atomicAdd(cnt_next + ch0, uint32_t(__popc(b0)));
-        if (b1 && lane == uint32_t(__ffs(b1) - 1))
-            atomicAdd(cnt_next + ch, uint32_t(__popc(b1)));
+        for (uint32_t b = b0; b < b1; b++) {
+            const uint32_t before = b ? chunk_end[b - 1] : 0u;
+            const uint32_t i1 = min(n, (b + 1) * chunk);
+            uint32_t run = before;
+            for (uint32_t base = b * chunk; base < i1 && run < r1; base += kPT) {
+                const uint32_t i = base + threadIdx.x;
+                const uint32_t f = i < i1 ? lv.flag[i] : 0u;
+                uint32_t total;
+                const uint32_t rank = run + cta_scan(f, &total, sm32);
+                if (f && rank >= r0 && rank < r1) {
+                    lv.exp[i] = rank;
+                    list[rank - r0] = i;
+                }
+                run += total;
+            }
+        }
+        __syncthreads();
+        const uint32_t ke = 8 * r1;
+        for (uint32_t kb = 8 * r0 + (threadIdx.x & ~31u); kb < ke; kb += kPT) {
+            const uint32_t k = kb + lane;
+            const bool act = k < ke;
+            uint32_t fl = 0, ch = 0xFFFFFFFFu;
+            if (act) {
+                uint32_t x, y, z, old;
+                spawn_child(t, lv, nx, list[(k >> 3) - r0], k & 7, k, x, y, z, old);
+                unsigned long long nn, vv;
+                classify_values<true>(t, ed, L + 1, nx, k, x, y, z, old, nn, vv);
+                nodes += nn;
+                voxels += vv;
+                fl = nx.flag[k];
+                ch = td_chunk(k, n_next, G);
+            }
+            const uint32_t ch0 = __shfl_sync(0xffffffffu, ch, 0);
+            const uint32_t b0 = __ballot_sync(0xffffffffu, act && fl && ch == ch0);
+            const uint32_t b1 = __ballot_sync(0xffffffffu, act && fl && ch != ch0);
+            if (lane == 0 && b0)
+                atomicAdd(cnt_next + ch0, uint32_t(__popc(b0)));
+            if (b1 && lane == uint32_t(__ffs(b1) - 1))
+                atomicAdd(cnt_next + ch, uint32_t(__popc(b1)));
+        }
+        __syncthreads();
     }
     warp_add(&ctr->num_nodes, nodes);
     warp_add(&ctr->num_voxels, voxels);
@@ -468,7 +498,7 @@ HD_D void foa_runs(const Table& t, uint32_t L, const Level& lv, const uint32_t* 
 template <int PW>
 HD_D void foa_sorted(const Table& t, uint32_t L, const Level& lv, const uint32_t* keys, const uint32_t* vals,
                      uint32_t n, uint32_t w, uint32_t nw, uint32_t* page, uint32_t* q, FoaCache& cache,
-                     EditCounters* ctr, const Repeats& rep)
+                     EditCounters* ctr)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t empty = t.g.buckets(L);
@@ -504,8 +534,28 @@ HD_D void foa_sorted(const Table& t, uint32_t L, const Level& lv, const uint32_t
                 if (same < 128)
                     break;
             }
-            foa_segment<PW>(t, L, lv, vals, j0, j1, bucket, page, q, cache, foa, added, scanned, rep);
+            foa_segment<PW>(t, L, lv, vals, j0, j1, bucket, page, q, cache, foa, added, scanned);
         }
+    }
+    foa_counts(t, L, ctr, foa, added, scanned);
+}
+
+// Find-or-add of a big level whose repeats are known: its bucket runs, listed
+// by their starts in any order, dealt out to the nw warps in turn.
+template <int PW>
+HD_D void foa_listed(const Table& t, uint32_t L, const Level& lv, const uint32_t* keys, const uint32_t* vals, uint32_t n,
+                     const uint32_t* starts, uint32_t runs, uint32_t w, uint32_t nw, uint32_t* page, uint32_t* q,
+                     FoaCache& cache, EditCounters* ctr, const Repeats& rep)
+{
+    unsigned long long foa = 0, added = 0, scanned = 0;
+    for (uint32_t r = w; r < runs; r += nw) {
+        const uint32_t j0 = __ldcg(starts + r), bucket = __ldcg(keys + j0);
+        uint32_t j1 = j0 + 1;
+        do
+            j1 = end_of_repeats(rep, j1);
+        while (j1 < n && __ldcg(keys + j1) == bucket && ++j1 < n);
+        j1 = min(j1, n);
+        foa_segment<PW>(t, L, lv, vals, j0, j1, bucket, page, q, cache, foa, added, scanned, rep);
     }
     foa_counts(t, L, ctr, foa, added, scanned);
 }
@@ -518,19 +568,28 @@ HD_D void foa_sorted(const Table& t, uint32_t L, const Level& lv, const uint32_t
 // it compared and wrote them 32 at a time: the leaf level of a box of radius
 // 250 (55,640 candidates) went from 1,063 to 94 us, the edit from 1.96 to 0.53
 // ms.
-HD_D void mark_repeats(const Level& lv, const uint32_t* keys, const uint32_t* vals, uint32_t n, uint32_t j0,
-                       uint32_t j1, uint32_t* same)
+// The bucket runs' starts are listed beside (starts / n_starts, in any order).
+HD_D void mark_repeats(const Level& lv, bool leaf, const uint32_t* keys, const uint32_t* vals, uint32_t n, uint32_t j0,
+                       uint32_t j1, uint32_t* same, uint32_t* starts, uint32_t* n_starts)
 {
+    const uint32_t lane = threadIdx.x & 31;
     for (uint32_t j = j0 + threadIdx.x; j - threadIdx.x < j1; j += kPT) {
-        bool eq = false;
-        if (j < j1 && j > 0 && j < n && __ldcg(keys + j) == __ldcg(keys + j - 1)) {
-            const uint4* a = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(__ldcg(vals + j)));
-            const uint4* b = reinterpret_cast<const uint4*>(lv.cand + kRow * uint64_t(__ldcg(vals + j - 1)));
-            eq = same_words(a[0], b[0]) && same_words(a[1], b[1]) && a[2].x == b[2].x;
+        bool eq = false, start = false;
+        if (j < j1) {
+            start = j == 0 || __ldcg(keys + j) != __ldcg(keys + j - 1);
+            if (!start)
+                eq = same_row(lv.cand + kRow * uint64_t(__ldcg(vals + j)),
+                              lv.cand + kRow * uint64_t(__ldcg(vals + j - 1)), leaf);
         }
-        const uint32_t bits = __ballot_sync(0xffffffffu, eq);
-        if ((threadIdx.x & 31) == 0 && j < j1)
+        const uint32_t bits = __ballot_sync(0xffffffffu, eq), sb = __ballot_sync(0xffffffffu, start);
+        if (lane == 0 && j < j1)
             same[j >> 5] = bits;
+        uint32_t at = 0;
+        if (lane == 0 && sb)
+            at = atomicAdd(n_starts, uint32_t(__popc(sb)));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (start)
+            starts[at + __popc(sb & ((1u << lane) - 1u))] = j;
     }
 }
 
@@ -635,50 +694,93 @@ HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, const uint32_t*
     return runs;
 }
 
-// Per digit row of a [kDigits][nb] count table: exclusive scan over the
-// chunks in place, the row total into rows.  Warps of the whole grid.
+// Chunks of a sorted level (their digit counts' rows) that the scatters sum
+// themselves, the least length of a chunk, and the chunks of n elements: one
+// a CTA, at most kSumRows of at most kPT elements for as long as they do.
+constexpr uint32_t kSumRows = 32;
+constexpr uint32_t kSortChunk = 256;
+HD_D uint32_t sort_chunks(uint32_t n, uint32_t G)
+{
+    const uint32_t few = (n + kSortChunk - 1) / kSortChunk;
+    return max(1u, few <= kSumRows ? few : n <= kSumRows * kPT ? kSumRows : min(G, (n + kChunkAlign - 1) / kChunkAlign));
+}
+
+// Per digit of the nb chunks' counts (rows of nd): exclusive scan over the
+// chunks in place, the total into rows.  A thread a digit and part of the
+// chunks would wait for each other; a warp reads 32 digits of a chunk at once
+// and 8 chunks ahead.
 HD_D void scan_rows(uint32_t* hist, uint32_t nb, uint32_t nd, uint32_t* rows)
 {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t gw = blockIdx.x * kPWarps + (threadIdx.x >> 5), nw = gridDim.x * kPWarps;
-    for (uint32_t d = gw; d < nd; d += nw) {
-        uint32_t run = 0;
-        for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
-            const uint32_t b = b0 + lane;
-            const uint32_t x = b < nb ? __ldcg(hist + d * nb + b) : 0u;
-            const uint32_t inc = warp_incl_scan(x);
-            if (b < nb)
-                hist[d * nb + b] = run + inc - x;
-            run += __shfl_sync(0xffffffffu, inc, 31);
+    const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    if (gw >= nd / 32)
+        return;
+    uint32_t* p = hist + gw * 32 + lane;
+    uint32_t run = 0;
+    for (uint32_t c0 = 0; c0 < nb; c0 += 8) {
+        uint32_t x[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++)
+            x[k] = c0 + k < nb ? __ldcg(p + (c0 + k) * nd) : 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            if (c0 + k < nb)
+                p[(c0 + k) * nd] = run;
+            run += x[k];
         }
-        if (lane == 0)
-            rows[d] = run;
     }
+    rows[gw * 32 + lane] = run;
 }
 
 // Stable scatter of chunk `cb` of (keys, vals) by digit (key >> shift) & (nd
-// - 1): bases from the row totals and this chunk's row offsets; warps of a
-// tile take their turn in order.  Keys of `empty` and above are left out.
+// - 1); warps of a tile take their turn in order.  Keys of `empty` and above
+// are left out.  hist: the digit counts of every chunk, a row of nd a chunk.
+// With up to kSumRows chunks each CTA sums the rows itself (totals and the
+// chunks before its own), which spares the scan's phase (2-4 us a pass); more
+// rows are scanned (scan_rows, totals in rows): 152 of them summed by every
+// CTA took 20 us.
 // With hist_next, counts each element's next digit in the chunk (of chunk_next
-// positions, nb_next of them) its output position falls in, equal ones of a
-// warp with one atomic.  (Entries resolved at once, keyed `empty`, were sorted
+// positions) its output position falls in, equal ones of a warp with one
+// atomic.  (Entries resolved at once, keyed `empty`, were sorted
 // along and met in one counter: 55 us of a level of 184,528 entries, now 24.)
 HD_D void scatter_chunk(const uint32_t* keys, const uint32_t* vals, uint32_t n, uint32_t nb, uint32_t cb,
                         uint32_t shift, uint32_t nd, uint32_t empty, const uint32_t* hist, const uint32_t* rows,
-                        uint32_t* keys_out, uint32_t* vals_out, uint32_t* hist_next, uint32_t next_shift,
-                        uint32_t nb_next, uint32_t chunk_next, uint32_t* run, uint32_t* sm32)
+                        uint32_t* keys_out,
+                        uint32_t* vals_out, uint32_t* hist_next, uint32_t next_shift,
+                        uint32_t chunk_next, uint32_t* run, uint32_t* sm32)
 {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t chunk = chunk_len(n, nb, kChunkAlign);
-    // digit bases: exclusive scan of the row totals (nd <= kPT)
-    {
+    if (nb > kSumRows) {
         const uint32_t d = threadIdx.x;
         const uint32_t r = d < nd ? __ldcg(rows + d) : 0u;
         uint32_t total;
         const uint32_t ex = cta_scan(r, &total, sm32);
         if (d < nd)
-            run[d] = ex + __ldcg(hist + d * nb + cb);
+            run[d] = ex + __ldcg(hist + cb * nd + d);
+        __syncthreads();
+    } else {
+        uint32_t* sum = run + kDigits;
+        for (uint32_t d = threadIdx.x; d < nd; d += kPT)
+            run[d] = sum[d] = 0;
+        __syncthreads();
+        // kPT / nd threads a digit, each every kPT / nd-th row
+        const uint32_t d = threadIdx.x & (nd - 1), parts = kPT / nd;
+        uint32_t total = 0, before = 0;
+#pragma unroll 8
+        for (uint32_t c = threadIdx.x / nd; c < nb; c += parts) {
+            const uint32_t x = __ldcg(hist + c * nd + d);
+            total += x;
+            before += c < cb ? x : 0u;
+        }
+        atomicAdd(sum + d, total);
+        atomicAdd(run + d, before);
+        __syncthreads();
+        uint32_t all;
+        const uint32_t ex = cta_scan(threadIdx.x < nd ? sum[threadIdx.x] : 0u, &all, sm32);
+        if (threadIdx.x < nd)
+            run[threadIdx.x] += ex;
         __syncthreads();
     }
     const uint32_t i0 = cb * chunk, i1 = min(n, i0 + chunk);
@@ -705,7 +807,7 @@ HD_D void scatter_chunk(const uint32_t* keys, const uint32_t* vals, uint32_t n, 
                     vals_out[pos] = val;
                 }
                 if (hist_next) {
-                    const uint32_t at = valid ? ((key >> next_shift) & (nd - 1)) * nb_next + pos / chunk_next
+                    const uint32_t at = valid ? pos / chunk_next * nd + ((key >> next_shift) & (nd - 1))
                                               : 0x80000000u + lane;
                     const uint32_t same = __match_any_sync(0xffffffffu, at);
                     if (valid && lane == uint32_t(__ffs(same) - 1))
@@ -765,7 +867,7 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
             *sm.ed = a.edits ? make_editor(a.edits[idx]) : a.one;
             ctl->ed = *sm.ed;
             for (uint32_t L = 0; L < HD_MAX_DEPTH; L++)
-                ctl->count[L] = ctl->ncand[L] = ctl->nruns[L] = 0;
+                ctl->count[L] = ctl->ncand[L] = ctl->nruns[L] = ctl->nstarts[L] = 0;
             ctl->count[0] = 1;
             const Level l0 = a.lv[0];
             l0.x[0] = 0;
@@ -1044,14 +1146,10 @@ __global__ void __launch_bounds__(kPT, 1)
             for (;;) {
                 const uint32_t n = __ldcg(&ctl->count[L]);
                 const uint32_t* cnt_cur = a.bsum + (L % 3) * G;
-                uint32_t before = 0, all = 0;
-                for (uint32_t b = threadIdx.x; b < G; b += kPT) {
-                    const uint32_t v = __ldcg(cnt_cur + b);
-                    all += v;
-                    before += b < cta ? v : 0u;
-                }
-                uint32_t tb, ta;
-                cta_scan(before, &tb, sm32);
+                uint32_t all = 0;
+                for (uint32_t b = threadIdx.x; b < G; b += kPT)
+                    all += __ldcg(cnt_cur + b);
+                uint32_t ta;
                 cta_scan(all, &ta, sm32);
                 if (ta == 0)
                     break; // nothing descends: L is the deepest level
@@ -1063,17 +1161,10 @@ __global__ void __launch_bounds__(kPT, 1)
                 }
                 if (threadIdx.x == 0)
                     a.bsum[((L + 2) % 3) * G + cta] = 0;
-                // positions and the list of descended entries (keys2 is
-                // free until the edit's bottom-up levels), then the children
-                // spread evenly over the CTAs
-                const uint32_t chunk = chunk_len(n, G, kChunkAlign);
-                const uint32_t i0 = min(n, cta * chunk), i1 = min(n, i0 + chunk);
-                td_positions(a.lv[L], i0, i1, tb, a.keys2, sm32);
-                if (!grid_sync(ctl, t.error, nbar))
-                    return;
                 const uint32_t cch = chunk_len(uint32_t(n_next), G, kChunkAlign);
                 const uint32_t k0 = min(uint32_t(n_next), cta * cch), k1 = min(uint32_t(n_next), k0 + cch);
-                td_children(t, ed_s, a.lv, L, k0, k1, uint32_t(n_next), G, a.keys2, a.bsum + ((L + 1) % 3) * G, ctr);
+                td_children(t, ed_s, a.lv, L, n, k0, k1, uint32_t(n_next), G, cnt_cur, a.bsum + ((L + 1) % 3) * G,
+                            ctr, sm32, sm.list, sm.list + kListRanks);
                 if (cta == 0 && threadIdx.x == 0)
                     ctl->count[L + 1] = uint32_t(n_next);
                 if (!grid_sync(ctl, t.error, nbar))
@@ -1103,7 +1194,7 @@ __global__ void __launch_bounds__(kPT, 1)
         // bottom-up, big levels: six phases each; small ones go back to CTA 0
         while (__ldcg(&ctl->count[L]) > kSmall && __ldcg(t.error) == 0) {
             const uint32_t n = __ldcg(&ctl->count[L]);
-            const uint32_t nb = min(G, (n + kChunkAlign - 1) / kChunkAlign);
+            const uint32_t nb = sort_chunks(n, G);
             const uint32_t chunk = chunk_len(n, nb, kChunkAlign);
             uint32_t key_bits = 1;
             while ((1u << key_bits) <= t.g.buckets(L))
@@ -1114,7 +1205,7 @@ __global__ void __launch_bounds__(kPT, 1)
             if (cta < nb) {
                 for (uint32_t d = threadIdx.x; d < nd; d += kPT) {
                     cnt[d] = 0;
-                    a.hist2[d * nb + cta] = 0;
+                    a.hist2[cta * nd + d] = 0;
                 }
                 __syncthreads();
                 const uint32_t i0 = cta * chunk, i1 = min(n, i0 + chunk);
@@ -1132,46 +1223,51 @@ __global__ void __launch_bounds__(kPT, 1)
                     atomicAdd(&ctl->ncand[L], mine);
                 __syncthreads();
                 for (uint32_t d = threadIdx.x; d < nd; d += kPT)
-                    a.hist[d * nb + cta] = cnt[d];
+                    a.hist[cta * nd + d] = cnt[d];
             }
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             // the second pass and the find-or-add: candidates only
             const uint32_t ncand = __ldcg(&ctl->ncand[L]);
-            const uint32_t nb2 = max(1u, min(G, (ncand + kChunkAlign - 1) / kChunkAlign));
+            const uint32_t nb2 = sort_chunks(ncand, G);
             const uint32_t chunk2 = max(kChunkAlign, chunk_len(ncand, nb2, kChunkAlign));
-            // 2. pass-1 rows
-            scan_rows(a.hist, nb, nd, a.rows);
-            if (!grid_sync(ctl, t.error, nbar))
-                return;
-            // 3. pass-1 scatter, pass-2 counts
+            // 2. pass 1, pass-2 counts
+            if (nb > kSumRows) {
+                scan_rows(a.hist, nb, nd, a.rows);
+                if (!grid_sync(ctl, t.error, nbar))
+                    return;
+            }
             if (cta < nb)
                 scatter_chunk(a.keys, a.vals, n, nb, cta, 0, nd, empty, a.hist, a.rows, a.keys2, a.vals2, a.hist2,
-                              dbits, nb2, chunk2, run, sm32);
+                              dbits, chunk2, run, sm32);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
-            // 4. pass-2 rows
-            scan_rows(a.hist2, nb2, nd, a.rows2);
-            if (!grid_sync(ctl, t.error, nbar))
-                return;
-            // 5. pass-2 scatter
+            // 3. pass 2
+            if (nb2 > kSumRows) {
+                scan_rows(a.hist2, nb2, nd, a.rows2);
+                if (!grid_sync(ctl, t.error, nbar))
+                    return;
+            }
             if (cta < nb2)
                 scatter_chunk(a.keys2, a.vals2, ncand, nb2, cta, dbits, nd, empty, a.hist2, a.rows2, a.keys, a.vals,
-                              nullptr, 0, 0, 0, run, sm32);
+                              nullptr, 0, 0, run, sm32);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
-            // 6. find-or-add, one warp per bucket run
-            Repeats rep{};
+            // 4. find-or-add, one warp per bucket run
+            uint32_t *page = sm.page + warp * kPage, *q = sm.q + warp * kFoaQuery;
             if (ncand >= kRepeatLevel) {
                 const uint32_t part = chunk_len(ncand, G, 32);
                 const uint32_t p0 = min(ncand, cta * part), p1 = min(ncand, p0 + part);
-                mark_repeats(a.lv[L], a.keys, a.vals, ncand, p0, p1, a.same);
+                mark_repeats(a.lv[L], L == leafl, a.keys, a.vals, ncand, p0, p1, a.same, a.keys2, &ctl->nstarts[L]);
                 if (!grid_sync(ctl, t.error, nbar))
                     return;
-                rep = Repeats{a.same, (ncand + 31) / 32, a.runs, &ctl->nruns[L]};
+                const Repeats rep{a.same, (ncand + 31) / 32, a.runs, &ctl->nruns[L]};
+                foa_listed<PW>(t, L, a.lv[L], a.keys, a.vals, ncand, a.keys2, __ldcg(&ctl->nstarts[L]), warp * G + cta,
+                               G * kPWarps, page, q, sm.cache[warp], ctr, rep);
+            } else {
+                foa_sorted<PW>(t, L, a.lv[L], a.keys, a.vals, ncand, warp * G + cta, G * kPWarps, page, q,
+                               sm.cache[warp], ctr);
             }
-            foa_sorted<PW>(t, L, a.lv[L], a.keys, a.vals, ncand, cta * kPWarps + warp, G * kPWarps,
-                           sm.page + warp * kPage, sm.q + warp * kFoaQuery, sm.cache[warp], ctr, rep);
             if (!grid_sync(ctl, t.error, nbar))
                 return;
             if (const uint32_t nr = __ldcg(&ctl->nruns[L])) {

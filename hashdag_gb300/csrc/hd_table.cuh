@@ -35,17 +35,19 @@ HD_HD uint32_t append_position(uint32_t& size, uint32_t n, bool leaf)
 // Free-list pops may run concurrently; pushes happen only inside a GC.
 // Returns the page's number, which is also where it lies unless the pool is
 // direct-mapped (place_page).
-HD_D uint32_t claim_page(const Table& t)
+// free_now, limit: the list's count and the claim limit (pool_top[1], [2]) as
+// read beside the page-table entry, so that a claim is one round trip more.
+HD_D uint32_t claim_page(const Table& t, uint32_t free_now, uint32_t limit)
 {
     uint32_t* free_count = t.pool_top + 1;
-    if (__ldcg(free_count) != 0) {
+    if (free_now != 0) {
         const uint32_t k = atomicSub(free_count, 1u);
         if (int32_t(k) > 0)
             return __ldcg(t.free_pages + (k - 1));
         atomicAdd(free_count, 1u); // none left: undo
     }
     const uint32_t p = atomicAdd(t.pool_top, 1u);
-    if (p >= __ldcg(t.pool_top + 2)) { // the claim limit: the pool less the GC's reserve
+    if (p >= limit) { // the pool less the GC's reserve
         atomicSub(t.pool_top, 1u);
         return 0;
     }
@@ -69,9 +71,10 @@ HD_D bool map_pages(const Table& t, uint32_t level, uint32_t bucket, uint32_t fr
         return true;
     const uint32_t v0 = t.g.make_ptr(level, bucket, from) >> kPageShift;
     const uint32_t v1 = t.g.make_ptr(level, bucket, to - 1) >> kPageShift;
+    const uint32_t free_now = __ldcg(t.pool_top + 1), limit = __ldcg(t.pool_top + 2);
     for (uint32_t vp = v0; vp <= v1; vp++) {
         if (__ldcg(t.page_table + vp) == 0) {
-            const uint32_t p = claim_page(t);
+            const uint32_t p = claim_page(t, free_now, limit);
             if (!p) {
                 set_error(t.error, kErrPoolFull, level, bucket, __ldcg(t.pool_top + 2));
                 return false;
