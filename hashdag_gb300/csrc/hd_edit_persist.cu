@@ -239,11 +239,10 @@ HD_D uint32_t cta_scan(uint32_t v, uint32_t* total, uint32_t* sm32)
 // then every child of every descended entry spawned at 8 * exp + c and
 // classified; children's descend flags are counted per top-down chunk of
 // level L + 1 into cnt_next.  CTA-wide.
-HD_D void td_range(const Table& t, const Editor& ed, const Level* lvs, uint32_t L, uint32_t i0, uint32_t i1,
-                   uint32_t prefix, uint32_t n_next, uint32_t G, uint32_t* cnt_next, EditCounters* ctr,
+HD_D void td_range(const Table& t, const Editor& ed, const Level& lv, const Level& nx, uint32_t L, uint32_t i0,
+                   uint32_t i1, uint32_t prefix, uint32_t n_next, uint32_t G, uint32_t* cnt_next, EditCounters* ctr,
                    uint32_t* sm32, uint32_t* list)
 {
-    const Level lv = lvs[L], nx = lvs[L + 1];
     const uint32_t lane = threadIdx.x & 31;
     uint32_t run = prefix;
     unsigned long long nodes = 0, voxels = 0;
@@ -378,75 +377,152 @@ HD_D void td_children(const Table& t, const Editor& ed, const Level* lvs, uint32
     warp_add(&ctr->num_voxels, voxels);
 }
 
-// Top-down, one warp of CTA 0 alone: consecutive levels of at most 32
-// entries (the levels near the root), as td_range does them for a whole
-// level (positions, children spawned and classified, the next level's
-// per-chunk descend counts) but with warp votes in place of CTA scans and
-// barriers.  Returns the first level it did not descend from; status 0: that
-// level holds more than 32 entries (or is the leaf level), 1: it had no
-// descended entry (it is the deepest), 2: its children would exceed their
-// level's capacity.
-HD_D uint32_t td_tiny(const Table& t, const Editor& ed, const PArgs& a, uint32_t L, uint32_t n, EditCounters* ctr,
-                      uint32_t* list, uint32_t& status)
+// ---- tiny levels ----------------------------------------------------------------
+// The levels near the root hold a few entries, and an edit of any size passes
+// through all of them twice, each step waiting for the one before.  Levels of
+// at most kTiny entries that such a level spawned keep their arrays in CTA 0's
+// shared memory (the level arrays proper are written at the edit's end, and
+// only when its colours will read them), a lane an entry: what is left of a
+// level's chain is the table itself, two reads down (a node with its child
+// pointers, the old child's count) and two or three up (a bucket's size with
+// its filters, a page, a claim).  With the arrays in global memory, nodes read
+// word after word, a sort and CTA barriers a level took 1.6 us down and 5-6 us
+// up, now 0.9 and 3-4.5: an edit of radius 11 at 2^15 goes from 115 to 86 us.
+constexpr uint32_t kTiny = 32;
+struct __align__(16) TinyLevel {
+    uint32_t x[kTiny], y[kTiny], z[kTiny], old[kTiny], res[kTiny], cnt[kTiny], flag[kTiny], exp[kTiny];
+    uint8_t state[kTiny];
+};
+struct TinyState {
+    TinyLevel lv[HD_MAX_DEPTH];
+    uint32_t rows[kTiny * kRow]; // the candidates of the level being resolved
+    uint32_t sk[kTiny], sv[kTiny], rs[kTiny + 1]; // sorted, and their bucket runs' starts
+    uint32_t held;               // bit L: level L is held here
+    uint32_t failed;             // an append of the edit failed
+    uint32_t list[kTiny];        // descended entries by rank
+    uint32_t level, status, runs; // what the warp reports
+    uint32_t count[HD_MAX_DEPTH]; // CTA 0's copy of the entry counts
+};
+
+// Level L's arrays: the shared ones when it is held there
+HD_D Level held_level(const PArgs& a, const TinyState& ts, uint32_t L)
 {
-    const uint32_t lane = threadIdx.x & 31, G = gridDim.x, leafl = t.g.leaf_level;
+    Level l = a.lv[L];
+    if ((ts.held >> L) & 1u) {
+        TinyLevel& m = const_cast<TinyLevel&>(ts.lv[L]);
+        l.x = m.x, l.y = m.y, l.z = m.z, l.old = m.old, l.res = m.res, l.cnt = m.cnt, l.flag = m.flag, l.exp = m.exp;
+        l.state = m.state;
+    }
+    return l;
+}
+
+// Top-down, one warp of CTA 0 alone: consecutive held levels whose children
+// are at most kTiny (td_range's step: ranks, children spawned and classified).
+// A node is read with its 8 possible child pointers at once, a word a lane,
+// and each child takes its pointer from the lane that has it.  Returns the
+// first level it did not descend from; status 0: the level has more children
+// (or is the leaf level), 1: it had no descended entry (it is the deepest), 2:
+// its children would exceed their level's capacity.
+HD_D uint32_t td_tiny(const Table& t, const Editor& ed, const PArgs& a, TinyState& ts, uint32_t L, EditCounters* ctr,
+                      uint32_t& status)
+{
+    const uint32_t lane = threadIdx.x & 31, leafl = t.g.leaf_level;
     unsigned long long nodes = 0, voxels = 0;
     status = 0;
-    while (L < leafl && n <= 32) {
-        const Level lv = a.lv[L], nx = a.lv[L + 1];
-        const uint32_t f = lane < n ? lv.flag[lane] : 0u;
-        const uint32_t fb = __ballot_sync(0xffffffffu, f != 0);
-        const uint32_t total = __popc(fb);
-        if (total == 0) {
+    while (L < leafl) {
+        TinyLevel& m = ts.lv[L];
+        const uint32_t fb = __ballot_sync(0xffffffffu, lane < ts.count[L] && m.flag[lane]);
+        const uint32_t n_next = 8 * __popc(fb);
+        if (n_next == 0) {
             status = 1;
             break;
         }
-        const uint32_t n_next = 8 * total;
         if (n_next > a.cap[L + 1]) {
             status = 2;
             break;
         }
-        uint32_t* zero = a.bsum + ((L + 2) % 3) * G;
-        for (uint32_t k = lane; k < G; k += 32)
-            zero[k] = 0;
-        uint32_t* cnt_next = a.bsum + ((L + 1) % 3) * G;
-        if (f) {
-            const uint32_t off = __popc(fb & ((1u << lane) - 1u));
-            lv.exp[lane] = off;
-            list[off] = lane;
+        if (n_next > kTiny)
+            break;
+        if ((fb >> lane) & 1u) {
+            const uint32_t rank = __popc(fb & ((1u << lane) - 1u));
+            m.exp[lane] = rank;
+            ts.list[rank] = lane;
+        }
+        if (lane == 0) {
+            ts.held |= 1u << (L + 1);
+            ts.count[L + 1] = n_next;
+            a.ctl->count[L + 1] = n_next;
         }
         __syncwarp();
-        for (uint32_t k0 = 0; k0 < n_next; k0 += 32) {
-            const uint32_t k = k0 + lane;
-            const bool act = k < n_next;
-            uint32_t fl = 0, ch = 0xFFFFFFFFu;
-            if (act) {
-                uint32_t x, y, z, old;
-                spawn_child(t, lv, nx, list[k >> 3], k & 7, k, x, y, z, old);
-                unsigned long long nn, vv;
-                classify_values<true>(t, ed, L + 1, nx, k, x, y, z, old, nn, vv);
-                nodes += nn;
-                voxels += vv;
-                fl = nx.flag[k];
-                ch = td_chunk(k, n_next, G);
+        const uint32_t c = lane & 7;
+        const bool act = lane < n_next;
+        uint32_t x = 0, y = 0, z = 0, old = kInvalid, head = 0, word = 0;
+        if (act) {
+            const uint32_t p = ts.list[lane >> 3];
+            x = (m.x[p] << 1) | ((c >> 2) & 1);
+            y = (m.y[p] << 1) | ((c >> 1) & 1);
+            z = (m.z[p] << 1) | (c & 1);
+            const uint32_t node = m.old[p];
+            if (node != kInvalid) {
+                const uint32_t* w = t.sys_cg(node);
+                head = __ldcg(w);
+                word = __ldcg(w + 1 + c); // (past a smaller node's end: not used)
             }
-            const uint32_t ch0 = __shfl_sync(0xffffffffu, ch, 0);
-            const uint32_t b0 = __ballot_sync(0xffffffffu, act && fl && ch == ch0);
-            const uint32_t b1 = __ballot_sync(0xffffffffu, act && fl && ch != ch0);
-            if (lane == 0 && b0)
-                atomicAdd(cnt_next + ch0, uint32_t(__popc(b0)));
-            if (b1 && lane == uint32_t(__ffs(b1) - 1))
-                atomicAdd(cnt_next + ch, uint32_t(__popc(b1)));
         }
-        if (lane == 0)
-            a.ctl->count[L + 1] = n_next;
+        const uint32_t from = (lane & ~7u) + popc32(head & ((1u << c) - 1u));
+        const uint32_t child = __shfl_sync(0xffffffffu, word, from);
+        if ((head >> c) & 1u)
+            old = child;
+        if (act) {
+            TinyLevel& k = ts.lv[L + 1];
+            k.x[lane] = x;
+            k.y[lane] = y;
+            k.z[lane] = z;
+            k.old[lane] = old;
+            unsigned long long nn, vv;
+            classify_values<true>(t, ed, L + 1, held_level(a, ts, L + 1), lane, x, y, z, old, nn, vv);
+            nodes += nn;
+            voxels += vv;
+        }
         __syncwarp(); // the next level reads the flags other lanes wrote
-        n = n_next;
         L++;
     }
     warp_add(&ctr->num_nodes, nodes);
     warp_add(&ctr->num_voxels, voxels);
     return L;
+}
+
+// Bottom-up, one warp: candidates of level L (at most kTiny entries, a lane
+// each; held or not) into ts.rows, grouped by bucket without a sort: the
+// lanes of a bucket know each other, groups are in the order of their first
+// lanes, and a group's lanes are in entry order.  Returns the bucket runs.
+HD_D uint32_t tiny_candidates(const Table& t, const PArgs& a, TinyState& ts, uint32_t L, uint32_t deepest, uint32_t n)
+{
+    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    Level lv = held_level(a, ts, L);
+    lv.cand = ts.rows;
+    const Level child = L < deepest ? held_level(a, ts, L + 1) : Level{};
+    const uint32_t key = lane < n ? candidate_entry<true>(t, L, lv, child, lane) : kNoBucket;
+    const uint32_t cb = __ballot_sync(0xffffffffu, key != kNoBucket);
+    if (!cb)
+        return 0;
+    const uint32_t peers = __match_any_sync(0xffffffffu, key) & cb;
+    const bool lead = key != kNoBucket && (peers & lt) == 0;
+    const uint32_t leads = __ballot_sync(0xffffffffu, lead);
+    // candidates of the groups before: their sizes summed at their leaders
+    const uint32_t end = warp_incl_scan(lead ? uint32_t(__popc(peers)) : 0u);
+    const uint32_t first = __shfl_sync(0xffffffffu, end, key != kNoBucket ? __ffs(peers) - 1 : 0) - __popc(peers);
+    if (key != kNoBucket) {
+        const uint32_t at = first + __popc(peers & lt);
+        ts.sk[at] = key;
+        ts.sv[at] = lane;
+        if (lead)
+            ts.rs[__popc(leads & lt)] = at;
+    }
+    if (lane == 0)
+        ts.rs[__popc(leads)] = __popc(cb);
+    __syncwarp();
+    return __popc(leads);
 }
 
 // Bottom-up candidates of entries [i0, i1) of level L: key = level-local
@@ -480,12 +556,13 @@ HD_D void foa_counts(const Table& t, uint32_t L, EditCounters* ctr, unsigned lon
 template <int PW>
 HD_D void foa_runs(const Table& t, uint32_t L, const Level& lv, const uint32_t* keys, const uint32_t* vals,
                    const uint32_t* starts, uint32_t runs, uint32_t w, uint32_t nw, uint32_t* page, uint32_t* q,
-                   FoaCache& cache, EditCounters* ctr)
+                   FoaCache& cache, EditCounters* ctr, uint32_t* failed = nullptr)
 {
     unsigned long long foa = 0, added = 0, scanned = 0;
     for (uint32_t r = w; r < runs; r += nw) {
         const uint32_t j0 = starts[r], j1 = starts[r + 1];
-        foa_segment<PW>(t, L, lv, vals, j0, j1, keys[j0], page, q, cache, foa, added, scanned);
+        if (!foa_segment<PW>(t, L, lv, vals, j0, j1, keys[j0], page, q, cache, foa, added, scanned) && failed)
+            *failed = 1;
     }
     foa_counts(t, L, ctr, foa, added, scanned);
 }
@@ -621,7 +698,7 @@ HD_D void fill_runs(const Level& lv, const uint32_t* vals, const FollowerRun* ru
     }
 }
 
-// CTA 0 alone: stable sort of the n (<= kPT) candidates of a small level by
+// CTA 0 alone: stable sort of the n (kTiny < n <= kPT) candidates of a small level by
 // (bucket, entry) in registers, one a thread: a bitonic network with lane
 // shuffles, and shared memory for the steps across warps (two buffers, so
 // one barrier a step; a rank sort, n reads a thread, took 15.6 us at n = 784).
@@ -663,24 +740,6 @@ HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, const uint32_t*
     if (i < n) {
         sk[i] = key;
         sv[i] = uint32_t(x);
-    }
-    if (n <= 32) {
-        // one warp holds them all
-        if (i < 32) {
-            const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-            const bool start = cand && (lane == 0 || prev != key);
-            const uint32_t sb = __ballot_sync(0xffffffffu, start), cb = __ballot_sync(0xffffffffu, cand);
-            if (start)
-                rs[__popc(sb & ((1u << lane) - 1u))] = i;
-            if (lane == 0) {
-                rs[__popc(sb)] = __popc(cb);
-                sm32[0] = __popc(sb);
-            }
-        }
-        __syncthreads();
-        const uint32_t runs = sm32[0];
-        __syncthreads();
-        return runs;
     }
     const uint32_t ncand = __syncthreads_count(cand); // also: sk is written
     const bool start = cand && (i == 0 || sk[i - 1] != key);
@@ -847,6 +906,7 @@ struct Smem {
     uint32_t* list;
     uint32_t* sm32;
     Editor* ed;
+    TinyState* tiny;
 };
 
 // CTA 0: the next edit of the batch (or the stop); level 0 classified.
@@ -869,11 +929,12 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
             for (uint32_t L = 0; L < HD_MAX_DEPTH; L++)
                 ctl->count[L] = ctl->ncand[L] = ctl->nruns[L] = ctl->nstarts[L] = 0;
             ctl->count[0] = 1;
-            const Level l0 = a.lv[0];
-            l0.x[0] = 0;
-            l0.y[0] = 0;
-            l0.z[0] = 0;
-            l0.old[0] = __ldcg(a.d_root);
+            TinyState& ts = *sm.tiny;
+            ts.held = 1;
+            ts.failed = 0;
+            ts.count[0] = 1;
+            ts.lv[0].x[0] = ts.lv[0].y[0] = ts.lv[0].z[0] = 0;
+            ts.lv[0].old[0] = __ldcg(a.d_root);
             a.out[idx].ctr = EditCounters{};
             a.out[idx].t_begin = now_ns();
         }
@@ -886,7 +947,7 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
         return false;
     if (threadIdx.x == 0) {
         unsigned long long nn, vv;
-        classify_entry<true>(t, *sm.ed, 0, a.lv[0], 0, nn, vv);
+        classify_entry<true>(t, *sm.ed, 0, held_level(a, *sm.tiny, 0), 0, nn, vv);
         EditCounters* ctr = &a.out[ctl->idx].ctr;
         atomicAdd(&ctr->num_nodes, nn);
         atomicAdd(&ctr->num_voxels, vv);
@@ -896,15 +957,27 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
 }
 
 // CTA 0, after level 0's find-or-add: the new root, or the stop.
-HD_D void finish_edit(const Table& t, const PArgs& a)
+HD_D void finish_edit(const Table& t, const PArgs& a, const Smem& sm)
 {
     Ctl* ctl = a.ctl;
+    if (a.hold_root) {
+        // the colour phase reads the level arrays: a warp a held level
+        const TinyState& ts = *sm.tiny;
+        const uint32_t L = threadIdx.x >> 5, k = threadIdx.x & 31;
+        if (L < HD_MAX_DEPTH && ((ts.held >> L) & 1u) && k < ts.count[L]) {
+            const TinyLevel& m = ts.lv[L];
+            const Level l = a.lv[L];
+            l.x[k] = m.x[k], l.y[k] = m.y[k], l.z[k] = m.z[k], l.old[k] = m.old[k];
+            l.res[k] = m.res[k], l.cnt[k] = m.cnt[k], l.flag[k] = m.flag[k], l.exp[k] = m.exp[k];
+            l.state[k] = m.state[k];
+        }
+    }
     if (threadIdx.x == 0) {
         const uint32_t idx = ctl->idx;
         if (__ldcg(t.error) != 0) {
             ctl->stop = kTableError;
         } else {
-            const uint32_t r = __ldcg(a.lv[0].res);
+            const uint32_t r = sm.tiny->lv[0].res[0];
             if (r == kInvalid || r == kNotFound) {
                 ctl->stop = kEmptyScene;
             } else {
@@ -929,6 +1002,7 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
     Ctl* ctl = a.ctl;
     const uint32_t G = gridDim.x, leafl = t.g.leaf_level;
     const uint32_t warp = threadIdx.x >> 5;
+    TinyState& ts = *sm.tiny;
     __shared__ bool meet;
     const unsigned long long t_in = now_ns();
     for (;;) {
@@ -936,7 +1010,7 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
             // the edit ends; the next one begins at once when every other CTA
             // already waits at the coming barrier (it reads no more of this
             // edit's state) and has not waited a good part of its bound
-            finish_edit(t, a);
+            finish_edit(t, a, sm);
             if (threadIdx.x == 0) {
                 const unsigned long long set_ns = __ldcg(&ctl->wait_ns);
                 ctl->phase = kPhNone;
@@ -958,33 +1032,29 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
         }
         EditCounters* ctr = &a.out[ctl->idx].ctr;
         if (ls == kLsTopDown) {
-            __shared__ uint32_t tiny[2];
             while (L < leafl) {
-                uint32_t n = ctl->count[L];
-                if (n <= 32) {
-                    // the levels of at most 32 entries: warp 0 alone
+                if ((ts.held >> L) & 1u) {
+                    // the held levels: warp 0 alone
                     if (warp == 0) {
                         uint32_t st;
-                        const uint32_t L2 = td_tiny(t, *sm.ed, a, L, n, ctr, sm.list, st);
+                        const uint32_t L2 = td_tiny(t, *sm.ed, a, ts, L, ctr, st);
                         if ((threadIdx.x & 31) == 0) {
-                            tiny[0] = L2;
-                            tiny[1] = st;
+                            ts.level = L2;
+                            ts.status = st;
                         }
                     }
                     __syncthreads();
-                    L = tiny[0];
-                    const uint32_t st = tiny[1];
-                    __syncthreads();
-                    if (st == 2) {
+                    L = ts.level;
+                    if (ts.status == 2) {
                         if (threadIdx.x == 0)
                             ctl->stop = kCapacity;
                         __syncthreads();
                         return;
                     }
-                    if (st == 1 || L >= leafl)
+                    if (ts.status == 1 || L >= leafl)
                         break;
-                    n = ctl->count[L];
                 }
+                const uint32_t n = ts.count[L];
                 if (n > kSmall) {
                     if (threadIdx.x == 0) {
                         ctl->phase = kPhTopDown;
@@ -993,9 +1063,10 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
                     __syncthreads();
                     return;
                 }
+                const Level lv = held_level(a, ts, L), nx = a.lv[L + 1];
                 uint32_t f = 0;
                 for (uint32_t i = threadIdx.x; i < n; i += kPT)
-                    f += a.lv[L].flag[i];
+                    f += lv.flag[i];
                 uint32_t total;
                 cta_scan(f, &total, sm.sm32);
                 if (total == 0)
@@ -1011,10 +1082,10 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
                 for (uint32_t k = threadIdx.x; k < G; k += kPT)
                     zero[k] = 0;
                 __syncthreads();
-                td_range(t, *sm.ed, a.lv, L, 0, n, 0, uint32_t(n_next), G, a.bsum + ((L + 1) % 3) * G, ctr, sm.sm32,
+                td_range(t, *sm.ed, lv, nx, L, 0, n, 0, uint32_t(n_next), G, a.bsum + ((L + 1) % 3) * G, ctr, sm.sm32,
                          sm.list);
                 if (threadIdx.x == 0)
-                    ctl->count[L + 1] = uint32_t(n_next);
+                    ctl->count[L + 1] = ts.count[L + 1] = uint32_t(n_next);
                 __syncthreads();
                 L++;
             }
@@ -1025,10 +1096,55 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
         }
         if (ls == kLsBottomUp) {
             const uint32_t deepest = ctl->deepest;
+            if (threadIdx.x == 0 && __ldcg(t.error) != 0)
+                ts.failed = 1; // (after a grid step)
+            __syncthreads();
             for (;;) {
-                if (__ldcg(t.error) != 0)
+                // after a failed append the levels above are not rebuilt
+                const bool failed = ts.failed;
+                __syncthreads(); // (warp 0 writes the state below)
+                if (failed)
                     break;
-                const uint32_t n = ctl->count[L];
+                if (ts.count[L] <= kTiny) {
+                    // one warp passes through the levels of at most one
+                    // bucket run; more runs are the CTA's
+                    if (warp == 0) {
+                        uint32_t l = L, runs;
+                        for (;;) {
+                            runs = tiny_candidates(t, a, ts, l, deepest, ts.count[l]);
+                            if (runs > 1)
+                                break;
+                            if (runs) {
+                                Level lv = held_level(a, ts, l);
+                                lv.cand = ts.rows;
+                                foa_runs<PW>(t, l, lv, ts.sk, ts.sv, ts.rs, runs, 0, 1, sm.page, sm.q, sm.cache[0], ctr,
+                                             &ts.failed);
+                                __syncwarp();
+                            }
+                            if (ts.failed || l == 0 || ts.count[l - 1] > kTiny)
+                                break;
+                            l--;
+                        }
+                        if ((threadIdx.x & 31) == 0) {
+                            ts.level = l;
+                            ts.runs = runs;
+                        }
+                    }
+                    __syncthreads();
+                    L = ts.level;
+                    if (const uint32_t runs = ts.runs; runs > 1) {
+                        Level lv = held_level(a, ts, L);
+                        lv.cand = ts.rows;
+                        foa_runs<PW>(t, L, lv, ts.sk, ts.sv, ts.rs, runs, warp, kPWarps, sm.page + warp * kPage,
+                                     sm.q + warp * kFoaQuery, sm.cache[warp], ctr, &ts.failed);
+                        __syncthreads();
+                    }
+                    if (L == 0)
+                        break;
+                    L--;
+                    continue;
+                }
+                const uint32_t n = ts.count[L];
                 if (n > kSmall) {
                     if (threadIdx.x == 0) {
                         ctl->phase = kPhBottomUp;
@@ -1057,7 +1173,7 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
                     return;
                 }
                 foa_runs<PW>(t, L, a.lv[L], sm.sk, sm.sv, sm.rs, runs, warp, kPWarps, sm.page + warp * kPage,
-                             sm.q + warp * kFoaQuery, sm.cache[warp], ctr);
+                             sm.q + warp * kFoaQuery, sm.cache[warp], ctr, &ts.failed);
                 // the CTA barrier makes this level's results (lv.res, appended
                 // nodes) visible to CTA 0's next level; the grid barrier
                 // (a CTA barrier, then a fence by its thread 0) to the grid
@@ -1097,6 +1213,7 @@ __global__ void __launch_bounds__(kPT, 1)
     sm.list = sm.page;
     sm.sm32 = sm32;
     sm.ed = &ed_s;
+    sm.tiny = reinterpret_cast<TinyState*>(sm.rs + kPT + 4);
     uint32_t* run = sm.page;
     Ctl* ctl = a.ctl;
     const uint32_t G = gridDim.x, cta = blockIdx.x;
@@ -1166,7 +1283,7 @@ __global__ void __launch_bounds__(kPT, 1)
                 td_children(t, ed_s, a.lv, L, n, k0, k1, uint32_t(n_next), G, cnt_cur, a.bsum + ((L + 1) % 3) * G,
                             ctr, sm32, sm.list, sm.list + kListRanks);
                 if (cta == 0 && threadIdx.x == 0)
-                    ctl->count[L + 1] = uint32_t(n_next);
+                    ctl->count[L + 1] = sm.tiny->count[L + 1] = uint32_t(n_next);
                 if (!grid_sync(ctl, t.error, nbar))
                     return;
                 L++;
@@ -1287,7 +1404,7 @@ __global__ void __launch_bounds__(kPT, 1)
 
 // ---- host side --------------------------------------------------------------------
 
-static size_t persist_smem() { return persist_smem_core() + size_t(kPT) * 4 * 3 + 16; }
+static size_t persist_smem() { return persist_smem_core() + size_t(kPT) * 4 * 3 + 16 + sizeof(TinyState); }
 
 template <int PW>
 static const void* persist_kernel()
