@@ -174,8 +174,24 @@ void trace_primary(hd_ctx* c, const hd_camera& cam, uint32_t w, uint32_t h, uint
 // and a 4-word head (ray count, two work counters).
 inline uint64_t shadow_list_words(uint64_t px) { return 4 * px + 4; }
 // Doubles of one view's camera tables (trace_views): a column entry per
-// column and a row entry per row, 3 doubles each.
-__host__ __device__ inline uint64_t camera_table_words(uint32_t w, uint32_t h) { return 3ull * (uint64_t(w) + h); }
+// column and a row entry per row, 3 doubles each, then the same entries as 4
+// floats each (16-byte aligned).
+__host__ __device__ inline uint64_t camera_double_words(uint32_t w, uint32_t h)
+{
+    return (3ull * (uint64_t(w) + h) + 1) & ~1ull;
+}
+__host__ __device__ inline uint64_t camera_table_words(uint32_t w, uint32_t h)
+{
+    return camera_double_words(w, h) + 2ull * (uint64_t(w) + h);
+}
+__host__ __device__ inline float4* camera_float_table(double* tables, uint32_t w, uint32_t h)
+{
+    return reinterpret_cast<float4*>(tables + camera_double_words(w, h));
+}
+__host__ __device__ inline const float4* camera_float_table(const double* tables, uint32_t w, uint32_t h)
+{
+    return reinterpret_cast<const float4*>(tables + camera_double_words(w, h));
+}
 void trace_shadow(hd_ctx* c, const hd_camera& cam, uint32_t w, uint32_t h, const uint32_t* d_paths,
                   const float light[3], float bias, uint8_t* d_mask, unsigned long long* d_counters = nullptr,
                   cudaStream_t stream = nullptr, const uint32_t* d_root = nullptr, uint32_t* d_list = nullptr);
