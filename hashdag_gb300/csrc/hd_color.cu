@@ -14,6 +14,7 @@
 // byte-swapped words) into a leaf, new slots get colour nodes and leaves
 // as edit_threaded allocates them, and the replaced leaves go to an undo
 // frame (HashDAGUndoRedo, hash_dag.h:20-212).
+#include <cstring>
 #include <functional>
 #include <vector>
 
@@ -666,8 +667,165 @@ void copy_source(hd_ctx* c, Editor& ed)
 
 // ---- the colour phase of an edit -------------------------------------------------
 
-// Top-down: colour nodes of the next level's entries (levels < T), the slot
-// reference at level T.
+// What an edit does per entry of the levels down to T and per task is little
+// (tens to a few thousand entries), and a launch per level and per scan, with
+// waits in between, took longer than its work: 60 launches and 12 waits an
+// edit.  One block of kTreeThreads threads goes through all of it in three
+// launches (k_col_down, k_col_sizes, k_col_up), whatever the edit's size: with
+// several entries per thread in flight a level of 50,000 entries takes it some
+// 25 us.  Twelve edits of radius 8 to 64 at 2^13 with their undos: 10.0 ms with
+// the launches per level, 5.6 so.
+constexpr uint32_t kTreeThreads = 1024;
+struct TreeLevel {
+    const uint32_t *flag, *exp;
+    uint32_t *cn, *newnode;
+    uint32_t n;
+};
+struct Tree {
+    TreeLevel lv[HD_MAX_DEPTH + 1]; // levels 0 .. T
+    uint32_t T;
+};
+// What the host learns of the colour phase, and what it takes from step to step.
+struct ColHead {
+    uint64_t total;       // colours
+    uint32_t pieces;      // of kPieceColors
+    uint32_t blocks, macro_words, weight_words, new_slots;
+    uint32_t replaced; // leaves: tasks with colours
+    uint64_t node_top, pad;
+};
+// A replaced leaf of the undo history.
+struct Replaced {
+    LeafDesc prev, next;
+    uint32_t leaf, pad[3];
+};
+
+template <typename A, typename B>
+struct Two {
+    A a;
+    B b;
+};
+// Exclusive sums over a block of kTreeThreads threads; sums: 33 entries in
+// shared memory, total: of all threads.
+template <typename A, typename B>
+HD_D Two<A, B> block_scan(const Two<A, B>& v, Two<A, B>& total, Two<A, B>* sums)
+{
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto scan = [&](Two<A, B> x) {
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const A a = __shfl_up_sync(0xffffffffu, x.a, o);
+            const B b = __shfl_up_sync(0xffffffffu, x.b, o);
+            if (lane >= o) {
+                x.a += a;
+                x.b += b;
+            }
+        }
+        return x;
+    };
+    const Two<A, B> inc = scan(v);
+    if (lane == 31)
+        sums[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const Two<A, B> w = sums[lane], wi = scan(w);
+        sums[lane] = {A(wi.a - w.a), B(wi.b - w.b)};
+        if (lane == 31)
+            sums[32] = wi;
+    }
+    __syncthreads();
+    const Two<A, B> before = sums[warp];
+    total = sums[32];
+    __syncthreads();
+    return {A(inc.a - v.a + before.a), B(inc.b - v.b + before.b)};
+}
+
+// Leaf packing works on pieces of a task's colours, a warp each.  A warp per
+// task (the edits have a few hundred tasks, of up to tens of thousands of
+// colours) walked its colours 32 at a time with a load's latency in each step:
+// 234 us to count and 269 us to pack an edit of the twelve of radius 8 to 64 at
+// 2^13, with pieces 4.4 and 5.9 us.  A piece lies in one macro block; its
+// colours are loaded together.
+constexpr uint32_t kPieceSteps = 8, kPieceColors = 32 * kPieceSteps;
+static_assert(kColorsPerMacro % kPieceColors == 0, "a piece lies in one macro block");
+
+// Top-down: colour nodes of the entries of levels 1 .. T - 1, the slot
+// references at level T (spawn: not done while the levels were made); then
+// level T's tasks: their colours' places (base) and pieces (first), the
+// children's offsets and tasks from there on.  One block.
+__global__ void __launch_bounds__(kTreeThreads)
+    k_col_down(ColorTable ct, __grid_constant__ const Tree tree, Level lvT, bool spawn, uint64_t* len, uint64_t* base,
+               uint32_t* first, ColHead* head)
+{
+    __shared__ Two<uint64_t, uint32_t> sums[33];
+    const uint32_t T = tree.T;
+    if (spawn) {
+        if (threadIdx.x == 0)
+            tree.lv[0].cn[0] = 0;
+        __syncthreads();
+        for (uint32_t L = 0; L < T; L++) {
+            const TreeLevel& lv = tree.lv[L];
+            uint32_t* next = tree.lv[L + 1].cn;
+            // two threads an entry: four children each
+#pragma unroll 4
+            for (uint32_t j = threadIdx.x; j < 2 * lv.n; j += kTreeThreads) {
+                const uint32_t i = j >> 1, h = (j & 1) * 4;
+                if (!lv.flag[i])
+                    continue;
+                const uint32_t cn = lv.cn[i];
+                const bool has = L == 0 || cn != 0;
+                uint32_t* to = next + 8 * lv.exp[i] + h;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++)
+                    to[k] = has ? ct.nodes[cn + h + k] : 0u;
+            }
+            __syncthreads();
+        }
+    }
+    constexpr uint32_t kItems = 4;
+    const uint32_t n = tree.lv[T].n;
+    Two<uint64_t, uint32_t> done{0, 0};
+    for (uint32_t i0 = 0; i0 < n; i0 += kTreeThreads * kItems) {
+        uint32_t k[kItems];
+        Two<uint64_t, uint32_t> mine{0, 0}, total;
+#pragma unroll
+        for (uint32_t j = 0; j < kItems; j++) {
+            const uint32_t i = i0 + threadIdx.x * kItems + j;
+            k[j] = 0;
+            if (i < n) {
+                k[j] = (lvT.state[i] != kSkip && lvT.res[i] != kInvalid) ? lvT.cnt[i] : 0;
+                lvT.noff[i] = 0;
+                lvT.ooff[i] = 0;
+                lvT.task[i] = i;
+            }
+            mine.a += k[j];
+            mine.b += uint32_t((uint64_t(k[j]) + kPieceColors - 1) / kPieceColors);
+        }
+        Two<uint64_t, uint32_t> at = block_scan(mine, total, sums);
+        at.a += done.a;
+        at.b += done.b;
+#pragma unroll
+        for (uint32_t j = 0; j < kItems; j++) {
+            const uint32_t i = i0 + threadIdx.x * kItems + j;
+            if (i < n) {
+                len[i] = k[j];
+                base[i] = at.a;
+                first[i] = at.b;
+            }
+            at.a += k[j];
+            at.b += uint32_t((uint64_t(k[j]) + kPieceColors - 1) / kPieceColors);
+        }
+        done.a += total.a;
+        done.b += total.b;
+    }
+    if (threadIdx.x == 0) {
+        first[n] = done.b;
+        head->total = done.a;
+        head->pieces = done.b;
+    }
+}
+
+// The next level's colour nodes of one level's entries (edits whose levels are
+// made one by one).
 __global__ void k_col_spawn(ColorTable ct, uint32_t level, uint32_t n, Level lv, Level next)
 {
     HD_GRID_STRIDE(i, n)
@@ -686,30 +844,6 @@ void color_spawn(hd_ctx* c, uint32_t level, uint32_t n, const Level& lv, const L
 {
     k_col_spawn<<<grid_for(n, 128), 128, 0, c->stream>>>(c->ct, level, n, lv, next);
     HD_LAUNCH_CHECK();
-}
-
-// Leaf packing works on pieces of a task's colours, a warp each.  A warp per
-// task (the edits have a few hundred tasks, of up to tens of thousands of
-// colours) walked its colours 32 at a time with a load's latency in each step:
-// 234 us to count and 269 us to pack an edit of the twelve of radius 8 to 64 at
-// 2^13, with pieces 4.4 and 5.9 us.  A piece lies in one macro block; its
-// colours are loaded together.
-constexpr uint32_t kPieceSteps = 8, kPieceColors = 32 * kPieceSteps;
-static_assert(kColorsPerMacro % kPieceColors == 0, "a piece lies in one macro block");
-
-// Level T: the tasks; offsets 0, task = own index.
-__global__ void k_col_tasks(uint32_t n, Level lv, uint64_t* len, uint32_t* pieces)
-{
-    HD_GRID_STRIDE(i, n)
-    {
-        const bool task = lv.state[i] != kSkip;
-        lv.noff[i] = 0;
-        lv.ooff[i] = 0;
-        lv.task[i] = uint32_t(i);
-        const uint32_t k = (task && lv.res[i] != kInvalid) ? lv.cnt[i] : 0;
-        len[i] = k;
-        pieces[i] = (k + kPieceColors - 1) / kPieceColors;
-    }
 }
 
 // Offsets of the children of descended entries (levels T .. leaf - 1).
@@ -783,15 +917,26 @@ HD_D uint64_t new_color(const Editor& e, float px, float py, float pz, bool prev
     return single_color(e.sphere() ? F3{1, 0, 0} : F3{1, 0, 1});
 }
 
-// Emission of one level's colours into out[base[task] + offset ...]; a warp
-// per entry.
-__global__ void k_col_emit(Table t, ColorTable ct, Editor ed, uint32_t level, uint32_t n, Level lv, Level lvT,
+// Emission of the colours of levels T .. deepest into out[base[task] + offset
+// ...]; a warp per entry, all levels in one launch.
+struct EmitLevels {
+    Level lv[HD_MAX_DEPTH];
+    uint64_t end[HD_MAX_DEPTH]; // entries up to and including the level
+    uint32_t T;
+};
+__global__ void k_col_emit(Table t, ColorTable ct, Editor ed, __grid_constant__ const EmitLevels levels, uint64_t n,
                            const uint64_t* __restrict__ base, uint64_t* out)
 {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t D = t.g.depth, leafl = t.g.leaf_level;
+    const uint32_t leafl = t.g.leaf_level;
+    const Level& lvT = levels.lv[levels.T];
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x / 32);
-    for (uint64_t i = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; i < n; i += warps) {
+    for (uint64_t j = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; j < n; j += warps) {
+        uint32_t level = levels.T;
+        while (j >= levels.end[level])
+            level++;
+        const Level& lv = levels.lv[level];
+        const uint64_t i = level == levels.T ? j : j - levels.end[level - 1];
         const uint8_t st = lv.state[i];
         if (st == kSkip || st == kEmptied || st == kDescend)
             continue;
@@ -835,7 +980,6 @@ __global__ void k_col_emit(Table t, ColorTable ct, Editor ed, uint32_t level, ui
                 dst[popc64(newmask & (bit - 1))] = se ? new_color(ed, px, py, pz, prev, true, prev_col) : prev_col;
             }
         }
-        (void)D;
     }
 }
 
@@ -913,19 +1057,87 @@ __global__ void __launch_bounds__(256) k_col_count(uint32_t n, uint32_t n_pieces
     }
 }
 
-// Each task's macro words, weight words and whether it needs a new slot (one
-// with colours and without a unique leaf of its own).  bits_before: the bits
-// before each piece, modulo 2^32 (a task has fewer).
-__global__ void k_col_sizes(uint32_t n, Level lvT, const uint32_t* __restrict__ first,
-                            const uint64_t* __restrict__ len, const uint32_t* __restrict__ bits_before, uint32_t* nm,
-                            uint32_t* nw, uint32_t* need_new)
+// The pieces' sums: blocks and bits before each piece (bits modulo 2^32; a task
+// has fewer).  Then each task's macro and weight words and where they begin,
+// its rank among the tasks that need a new slot (with colours and without a
+// unique leaf of their own) and among those with colours.  One block.
+__global__ void __launch_bounds__(kTreeThreads)
+    k_col_sizes(uint32_t n, uint32_t n_pieces, Level lvT, const uint32_t* __restrict__ first,
+                const uint64_t* __restrict__ len, const uint32_t* __restrict__ piece_blocks,
+                const uint32_t* __restrict__ piece_bits, uint32_t* blocks_before, uint32_t* bits_before, uint32_t* nm,
+                uint32_t* nw, uint32_t* mo, uint32_t* wo, uint32_t* need_new, uint32_t* rank, uint32_t* row,
+                ColHead* head)
 {
-    HD_GRID_STRIDE(i, n)
-    {
-        const uint32_t bits = bits_before[first[i + 1]] - bits_before[first[i]];
-        nm[i] = uint32_t(2 * ((len[i] + kColorsPerMacro - 1) / kColorsPerMacro));
-        nw[i] = uint32_t((uint64_t(bits) + 31) / 32);
-        need_new[i] = len[i] > 0 && !(lvT.cn[i] & kLeafFlag);
+    using Pair = Two<uint32_t, uint32_t>;
+    __shared__ Pair sums[33];
+    constexpr uint32_t kPieces = 8;
+    Pair done{0, 0};
+    for (uint64_t p0 = 0; p0 < n_pieces; p0 += kTreeThreads * kPieces) {
+        Pair v[kPieces], mine{0, 0}, total;
+#pragma unroll
+        for (uint32_t j = 0; j < kPieces; j++) {
+            const uint64_t p = p0 + threadIdx.x * kPieces + j;
+            v[j] = p < n_pieces ? Pair{piece_blocks[p], piece_bits[p]} : Pair{0, 0};
+            mine.a += v[j].a;
+            mine.b += v[j].b;
+        }
+        Pair at = block_scan(mine, total, sums);
+        at.a += done.a;
+        at.b += done.b;
+#pragma unroll
+        for (uint32_t j = 0; j < kPieces; j++) {
+            const uint64_t p = p0 + threadIdx.x * kPieces + j;
+            if (p < n_pieces) {
+                blocks_before[p] = at.a;
+                bits_before[p] = at.b;
+            }
+            at.a += v[j].a;
+            at.b += v[j].b;
+        }
+        done.a += total.a;
+        done.b += total.b;
+    }
+    if (threadIdx.x == 0) {
+        blocks_before[n_pieces] = done.a;
+        bits_before[n_pieces] = done.b;
+    }
+    __syncthreads();
+    Pair words{0, 0}, slots{0, 0};
+    for (uint32_t i0 = 0; i0 < n; i0 += kTreeThreads) {
+        const uint32_t i = i0 + threadIdx.x;
+        Pair w{0, 0}, r{0, 0}, total;
+        if (i < n) {
+            const uint64_t L = len[i];
+            const uint32_t bits = bits_before[first[i + 1]] - bits_before[first[i]];
+            w.a = uint32_t(2 * ((L + kColorsPerMacro - 1) / kColorsPerMacro));
+            w.b = uint32_t((uint64_t(bits) + 31) / 32);
+            r.a = L > 0 && !(lvT.cn[i] & kLeafFlag);
+            r.b = L > 0;
+        }
+        const Pair wa = block_scan(w, total, sums);
+        if (i < n) {
+            nm[i] = w.a;
+            nw[i] = w.b;
+            mo[i] = words.a + wa.a;
+            wo[i] = words.b + wa.b;
+        }
+        words.a += total.a;
+        words.b += total.b;
+        const Pair ra = block_scan(r, total, sums);
+        if (i < n) {
+            need_new[i] = r.a;
+            rank[i] = slots.a + ra.a;
+            row[i] = slots.b + ra.b;
+        }
+        slots.a += total.a;
+        slots.b += total.b;
+    }
+    if (threadIdx.x == 0) {
+        head->blocks = done.a;
+        head->macro_words = words.a;
+        head->weight_words = words.b;
+        head->new_slots = slots.a;
+        head->replaced = slots.b;
     }
 }
 
@@ -998,82 +1210,101 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Descriptors in place; new slots get leaf indices leaf_top + rank; the
-// replaced descriptors go to the undo diff.
-__global__ void k_col_commit(ColorTable ct, uint32_t n, Level lvT, const uint64_t* __restrict__ len,
-                             const uint32_t* __restrict__ need_new, const uint32_t* __restrict__ rank,
-                             uint64_t leaf_top, const LeafDesc* __restrict__ desc, uint32_t* slot_out,
-                             LeafDesc* prev_out)
+// Descriptors in place: new slots get leaf indices leaf_top + rank, the
+// replaced descriptors go to the undo diff.  Then, bottom-up, colour nodes
+// (edit_threaded's allocateColorNode, hash_dag_edits.h:152-161): an entry
+// above T whose child got a new leaf or node and that has no colour node
+// gets one; and the links to what is new.  One block.
+struct ColTops {
+    uint64_t node, leaf, block, macro, weight;
+};
+__global__ void __launch_bounds__(kTreeThreads)
+    k_col_up(ColorTable ct, __grid_constant__ const Tree tree, const uint64_t* __restrict__ len,
+             const uint32_t* __restrict__ rank, const uint32_t* __restrict__ row,
+             const LeafDesc* __restrict__ desc, ColTops tops, ColHead* head, Replaced* replaced)
 {
-    HD_GRID_STRIDE(i, n)
+    __shared__ Two<uint32_t, uint32_t> sums[33];
+    const uint32_t T = tree.T;
     {
-        if (!len[i])
-            continue;
-        uint32_t slot = lvT.cn[i];
-        LeafDesc prev{};
-        if (need_new[i]) {
-            slot = kLeafFlag | uint32_t(leaf_top + rank[i]);
-            lvT.cn[i] = slot; // linked into the tree below
-        } else {
-            prev = ct.leaves[slot & ~kLeafFlag];
+        const TreeLevel& lv = tree.lv[T];
+#pragma unroll 2
+        for (uint32_t i = threadIdx.x; i < lv.n; i += kTreeThreads) {
+            if (!len[i])
+                continue;
+            uint32_t slot = lv.cn[i];
+            LeafDesc prev{};
+            if (lv.newnode[i]) {
+                slot = kLeafFlag | uint32_t(tops.leaf + rank[i]);
+                lv.cn[i] = slot; // linked into the tree below
+            } else {
+                prev = ct.leaves[slot & ~kLeafFlag];
+            }
+            const LeafDesc next = desc[i];
+            ct.leaves[slot & ~kLeafFlag] = next;
+            Replaced& r = replaced[row[i]];
+            r.prev = prev;
+            r.next = next;
+            r.leaf = slot & ~kLeafFlag;
         }
-        ct.leaves[slot & ~kLeafFlag] = desc[i];
-        slot_out[i] = slot;
-        prev_out[i] = prev;
     }
-}
-
-// Bottom-up colour-node allocation (edit_threaded's allocateColorNode,
-// hash_dag_edits.h:152-161): an entry above T whose child got a new leaf or
-// node and that has no colour node gets one.
-__global__ void k_col_need(uint32_t level, uint32_t T, uint32_t n, Level lv, Level next,
-                           const uint32_t* __restrict__ need_new_T, const uint32_t* __restrict__ newnode_next,
-                           uint32_t* newnode)
-{
-    HD_GRID_STRIDE(i, n)
-    {
-        bool any = false;
-        if (lv.flag[i]) {
-            const uint32_t base = 8 * lv.exp[i];
+    uint64_t node_top = tops.node;
+    for (uint32_t L = T - 1; L >= 1; L--) {
+        __syncthreads();
+        const TreeLevel& lv = tree.lv[L];
+        const uint32_t* below = tree.lv[L + 1].newnode;
+        for (uint32_t i0 = 0; i0 < lv.n; i0 += kTreeThreads) {
+            const uint32_t i = i0 + threadIdx.x;
+            bool any = false;
+            if (i < lv.n && lv.flag[i]) {
+                const uint32_t base = 8 * lv.exp[i];
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++)
+                    any |= below[base + k] != 0;
+            }
+            const bool add = any && lv.cn[i] == 0;
+            Two<uint32_t, uint32_t> total;
+            const uint32_t at = block_scan(Two<uint32_t, uint32_t>{add ? 1u : 0u, 0u}, total, sums).a;
+            if (i < lv.n)
+                lv.newnode[i] = add;
+            if (add)
+                lv.cn[i] = uint32_t(node_top + 8ull * at);
+            node_top += 8ull * total.a;
+        }
+    }
+    __syncthreads();
+    for (uint32_t L = 0; L < T; L++) {
+        const TreeLevel &lv = tree.lv[L], &next = tree.lv[L + 1];
+#pragma unroll 2
+        for (uint32_t i = threadIdx.x; i < lv.n; i += kTreeThreads) {
+            if (!lv.flag[i])
+                continue;
+            const uint32_t base = 8 * lv.exp[i], cn = lv.cn[i];
+#pragma unroll
             for (uint32_t k = 0; k < 8; k++)
-                any |= (level + 1 == T) ? need_new_T[base + k] != 0 : newnode_next[base + k] != 0;
+                if (next.newnode[base + k])
+                    ct.nodes[cn + k] = next.cn[base + k];
         }
-        newnode[i] = any && level > 0 && lv.cn[i] == 0;
     }
-}
-__global__ void k_col_alloc(uint32_t n, Level lv, const uint32_t* __restrict__ newnode, const uint32_t* __restrict__ rank,
-                            uint64_t node_top)
-{
-    HD_GRID_STRIDE(i, n)
-    {
-        if (newnode[i])
-            lv.cn[i] = uint32_t(node_top + 8ull * rank[i]);
-    }
-}
-__global__ void k_col_link(ColorTable ct, uint32_t level, uint32_t T, uint32_t n, Level lv, Level next,
-                           const uint32_t* __restrict__ need_new_T, const uint32_t* __restrict__ newnode_next)
-{
-    HD_GRID_STRIDE(i, n)
-    {
-        if (!lv.flag[i])
-            continue;
-        const uint32_t base = 8 * lv.exp[i];
-        for (uint32_t k = 0; k < 8; k++) {
-            const bool link = (level + 1 == T) ? need_new_T[base + k] != 0 : newnode_next[base + k] != 0;
-            if (link)
-                ct.nodes[lv.cn[i] + k] = next.cn[base + k];
-        }
+    if (threadIdx.x == 0) {
+        ct.top[0] = head->node_top = node_top;
+        ct.top[1] = tops.leaf + head->new_slots;
+        ct.top[2] = tops.block + head->blocks;
+        ct.top[3] = tops.macro + head->macro_words;
+        ct.top[4] = tops.weight + head->weight_words;
     }
 }
 
 // The colour phase of an edit, after its geometry: lv / count / deepest as
-// edit_one left them (levels T .. deepest hold the tasks' subtrees).  Fills
-// frame (replaced leaves) for the undo history.
+// edit_one left them (levels T .. deepest hold the tasks' subtrees; spawned:
+// with the colour nodes of the levels down to T).  Its last results are on
+// their way to the host when it returns: the caller waits for the stream and
+// calls edit_colors_done.
 void edit_colors(hd_ctx* c, const Editor& ed, std::vector<Level>& lv, const std::vector<uint32_t>& count,
-                 uint32_t deepest, UndoFrame& frame)
+                 uint32_t deepest, bool spawned, ColorsBack& back)
 {
     const Geom& g = c->g;
     const uint32_t T = g.T;
+    back.bytes.clear();
     if (!c->colors || deepest < T || count[T] == 0)
         return;
     cudaStream_t st = c->stream;
@@ -1081,116 +1312,99 @@ void edit_colors(hd_ctx* c, const Editor& ed, std::vector<Level>& lv, const std:
     const uint32_t nT = count[T];
     uint64_t* len = s.get<uint64_t>("ec_len", uint64_t(nT) + 1);
     uint64_t* base = s.get<uint64_t>("ec_base", uint64_t(nT) + 1);
-    uint64_t* d_tot64 = s.get<uint64_t>("ec_tot64", 2);
-    uint32_t* pieces = s.get<uint32_t>("ec_pieces", uint64_t(nT) + 1);
     uint32_t* first = s.get<uint32_t>("ec_first", uint64_t(nT) + 1); // each task's first piece, then their number
-    k_col_tasks<<<grid_for(nT, 256), 256, 0, st>>>(nT, lv[T], len, pieces);
+    uint32_t* need_new = s.get<uint32_t>("ec_neednew", uint64_t(nT) + 1);
+    // the head, the replaced leaves behind it
+    uint8_t* d_back = s.get<uint8_t>("ec_back", sizeof(ColHead) + sizeof(Replaced) * (uint64_t(nT) + 1));
+    static_assert(sizeof(ColHead) % 16 == 0 && sizeof(Replaced) % 16 == 0, "aligned");
+    ColHead* head = reinterpret_cast<ColHead*>(d_back);
+    Replaced* replaced = reinterpret_cast<Replaced*>(d_back + sizeof(ColHead));
+    uint64_t above = 0;
+    for (uint32_t L = 0; L < T; L++)
+        above += count[L];
+    uint32_t* newnode = s.get<uint32_t>("ec_newnode", above + 1);
+    Tree tree{};
+    tree.T = T;
+    for (uint32_t L = 0; L <= T; L++) {
+        tree.lv[L] = {lv[L].flag, lv[L].exp, lv[L].cn, L < T ? newnode : need_new, count[L]};
+        newnode += count[L];
+    }
+    k_col_down<<<1, kTreeThreads, 0, st>>>(c->ct, tree, lv[T], !spawned, len, base, first, head);
     HD_LAUNCH_CHECK();
     for (uint32_t L = T; L < deepest; L++) {
         k_col_offsets<<<grid_for(count[L], 256), 256, 0, st>>>(count[L], lv[L], lv[L + 1]);
         HD_LAUNCH_CHECK();
     }
-    exclusive_scan<uint64_t, uint64_t>(s, len, base, nT, d_tot64, st);
-    exclusive_scan<uint32_t, uint32_t>(s, pieces, first, nT, first + nT, st);
-    uint32_t n_pieces = 0;
-    HD_CUDA(cudaMemcpyAsync(&n_pieces, first + nT, 4, cudaMemcpyDeviceToHost, st));
-    const uint64_t total = read_scalar(d_tot64, st);
-    uint64_t* out = s.get<uint64_t>("ec_out", total + 1);
+    ColHead h = read_scalar(head, st);
+    const uint32_t n_pieces = h.pieces;
+    uint64_t* out = s.get<uint64_t>("ec_out", h.total + 1);
+    EmitLevels emit{};
+    emit.T = T;
+    uint64_t entries = 0;
     for (uint32_t L = T; L <= deepest; L++) {
-        const uint64_t threads = uint64_t(count[L]) * 32;
-        k_col_emit<<<grid_for(threads, 256, 152 * 16), 256, 0, st>>>(c->t, c->ct, ed, L, count[L], lv[L], lv[T], base,
-                                                                     out);
-        HD_LAUNCH_CHECK();
+        emit.lv[L] = lv[L];
+        emit.end[L] = entries += count[L];
     }
+    k_col_emit<<<grid_for(entries * 32, 256, 152 * 16), 256, 0, st>>>(c->t, c->ct, ed, emit, entries, base, out);
+    HD_LAUNCH_CHECK();
     uint32_t* nm = s.get<uint32_t>("ec_nm", uint64_t(nT) + 1);
     uint32_t* nw = s.get<uint32_t>("ec_nw", uint64_t(nT) + 1);
     uint32_t* mo = s.get<uint32_t>("ec_mo", uint64_t(nT) + 1);
     uint32_t* wo = s.get<uint32_t>("ec_wo", uint64_t(nT) + 1);
-    uint32_t* need_new = s.get<uint32_t>("ec_neednew", uint64_t(nT) + 1);
     uint32_t* rank = s.get<uint32_t>("ec_rank", uint64_t(nT) + 1);
+    uint32_t* row = s.get<uint32_t>("ec_row", uint64_t(nT) + 1);
     uint32_t* piece_blocks = s.get<uint32_t>("ec_piece_blocks", uint64_t(n_pieces) + 1);
     uint32_t* piece_bits = s.get<uint32_t>("ec_piece_bits", uint64_t(n_pieces) + 1);
     uint32_t* blocks_before = s.get<uint32_t>("ec_blocks_before", uint64_t(n_pieces) + 1);
     uint32_t* bits_before = s.get<uint32_t>("ec_bits_before", uint64_t(n_pieces) + 1);
-    uint32_t* d_tot = s.get<uint32_t>("ec_tot", 4);
     const uint32_t piece_grid = grid_for(uint64_t(n_pieces) * 32, 256, 152 * 16);
     k_col_count<<<piece_grid, 256, 0, st>>>(nT, n_pieces, first, len, base, out, piece_blocks, piece_bits);
     HD_LAUNCH_CHECK();
-    exclusive_scan<uint32_t, uint32_t>(s, piece_blocks, blocks_before, n_pieces, blocks_before + n_pieces, st);
-    exclusive_scan<uint32_t, uint32_t>(s, piece_bits, bits_before, n_pieces, bits_before + n_pieces, st);
-    k_col_sizes<<<grid_for(nT, 256), 256, 0, st>>>(nT, lv[T], first, len, bits_before, nm, nw, need_new);
+    k_col_sizes<<<1, kTreeThreads, 0, st>>>(nT, n_pieces, lv[T], first, len, piece_blocks, piece_bits, blocks_before,
+                                            bits_before, nm, nw, mo, wo, need_new, rank, row, head);
     HD_LAUNCH_CHECK();
-    exclusive_scan<uint32_t, uint32_t>(s, nm, mo, nT, d_tot + 1, st);
-    exclusive_scan<uint32_t, uint32_t>(s, nw, wo, nT, d_tot + 2, st);
-    exclusive_scan<uint32_t, uint32_t>(s, need_new, rank, nT, d_tot + 3, st);
-    HD_CUDA(cudaMemcpyAsync(d_tot, blocks_before + n_pieces, 4, cudaMemcpyDeviceToDevice, st));
-    uint32_t tot[4];
-    HD_CUDA(cudaMemcpyAsync(tot, d_tot, 16, cudaMemcpyDeviceToHost, st));
-    HD_CUDA(cudaStreamSynchronize(st));
-    const uint32_t need_new_total = tot[3];
+    h = read_scalar(head, st);
     // renders in flight read the leaves about to be replaced: wait for them
     for (cudaEvent_t e : c->color_fences)
         HD_CUDA(cudaStreamWaitEvent(st, e, 0));
     // nodes: at most one per entry above T
-    uint64_t max_nodes = 0;
-    for (uint32_t L = 1; L < T; L++)
-        max_nodes += 8ull * count[L];
-    const uint64_t add[5] = {max_nodes, need_new_total, tot[0], tot[1], tot[2]};
+    const uint64_t add[5] = {8 * (above - count[0]), h.new_slots, h.blocks, h.macro_words, h.weight_words};
     color_reserve(c, add);
     LeafDesc* desc = s.get<LeafDesc>("ec_desc", uint64_t(nT) + 1);
     k_col_pack<<<piece_grid, 256, 0, st>>>(c->ct, nT, n_pieces, first, len, base, out, blocks_before, bits_before, nm, nw,
                                            mo, wo, c->ctop[2], c->ctop[3], c->ctop[4], desc);
     HD_LAUNCH_CHECK();
-    uint32_t* slot_out = s.get<uint32_t>("ec_slot", uint64_t(nT) + 1);
-    LeafDesc* prev_out = s.get<LeafDesc>("ec_prev", uint64_t(nT) + 1);
-    k_col_commit<<<grid_for(nT, 256), 256, 0, st>>>(c->ct, nT, lv[T], len, need_new, rank, c->ctop[1], desc,
-                                                    slot_out, prev_out);
+    k_col_up<<<1, kTreeThreads, 0, st>>>(c->ct, tree, len, rank, row, desc,
+                                         ColTops{c->ctop[0], c->ctop[1], c->ctop[2], c->ctop[3], c->ctop[4]}, head,
+                                         replaced);
     HD_LAUNCH_CHECK();
-    // colour nodes, bottom-up, then the links
-    std::vector<uint32_t*> newnode(T + 1, nullptr);
-    newnode[T] = need_new;
-    uint64_t node_top = c->ctop[0];
-    for (uint32_t L = T - 1; L >= 1; L--) {
-        char nm_[32];
-        snprintf(nm_, sizeof(nm_), "ec_newnode_%u", L);
-        newnode[L] = s.get<uint32_t>(nm_, uint64_t(count[L]) + 1);
-        k_col_need<<<grid_for(count[L], 256), 256, 0, st>>>(L, T, count[L], lv[L], lv[L + 1], need_new,
-                                                            newnode[L + 1], newnode[L]);
-        HD_LAUNCH_CHECK();
-        uint32_t* r = s.get<uint32_t>("ec_noderank", uint64_t(count[L]) + 1);
-        exclusive_scan<uint32_t, uint32_t>(s, newnode[L], r, count[L], d_tot, st);
-        const uint32_t k = read_scalar(d_tot, st);
-        k_col_alloc<<<grid_for(count[L], 256), 256, 0, st>>>(count[L], lv[L], newnode[L], r, node_top);
-        HD_LAUNCH_CHECK();
-        node_top += 8ull * k;
+    back.bytes.resize(sizeof(ColHead) + sizeof(Replaced) * h.replaced);
+    HD_CUDA(cudaMemcpyAsync(back.bytes.data(), d_back, back.bytes.size(), cudaMemcpyDeviceToHost, st));
+}
+
+// After the stream has been waited for: the pools' new tops, and the replaced
+// leaves (a new slot had no leaf: an empty descriptor) for the undo history.
+void edit_colors_done(hd_ctx* c, const ColorsBack& back, UndoFrame& frame)
+{
+    if (back.bytes.empty())
+        return;
+    ColHead h;
+    std::memcpy(&h, back.bytes.data(), sizeof(h));
+    c->ctop[0] = h.node_top;
+    c->ctop[1] += h.new_slots;
+    c->ctop[2] += h.blocks;
+    c->ctop[3] += h.macro_words;
+    c->ctop[4] += h.weight_words;
+    frame.leaf.reserve(h.replaced);
+    frame.prev.reserve(h.replaced);
+    frame.next.reserve(h.replaced);
+    for (uint32_t i = 0; i < h.replaced; i++) {
+        Replaced r;
+        std::memcpy(&r, back.bytes.data() + sizeof(ColHead) + sizeof(Replaced) * i, sizeof(r));
+        frame.leaf.push_back(r.leaf);
+        frame.prev.push_back(r.prev);
+        frame.next.push_back(r.next);
     }
-    for (uint32_t L = 0; L < T; L++) {
-        k_col_link<<<grid_for(count[L], 256), 256, 0, st>>>(c->ct, L, T, count[L], lv[L], lv[L + 1], need_new,
-                                                            newnode[L + 1]);
-        HD_LAUNCH_CHECK();
-    }
-    c->ctop[0] = node_top;
-    c->ctop[1] += need_new_total;
-    c->ctop[2] += tot[0];
-    c->ctop[3] += tot[1];
-    c->ctop[4] += tot[2];
-    const unsigned long long tops[5] = {c->ctop[0], c->ctop[1], c->ctop[2], c->ctop[3], c->ctop[4]};
-    HD_CUDA(cudaMemcpyAsync(c->ct.top, tops, sizeof(tops), cudaMemcpyHostToDevice, st));
-    // undo diff: replaced leaves (new slots had no leaf: an empty descriptor)
-    std::vector<uint64_t> h_len(nT);
-    std::vector<uint32_t> h_slot(nT);
-    std::vector<LeafDesc> h_prev(nT), h_next(nT);
-    HD_CUDA(cudaMemcpyAsync(h_len.data(), len, 8ull * nT, cudaMemcpyDeviceToHost, st));
-    HD_CUDA(cudaMemcpyAsync(h_slot.data(), slot_out, 4ull * nT, cudaMemcpyDeviceToHost, st));
-    HD_CUDA(cudaMemcpyAsync(h_prev.data(), prev_out, sizeof(LeafDesc) * nT, cudaMemcpyDeviceToHost, st));
-    HD_CUDA(cudaMemcpyAsync(h_next.data(), desc, sizeof(LeafDesc) * nT, cudaMemcpyDeviceToHost, st));
-    HD_CUDA(cudaStreamSynchronize(st));
-    for (uint32_t i = 0; i < nT; i++)
-        if (h_len[i]) {
-            frame.leaf.push_back(h_slot[i] & ~kLeafFlag);
-            frame.prev.push_back(h_prev[i]);
-            frame.next.push_back(h_next[i]);
-        }
 }
 
 __global__ void k_set_leaves(ColorTable ct, const uint32_t* __restrict__ index, const LeafDesc* __restrict__ d,

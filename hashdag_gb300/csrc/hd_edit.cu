@@ -184,13 +184,12 @@ void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
         return edit_by_levels(c, e, stats);
     if (c->colors) {
         std::vector<Level> lv(pl->lv);
-        HD_CUDA(cudaMemsetAsync(lv[0].cn, 0, 4, st));
-        for (uint32_t L = 0; L < geo.deepest && L < c->g.T; L++)
-            color_spawn(c, L, geo.count[L], lv[L], lv[L + 1]);
-        edit_colors(c, ed, lv, geo.count, geo.deepest, frame);
+        ColorsBack back;
+        edit_colors(c, ed, lv, geo.count, geo.deepest, false, back);
         HD_CUDA(cudaMemcpyAsync(c->d_root, lv[0].res, 4, cudaMemcpyDeviceToDevice, st));
         HD_CUDA(cudaEventRecord(c->ev1, st));
         HD_CUDA(cudaStreamSynchronize(st));
+        edit_colors_done(c, back, frame);
     }
     c->root = geo.root;
     push_undo(c, std::move(frame));
@@ -281,14 +280,16 @@ void edit_by_levels(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
             c->t, uint32_t(L), lv[L], keys, vals, starts, d_cnt + 1, d_cnt, ctr);
         HD_LAUNCH_CHECK();
     }
+    ColorsBack back;
     if (colors && !check_error_peek(c))
-        edit_colors(c, ed, lv, count, deepest, frame);
+        edit_colors(c, ed, lv, count, deepest, true, back);
     k_edit_finish<<<1, 1, 0, st>>>(lv[0], c->d_root, c->t.error);
     HD_LAUNCH_CHECK();
     HD_CUDA(cudaEventRecord(c->ev1, st));
     EditCounters h{};
     HD_CUDA(cudaMemcpyAsync(&h, ctr, sizeof(h), cudaMemcpyDeviceToHost, st));
     HD_CUDA(cudaStreamSynchronize(st));
+    edit_colors_done(c, back, frame);
     const uint32_t err = check_error(c);
     if (err)
         throw StatusError{err == kErrCapacity ? HD_ERR_STATE : hd_status(err),

@@ -43,3 +43,39 @@ def test_packed_leaves_match_oracle(gpu, radius):
     assert [tuple(int(v) for v in row) for row in d.get_colors(pts)] == \
         [tuple(col.get_color(*(int(v) for v in p))) for p in pts]
     d.free()
+
+
+def test_many_tasks_match_oracle(gpu):
+    """A paint over most of a 2^11 scene: thousands of tasks, over 2^13 pieces."""
+    depth = 11
+    T = workloads.color_tree_levels(depth)
+    words = po.generate_basic_dag(workloads.SEED_SCENE, depth, T, flags=po.SCENE_SHELL)
+    ot = po.Table(po.default_config(depth, T))
+    ot.load_basic_dag(words)
+    col = po.Colors(ot)
+    col.from_scene(workloads.SEED_COLORS)
+    d = hd.HashDAG(depth)
+    d.load_from_DAG(words)
+    d.colors_from_scene(workloads.SEED_COLORS)
+    rng = np.random.default_rng(9)
+    s = scene.surface_points(workloads.SEED_SCENE, depth, 3000, rng)
+    c = tuple(float(v) + 0.5 for v in s[np.argsort(np.abs(s - 1024.0).sum(axis=1))][0])
+    got = d.edit_threads(hd.SpherePaintEditor(c, 800.0, 0x40A0F0))
+    want = col.edit(4, c, 800.0, rgb=0x40A0F0)
+    assert d.firstNodeIndex == ot.root
+    assert (got.num_voxels, got.num_nodes) == (want.num_voxels, want.num_nodes)
+    assert got.num_voxels > 256 * 8192
+    pts = s.astype(np.uint32)
+    pts = pts[d.get_values(pts) != 0]
+    assert len(pts) > 100
+
+    def colours():
+        return [tuple(int(v) for v in row) for row in d.get_colors(pts)]
+
+    painted = colours()
+    assert painted == [tuple(col.get_color(*(int(v) for v in p))) for p in pts]
+    d.undo()
+    assert colours() != painted
+    d.redo()
+    assert colours() == painted
+    d.free()
