@@ -24,6 +24,7 @@ struct hd_ctx {
     hd_config cfg{};
     hd::Geom g{};
     hd::Table t{};           // device pointers of the table
+    void* d_arrays = nullptr; // the allocation behind all of them but pool and meta
     cudaStream_t stream = nullptr;
     uint32_t* d_root = nullptr;        // firstNodeIndex on the device
     uint32_t root = 0;                 // host copy, refreshed after each call
