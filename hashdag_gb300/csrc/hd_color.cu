@@ -846,23 +846,36 @@ void color_spawn(hd_ctx* c, uint32_t level, uint32_t n, const Level& lv, const L
     HD_LAUNCH_CHECK();
 }
 
-// Offsets of the children of descended entries (levels T .. leaf - 1).
+// Offsets of the children of descended entries (levels T .. leaf - 1), a
+// thread per child.
 __global__ void k_col_offsets(uint32_t n, Level lv, Level next)
 {
-    HD_GRID_STRIDE(i, n)
-    {
-        if (lv.state[i] != kDescend)
-            continue;
-        const uint32_t base = 8 * lv.exp[i];
-        uint32_t no = lv.noff[i], oo = lv.ooff[i];
-        const uint32_t task = lv.task[i];
-        for (uint32_t k = 0; k < 8; k++) {
-            const uint32_t j = base + k;
-            next.noff[j] = no;
-            next.ooff[j] = oo;
-            next.task[j] = task;
-            no += next.res[j] != kInvalid ? next.cnt[j] : 0u;
-            oo += next.ocnt[j];
+    const uint32_t k = threadIdx.x & 7;
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    // whole warps stay in the loop (n8: 8 n, up to the next multiple of 32)
+    const uint64_t n8 = (8ull * n + 31) & ~31ull;
+    for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < n8; e += stride) {
+        const uint64_t i = e >> 3;
+        const bool on = i < n && lv.state[i] == kDescend;
+        uint32_t j = 0, cnt = 0, old = 0;
+        if (on) {
+            j = 8 * lv.exp[i] + k;
+            cnt = next.res[j] != kInvalid ? next.cnt[j] : 0u;
+            old = next.ocnt[j];
+        }
+        uint32_t c = cnt, o = old; // sums up to this child
+#pragma unroll
+        for (uint32_t s = 1; s < 8; s <<= 1) {
+            const uint32_t cu = __shfl_up_sync(0xffffffffu, c, s, 8), ou = __shfl_up_sync(0xffffffffu, o, s, 8);
+            if (k >= s) {
+                c += cu;
+                o += ou;
+            }
+        }
+        if (on) {
+            next.noff[j] = lv.noff[i] + c - cnt;
+            next.ooff[j] = lv.ooff[i] + o - old;
+            next.task[j] = lv.task[i];
         }
     }
 }
@@ -1262,10 +1275,12 @@ __global__ void __launch_bounds__(kTreeThreads)
                     any |= below[base + k] != 0;
             }
             const bool add = any && lv.cn[i] == 0;
-            Two<uint32_t, uint32_t> total;
-            const uint32_t at = block_scan(Two<uint32_t, uint32_t>{add ? 1u : 0u, 0u}, total, sums).a;
             if (i < lv.n)
                 lv.newnode[i] = add;
+            if (!__syncthreads_or(add))
+                continue; // nothing new, as in most edits of coloured places
+            Two<uint32_t, uint32_t> total;
+            const uint32_t at = block_scan(Two<uint32_t, uint32_t>{add ? 1u : 0u, 0u}, total, sums).a;
             if (add)
                 lv.cn[i] = uint32_t(node_top + 8ull * at);
             node_top += 8ull * total.a;
@@ -1332,7 +1347,7 @@ void edit_colors(hd_ctx* c, const Editor& ed, std::vector<Level>& lv, const std:
     k_col_down<<<1, kTreeThreads, 0, st>>>(c->ct, tree, lv[T], !spawned, len, base, first, head);
     HD_LAUNCH_CHECK();
     for (uint32_t L = T; L < deepest; L++) {
-        k_col_offsets<<<grid_for(count[L], 256), 256, 0, st>>>(count[L], lv[L], lv[L + 1]);
+        k_col_offsets<<<grid_for(8ull * count[L], 256), 256, 0, st>>>(count[L], lv[L], lv[L + 1]);
         HD_LAUNCH_CHECK();
     }
     ColHead h = read_scalar(head, st);
