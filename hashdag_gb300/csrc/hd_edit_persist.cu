@@ -13,14 +13,16 @@
 //    processed by CTA 0 alone while the other CTAs wait at the next grid
 //    barrier: consecutive small levels, the end of one edit and the start of
 //    the next cost one barrier in all, or none when no grid step came
-//    between.  A bottom-up small level whose candidates fall in more than
-//    kLocalRuns buckets hands its find-or-add to the whole grid.
+//    between (bottom-up, where an entry costs more: kSmallUp entries).
 //  * A big level top-down is one grid phase: each CTA finds the descended
 //    entries of its share of the children (per-chunk counts of descend flags
 //    were gathered while the level was classified), spawns and classifies
 //    them.
-//  * A big level bottom-up is four phases: candidates with their pass-1 digit
-//    counts, two stable radix passes on the level-local bucket (each CTA sums
+//  * A big level bottom-up is two phases: candidates, each put in the queue of
+//    the CTA that owns its bucket (bucket modulo CTAs), then every CTA sorts
+//    its queue and resolves its bucket runs, a warp each.  When a queue
+//    overflows (many candidates of few buckets: a box's faces), it is four:
+//    two stable radix passes on the level-local bucket (each CTA sums
 //    the digit counts itself; pass-2 counts gathered while pass 1 scatters),
 //    then find-or-add, one warp per bucket run; from kRepeatLevel candidates
 //    on, the repeats and the runs' starts are marked before it.
@@ -41,11 +43,15 @@ namespace {
 
 constexpr uint32_t kPT = 1024;             // threads per CTA (one CTA per SM)
 constexpr uint32_t kPWarps = kPT / 32;
-constexpr uint32_t kSmall = kPT;           // entries of a level CTA 0 handles alone
+// Entries of a level that CTA 0 handles alone, top-down and bottom-up: a grid
+// step costs a barrier (2.4-3.5 us), CTA 0 alone 4 us a level of 200 entries and
+// 27 us bottom-up at 1,000 (its 32 warps resolve a bucket run in 1.5-2.5 us).
+// Batches of 64 edits of radius 4-48 at 2^12 and 8-512 at 2^15: bottom-up limits
+// of 128, 256, 512 and 1,024 give 5.78, 5.69, 5.72, 5.80 and 13.4, 13.4, 13.5,
+// 13.7 ms; top-down ones of 256, 512 and 1,024 5.70, 5.68, 5.71 and 13.2, 13.1,
+// 13.2 ms.
+constexpr uint32_t kSmall = 512, kSmallUp = 256;
 constexpr uint32_t kDigits = 512;          // radix digits per pass at most (9 bits)
-// Bucket runs of a small level that CTA 0's warps resolve themselves (four
-// each, about 1.5 us a run); more are worth the two barriers of a grid step.
-constexpr uint32_t kLocalRuns = 4 * kPWarps;
 // Candidates of a big level from which repeats are looked for (a grid step).
 constexpr uint32_t kRepeatLevel = 4096;
 constexpr unsigned long long kWaitNs = 2000000000ull;
@@ -73,7 +79,7 @@ struct Ctl {
     uint32_t phase;     // the grid step CTA 0 asks for (kPh*)
     uint32_t level;     // its level
     uint32_t deepest;   // deepest level of the current edit
-    uint32_t n_small_runs; // bucket runs of the small level handed to the grid
+    uint32_t pad;
     Cmd cmd[2];
     uint32_t ncand[HD_MAX_DEPTH]; // big levels: candidates for find-or-add
     uint32_t nruns[HD_MAX_DEPTH]; // big levels: long runs of repeats
@@ -110,6 +116,8 @@ struct PArgs {
     uint32_t cap[HD_MAX_DEPTH];
     uint32_t *keys, *vals, *keys2, *vals2;
     uint32_t* bsum;      // 3 x G: per-chunk descend-flag counts, by level parity
+    unsigned long long* queue; // G x kPT: bucket << 32 | entry of the candidates a CTA owns
+    uint32_t* queued;    // HD_MAX_DEPTH x G: their numbers, by level
     uint32_t *hist, *hist2; // G x kDigits: a big level's digit counts per chunk
     uint32_t *rows, *rows2; // kDigits: their totals
     uint32_t* same;      // a big level's repeats, a bit per sorted candidate
@@ -698,18 +706,17 @@ HD_D void fill_runs(const Level& lv, const uint32_t* vals, const FollowerRun* ru
     }
 }
 
-// CTA 0 alone: stable sort of the n (kTiny < n <= kPT) candidates of a small level by
-// (bucket, entry) in registers, one a thread: a bitonic network with lane
+// A CTA alone: sort of n <= kPT items x (bucket << 32 | entry, one a thread: the
+// candidates of a small level, or a queue of a big one's) in registers: a bitonic network with lane
 // shuffles, and shared memory for the steps across warps (two buffers, so
 // one barrier a step; a rank sort, n reads a thread, took 15.6 us at n = 784).
 // The sorted buckets and entries go to sk / sv, the starts of the bucket runs
 // to rs (one more: their end); returns the number of runs.
-HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, const uint32_t* keys, const uint32_t* vals,
-                         unsigned long long* s64, uint32_t* sm32, uint32_t* sk, uint32_t* sv, uint32_t* rs)
+HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, unsigned long long x, unsigned long long* s64,
+                         uint32_t* sm32, uint32_t* sk, uint32_t* sv, uint32_t* rs)
 {
     const uint32_t empty = t.g.buckets(L);
     const uint32_t i = threadIdx.x, lane = i & 31;
-    unsigned long long x = i < n ? (uint64_t(keys[i]) << 32) | vals[i] : ~0ull;
     auto keep = [&](unsigned long long y, uint32_t k, uint32_t j) {
         const bool up = (i & k) == 0, low = (i & j) == 0;
         x = (low == up) == (x < y) ? x : y;
@@ -881,7 +888,7 @@ HD_D void scatter_chunk(const uint32_t* keys, const uint32_t* vals, uint32_t n, 
 // CTA 0's state between grid steps
 enum : uint32_t { kLsBegin = 0, kLsTopDown = 1, kLsBottomUp = 2, kLsFinish = 3 };
 // the grid step CTA 0 asks for
-enum : uint32_t { kPhNone = 0, kPhTopDown = 1, kPhBottomUp = 2, kPhGridFoa = 3 };
+enum : uint32_t { kPhNone = 0, kPhTopDown = 1, kPhBottomUp = 2 };
 
 // Bytes of the dynamic shared memory the find-or-add buffers and the small
 // sort share (a multiple of 16); the small level's sorted keys and entries
@@ -942,6 +949,8 @@ HD_D bool begin_edit(const Table& t, const PArgs& a, const Smem& sm)
     }
     for (uint32_t k = threadIdx.x; k < 3 * G; k += kPT)
         a.bsum[k] = 0;
+    for (uint32_t k = threadIdx.x; k < (t.g.leaf_level + 1) * G; k += kPT)
+        a.queued[k] = 0;
     __syncthreads();
     if (sm.sm32[32] != kRun)
         return false;
@@ -1145,7 +1154,7 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
                     continue;
                 }
                 const uint32_t n = ts.count[L];
-                if (n > kSmall) {
+                if (n > kSmallUp) {
                     if (threadIdx.x == 0) {
                         ctl->phase = kPhBottomUp;
                         ctl->level = L;
@@ -1155,23 +1164,9 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
                 }
                 candidates_range(t, a.lv, L, deepest, 0, n, a.keys, a.vals);
                 __syncthreads();
-                const uint32_t runs = small_sort(t, L, n, a.keys, a.vals, sm.s64, sm.sm32, sm.sk, sm.sv, sm.rs);
-                if (runs > kLocalRuns) {
-                    // many buckets: the grid resolves them
-                    if (threadIdx.x < n) {
-                        a.keys[threadIdx.x] = sm.sk[threadIdx.x];
-                        a.vals[threadIdx.x] = sm.sv[threadIdx.x];
-                    }
-                    for (uint32_t r = threadIdx.x; r <= runs; r += kPT)
-                        a.keys2[r] = sm.rs[r];
-                    if (threadIdx.x == 0) {
-                        ctl->phase = kPhGridFoa;
-                        ctl->level = L;
-                        ctl->n_small_runs = runs;
-                    }
-                    __syncthreads();
-                    return;
-                }
+                const unsigned long long x = threadIdx.x < n ? (uint64_t(a.keys[threadIdx.x]) << 32) | a.vals[threadIdx.x]
+                                                             : ~0ull;
+                const uint32_t runs = small_sort(t, L, n, x, sm.s64, sm.sm32, sm.sk, sm.sv, sm.rs);
                 foa_runs<PW>(t, L, a.lv[L], sm.sk, sm.sv, sm.rs, runs, warp, kPWarps, sm.page + warp * kPage,
                              sm.q + warp * kFoaQuery, sm.cache[warp], ctr, &ts.failed);
                 // the CTA barrier makes this level's results (lv.res, appended
@@ -1295,21 +1290,8 @@ __global__ void __launch_bounds__(kPT, 1)
                 ctl->deepest = L;
             phase = kPhBottomUp;
         }
-        if (phase == kPhGridFoa) {
-            // a small level's sorted candidates in many buckets
-            foa_runs<PW>(t, L, a.lv[L], a.keys, a.vals, a.keys2, __ldcg(&ctl->n_small_runs), warp * G + cta,
-                         G * kPWarps, sm.page + warp * kPage, sm.q + warp * kFoaQuery, sm.cache[warp], ctr);
-            if (!grid_sync(ctl, t.error, nbar))
-                return;
-            if (L == 0) {
-                ls = kLsFinish;
-                continue;
-            }
-            L--;
-            phase = kPhBottomUp;
-        }
-        // bottom-up, big levels: six phases each; small ones go back to CTA 0
-        while (__ldcg(&ctl->count[L]) > kSmall && __ldcg(t.error) == 0) {
+        // bottom-up, big levels; small ones go back to CTA 0
+        while (__ldcg(&ctl->count[L]) > kSmallUp && __ldcg(t.error) == 0) {
             const uint32_t n = __ldcg(&ctl->count[L]);
             const uint32_t nb = sort_chunks(n, G);
             const uint32_t chunk = chunk_len(n, nb, kChunkAlign);
@@ -1318,32 +1300,63 @@ __global__ void __launch_bounds__(kPT, 1)
                 key_bits++;
             const uint32_t dbits = (key_bits + 1) / 2, nd = 1u << dbits;
             const uint32_t empty = t.g.buckets(L);
-            // 1. candidates and their pass-1 digit counts
+            const bool digits = n > kPT; // a queue may overflow
+            // 1. candidates, to their owners, and their pass-1 digit counts
             if (cta < nb) {
-                for (uint32_t d = threadIdx.x; d < nd; d += kPT) {
-                    cnt[d] = 0;
-                    a.hist2[cta * nd + d] = 0;
+                if (digits) {
+                    for (uint32_t d = threadIdx.x; d < nd; d += kPT) {
+                        cnt[d] = 0;
+                        a.hist2[cta * nd + d] = 0;
+                    }
+                    __syncthreads();
                 }
-                __syncthreads();
                 const uint32_t i0 = cta * chunk, i1 = min(n, i0 + chunk);
                 candidates_range(t, a.lv, L, deepest, i0, i1, a.keys, a.vals);
                 uint32_t mine = 0;
                 for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPT) {
                     const uint32_t key = a.keys[i];
                     if (key < empty) {
-                        atomicAdd(&cnt[key & (nd - 1)], 1u);
+                        if (digits)
+                            atomicAdd(&cnt[key & (nd - 1)], 1u);
                         mine++;
+                        const uint32_t owner = key % G, at = atomicAdd(a.queued + L * G + owner, 1u);
+                        if (at < kPT)
+                            __stcg(a.queue + owner * kPT + at, uint64_t(key) << 32 | i);
                     }
                 }
-                mine = __reduce_add_sync(0xffffffffu, mine);
-                if ((threadIdx.x & 31) == 0 && mine)
-                    atomicAdd(&ctl->ncand[L], mine);
-                __syncthreads();
-                for (uint32_t d = threadIdx.x; d < nd; d += kPT)
-                    a.hist[cta * nd + d] = cnt[d];
+                if (digits) {
+                    mine = __reduce_add_sync(0xffffffffu, mine);
+                    if ((threadIdx.x & 31) == 0 && mine)
+                        atomicAdd(&ctl->ncand[L], mine);
+                    __syncthreads();
+                    for (uint32_t d = threadIdx.x; d < nd; d += kPT)
+                        a.hist[cta * nd + d] = cnt[d];
+                }
             }
             if (!grid_sync(ctl, t.error, nbar))
                 return;
+            // 2. the CTA's own candidates, unless a queue overflowed.  Each grid
+            // step costs 2.4-3.5 us whatever it does: with every level sorted
+            // by the grid (four steps and more) a level of 4,816 entries took
+            // 33 us, now about 20, and one of 1,216 28 and 18: batches of 64
+            // edits, as above, 6.22 -> 5.80 and 15.0 -> 13.6 ms.
+            {
+                const uint32_t* queued = a.queued + L * G;
+                bool over = false;
+                for (uint32_t k = threadIdx.x; k < G; k += kPT)
+                    over |= __ldcg(queued + k) > kPT;
+                if (!__syncthreads_or(over)) {
+                    const uint32_t own = __ldcg(queued + cta);
+                    const unsigned long long x = threadIdx.x < own ? __ldcg(a.queue + cta * kPT + threadIdx.x) : ~0ull;
+                    const uint32_t runs = small_sort(t, L, own, x, sm.s64, sm32, sm.sk, sm.sv, sm.rs);
+                    foa_runs<PW>(t, L, a.lv[L], sm.sk, sm.sv, sm.rs, runs, warp, kPWarps, sm.page + warp * kPage,
+                                 sm.q + warp * kFoaQuery, sm.cache[warp], ctr);
+                    if (!grid_sync(ctl, t.error, nbar))
+                        return;
+                    L--; // (level 0 holds one entry: never big)
+                    continue;
+                }
+            }
             // the second pass and the find-or-add: candidates only
             const uint32_t ncand = __ldcg(&ctl->ncand[L]);
             const uint32_t nb2 = sort_chunks(ncand, G);
@@ -1453,6 +1466,8 @@ PArgs persist_args(hd_ctx* c, const PersistLevels& pl, uint32_t grid, uint32_t n
     a.keys2 = pl.keys2;
     a.vals2 = pl.vals2;
     a.bsum = s.get<uint32_t>("ep_bsum", 3ull * grid);
+    a.queue = s.get<unsigned long long>("ep_queue", uint64_t(kPT) * grid);
+    a.queued = s.get<uint32_t>("ep_queued", uint64_t(HD_MAX_DEPTH) * grid);
     a.hist = s.get<uint32_t>("ep_hist", uint64_t(kDigits) * grid);
     a.hist2 = s.get<uint32_t>("ep_hist2", uint64_t(kDigits) * grid);
     a.rows = s.get<uint32_t>("ep_rows", kDigits);
