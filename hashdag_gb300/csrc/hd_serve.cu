@@ -236,12 +236,16 @@ void serve(hd_ctx* c, const hd_request* reqs, uint32_t n, const hd_serve_config&
             return true;
         };
         // admission: free pages above the threshold, or a GC first (again
-        // only once something was claimed since the last one)
+        // only once 1/128 of the pool was claimed since the last one: a GC that
+        // keeps its pages maps more with each run, as rebuilt parents move
+        // between buckets, so a loop that collects after every edit or two, as
+        // fast ones would, fills a small pool with its own collections)
         auto admit = [&] {
             if (cfg.gc_free_fraction <= 0)
                 return;
             const uint64_t f = free_pages(c);
-            if (double(f) < cfg.gc_free_fraction * double(c->cfg.pool_pages) && f < free_after_gc)
+            if (double(f) < cfg.gc_free_fraction * double(c->cfg.pool_pages) &&
+                f + c->cfg.pool_pages / 128 < free_after_gc)
                 run_gc();
         };
         auto fence_renders = [&] {
