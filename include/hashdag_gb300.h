@@ -249,7 +249,9 @@ hd_status hd_get_values(hd_ctx* ctx, const uint32_t* d_xyz, uint64_t n, uint8_t*
 /* One edit: the editor's top-down descent with the reference's early exits
  * (should_edit / is_empty / is_full, hash_dag_edits.h:356-444), the 64-voxel
  * leaf rebuild (:451-546), then bottom-up find_or_add of every changed node
- * (hash_table.h:470-560), level by level, in depth-first order. */
+ * (hash_table.h:470-560), level by level, in depth-first order.  The geometry
+ * runs in one persistent launch whose grid barriers are bounded waits: one
+ * that runs out gives HD_ERR_TIMEOUT. */
 hd_status hd_edit_apply(hd_ctx* ctx, const hd_edit* edit, hd_edit_stats* stats);
 /* Batched form of HashDAG::edit_threads over a list of edits: the same
  * result as calling hd_edit_apply for each in order (same table, same
