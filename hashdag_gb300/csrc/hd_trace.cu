@@ -872,7 +872,9 @@ __global__ void __launch_bounds__(128, 12)
 // list, tile by tile, with their ray origins, so that
 // the traversal kernel runs full warps of rays from neighbouring pixels and
 // carries none of the double-precision set-up; misses get mask 2 here.  Rows
-// are output rows (the layout of the paths image).
+// are output rows (the layout of the paths image).  1080p at 2^13: 63 us, 42 of
+// them the origins (a warp's double operation takes 16 cycles); blocks of 128 to
+// 512 threads and persistent warps that read ahead took 60 to 73.
 template <int FMA>
 __global__ void __launch_bounds__(64) k_shadow_list(__grid_constant__ const hd_camera cam, uint32_t W, uint32_t H,
                                                     const uint4* __restrict__ paths, F3 light, float bias,
