@@ -42,28 +42,50 @@ __global__ void k_gc_mark(Table t, const uint32_t* __restrict__ live, uint32_t n
     }
 }
 
-// A bitmap word that counts as its bits (exclusive_scan's input).
-struct BitsOf {
-    uint32_t word;
-    HD_HD operator uint32_t() const { return popc32(word); }
-};
-
-// The live list of a level, and its ranks: every word that has a bit with the
-// live count before it, for ChildMap.
-__global__ void k_bitmap_to_list(const uint32_t* __restrict__ bitmap, const uint32_t* __restrict__ pos, uint64_t n,
-                                 uint32_t base, uint32_t* __restrict__ list, uint2* __restrict__ ranks)
+// A level's live list from its mark bitmap, in two passes over it (16 MB for a
+// level of 2^16 buckets of 2,048 words, mostly empty): the bits of each tile of
+// kScanTile words, then, with the tiles' sums, the list and the ranks: every
+// word that has a bit with the live count before it, for ChildMap.  With the
+// counts scanned into an array of their own and added up in place, five passes:
+// 470 us a GC of a 2^14 scene, so 183.
+__global__ void __launch_bounds__(kScanThreads) k_gc_tile_bits(const uint32_t* __restrict__ bitmap, uint64_t n,
+                                                               uint32_t* __restrict__ sums)
 {
-    HD_GRID_STRIDE(i, n)
-    {
-        uint32_t b = bitmap[i];
+    const uint64_t base = uint64_t(blockIdx.x) * kScanTile;
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        const uint64_t k = base + uint64_t(i) * kScanThreads + threadIdx.x;
+        bits += k < n ? popc32(bitmap[k]) : 0u;
+    }
+    uint32_t total;
+    block_excl_scan(bits, &total);
+    if (threadIdx.x == 0)
+        sums[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(kScanThreads)
+    k_gc_list(const uint32_t* __restrict__ bitmap, const uint32_t* __restrict__ before, uint64_t n, uint32_t base,
+              uint32_t* __restrict__ list, uint2* __restrict__ ranks)
+{
+    const uint64_t at = uint64_t(blockIdx.x) * kScanTile + uint64_t(threadIdx.x) * kScanItems;
+    uint32_t w[kScanItems], bits = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        w[i] = at + i < n ? bitmap[at + i] : 0u;
+        bits += popc32(w[i]);
+    }
+    uint32_t total;
+    uint32_t o = before[blockIdx.x] + block_excl_scan(bits, &total);
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        uint32_t b = w[i];
         if (!b)
             continue;
-        uint32_t o = pos[i];
-        ranks[i] = make_uint2(b, o);
+        ranks[at + i] = make_uint2(b, o);
         while (b) {
             const uint32_t bit = __ffs(b) - 1;
             b &= b - 1;
-            list[o++] = base + uint32_t(i) * 32 + bit;
+            list[o++] = base + uint32_t(at + i) * 32 + bit;
         }
     }
 }
@@ -430,7 +452,9 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
     for (uint32_t L = 1; L <= leafl; L++)
         most_words = std::max<uint64_t>(most_words, (uint64_t(g.buckets(L)) * g.capacity(L) + 31) / 32);
     uint32_t* bitmap = s.get<uint32_t>("gc_bitmap", most_words);
-    uint32_t* pos = s.get<uint32_t>("gc_pos", most_words);
+    const uint64_t most_tiles = (most_words + kScanTile - 1) / kScanTile;
+    uint32_t* tile_bits = s.get<uint32_t>("gc_tile_bits", most_tiles);
+    uint32_t* tile_before = s.get<uint32_t>("gc_tile_before", most_tiles);
     std::vector<uint32_t> bbase(leafl + 1, 0);
     for (uint32_t L = 0; L < leafl; L++) {
         const uint32_t base = g.make_ptr(L + 1, 0, 0);
@@ -443,12 +467,14 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
         snprintf(nm, sizeof(nm), "gc_ranks_%u", L + 1);
         ranks[L + 1] = s.get<uint2>(nm, nwords);
         bbase[L + 1] = base;
-        exclusive_scan<BitsOf, uint32_t>(s, reinterpret_cast<const BitsOf*>(bitmap), pos, nwords, d_n, st);
+        const uint32_t tiles = uint32_t((nwords + kScanTile - 1) / kScanTile);
+        k_gc_tile_bits<<<tiles, kScanThreads, 0, st>>>(bitmap, nwords, tile_bits);
+        HD_LAUNCH_CHECK();
+        exclusive_scan<uint32_t, uint32_t>(s, tile_bits, tile_before, tiles, d_n, st);
         nlive[L + 1] = read_scalar(d_n, st);
         snprintf(nm, sizeof(nm), "gc_live_%u", L + 1);
         live[L + 1] = s.get<uint32_t>(nm, uint64_t(nlive[L + 1]) + 1);
-        k_bitmap_to_list<<<grid_for(nwords, 256), 256, 0, st>>>(bitmap, pos, nwords, base, live[L + 1],
-                                                                  ranks[L + 1]);
+        k_gc_list<<<tiles, kScanThreads, 0, st>>>(bitmap, tile_before, nwords, base, live[L + 1], ranks[L + 1]);
         HD_LAUNCH_CHECK();
     }
     uint32_t maxn = 1, max_buckets = 1;
