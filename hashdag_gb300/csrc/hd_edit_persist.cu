@@ -35,13 +35,13 @@
 #include <cstring>
 #include <vector>
 
+#include "hd_chunks.cuh"
 #include "hd_edit.cuh"
 
 namespace hd {
 
 namespace {
 
-constexpr uint32_t kPT = 1024;             // threads per CTA (one CTA per SM)
 constexpr uint32_t kPWarps = kPT / 32;
 // Entries of a level that CTA 0 handles alone, top-down and bottom-up: a grid
 // step costs a barrier (2.4-3.5 us), CTA 0 alone 4 us a level of 200 entries and
@@ -207,21 +207,6 @@ HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
     __syncthreads();
     return ok != 0;
 }
-
-HD_D uint32_t chunk_len(uint32_t n, uint32_t parts, uint32_t align)
-{
-    const uint32_t per = (n + parts - 1) / parts;
-    return (per + align - 1) / align * align;
-}
-
-// Grid phases split a level into one chunk per CTA, a multiple of the warp
-// width long (so that a warp's 32 consecutive slots fall in at most two
-// chunks): every CTA gets work once a level holds 32 entries per CTA.
-constexpr uint32_t kChunkAlign = 32;
-
-// Chunk of level entries a descend flag is counted in (the grid's top-down
-// chunking of that level).
-HD_D uint32_t td_chunk(uint32_t i, uint32_t n, uint32_t G) { return i / chunk_len(n, G, kChunkAlign); }
 
 // Block-wide exclusive scan (kPT threads) of v; *total = the block's sum.
 HD_D uint32_t cta_scan(uint32_t v, uint32_t* total, uint32_t* sm32)
@@ -758,17 +743,6 @@ HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, unsigned long l
         rs[runs] = ncand;
     __syncthreads();
     return runs;
-}
-
-// Chunks of a sorted level (their digit counts' rows) that the scatters sum
-// themselves, the least length of a chunk, and the chunks of n elements: one
-// a CTA, at most kSumRows of at most kPT elements for as long as they do.
-constexpr uint32_t kSumRows = 32;
-constexpr uint32_t kSortChunk = 256;
-HD_D uint32_t sort_chunks(uint32_t n, uint32_t G)
-{
-    const uint32_t few = (n + kSortChunk - 1) / kSortChunk;
-    return max(1u, few <= kSumRows ? few : n <= kSumRows * kPT ? kSumRows : min(G, (n + kChunkAlign - 1) / kChunkAlign));
 }
 
 // Per digit of the nb chunks' counts (rows of nd): exclusive scan over the
