@@ -748,14 +748,13 @@ HD_D uint32_t small_sort(const Table& t, uint32_t L, uint32_t n, unsigned long l
 // Per digit of the nb chunks' counts (rows of nd): exclusive scan over the
 // chunks in place, the total into rows.  A thread a digit and part of the
 // chunks would wait for each other; a warp reads 32 digits of a chunk at once
-// and 8 chunks ahead.
+// and 8 chunks ahead (fewer digits, of a level of few buckets: fewer lanes).
 HD_D void scan_rows(uint32_t* hist, uint32_t nb, uint32_t nd, uint32_t* rows)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    if (gw >= nd / 32)
+    const uint32_t d = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+    if (d >= nd)
         return;
-    uint32_t* p = hist + gw * 32 + lane;
+    uint32_t* p = hist + d;
     uint32_t run = 0;
     for (uint32_t c0 = 0; c0 < nb; c0 += 8) {
         uint32_t x[8];
@@ -769,7 +768,7 @@ HD_D void scan_rows(uint32_t* hist, uint32_t nb, uint32_t nd, uint32_t* rows)
             run += x[k];
         }
     }
-    rows[gw * 32 + lane] = run;
+    rows[d] = run;
 }
 
 // Stable scatter of chunk `cb` of (keys, vals) by digit (key >> shift) & (nd
