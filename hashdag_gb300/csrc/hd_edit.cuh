@@ -1035,8 +1035,13 @@ struct EditGeometry {
     uint32_t root, deepest;
     std::vector<uint32_t> count; // entries per level (0 below the deepest)
 };
+// The batched forms sort by bucket in two passes of at most 2^9 digits: tables
+// of at most 2^17 buckets a level (an entry without a bucket sorts behind
+// them).  Edits of others are made level by level.
+constexpr uint32_t kMaxSortBits = 17;
+inline bool two_pass_sort(const Geom& g) { return g.top_bits <= kMaxSortBits && g.low_bits <= kMaxSortBits; }
 // Buffers for one edit, or null when its levels may hold more entries than
-// the persistent launch is used for.
+// the persistent launch is used for, or have too many buckets.
 const PersistLevels* one_edit_levels(hd_ctx* c, const Editor& ed);
 // Runs one edit's geometry in one persistent launch; false when it does not
 // apply (a level outgrew its bound, or the kernel does not fit on an SM): the

@@ -171,6 +171,7 @@ __global__ void k_b_candidates(Table t, const BatchState* bs, uint32_t level, Le
 
 constexpr uint32_t kSortBlock = 256;
 constexpr uint32_t kMaxDigits = 512;
+static_assert(1u << (kMaxSortBits + 2) / 2 <= kMaxDigits, "two passes sort every key");
 
 // The sort uses as many blocks as its input needs (at least kSortBlock keys
 // each, at most the grid): a chunk of the input per block.
@@ -552,6 +553,8 @@ constexpr uint64_t kOneEditEntries = 1ull << 22;
 
 const PersistLevels* one_edit_levels(hd_ctx* c, const Editor& ed)
 {
+    if (!two_pass_sort(c->g))
+        return nullptr;
     std::vector<uint64_t> cap(c->g.leaf_level + 1, 0);
     edit_caps(c->g, ed, cap);
     for (uint64_t n : cap)
@@ -675,11 +678,12 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
     const auto t0 = std::chrono::steady_clock::now();
     cudaStream_t st = c->stream;
     hd_edit_stats sum{};
-    bool plain = c->colors;
+    bool plain = c->colors || !two_pass_sort(c->g);
     for (uint32_t i = 0; i < n && !plain; i++)
         plain = edits[i].tool > HD_TOOL_BOX_ADD;
     if (plain) {
-        // colours, paint and copy take the one-edit path, edit by edit
+        // colours, paint, copy and tables of too many buckets for the sort
+        // take the one-edit path, edit by edit
         float at = 0;
         for (uint32_t i = 0; i < n; i++) {
             hd_edit_stats s{};

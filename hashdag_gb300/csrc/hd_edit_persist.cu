@@ -52,6 +52,7 @@ constexpr uint32_t kPWarps = kPT / 32;
 // 13.2 ms.
 constexpr uint32_t kSmall = 512, kSmallUp = 256;
 constexpr uint32_t kDigits = 512;          // radix digits per pass at most (9 bits)
+static_assert(1u << (kMaxSortBits + 2) / 2 <= kDigits, "two passes sort every key");
 // Candidates of a big level from which repeats are looked for (a grid step).
 constexpr uint32_t kRepeatLevel = 4096;
 constexpr unsigned long long kWaitNs = 2000000000ull;

@@ -44,3 +44,11 @@ def check(kw, batched, mode=1):
 def test_few_buckets(gpu, batched):
     """2^6 buckets: two sort passes of 16 digits, fewer than a warp's lanes."""
     check({"top_bucket_bits": 6, "top_bucket_size": 1 << 16, "pool_pages": 200000}, batched)
+
+
+@pytest.mark.parametrize("batched, mode", [(False, 1), (True, 1), (True, 0)])
+def test_many_buckets(gpu, batched, mode):
+    """2^18 and 2^19 buckets, more than two passes of 2^9 digits sort: such
+    edits are made level by level."""
+    check({"top_levels": 7, "top_bucket_bits": 18, "top_bucket_size": 512, "low_bucket_bits": 19,
+           "low_bucket_size": 512, "pool_pages": 400000}, batched, mode)
