@@ -685,9 +685,11 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
         // colours, paint, copy and tables of too many buckets for the sort
         // take the one-edit path, edit by edit
         float at = 0;
+        c->batch_applied = 0;
         for (uint32_t i = 0; i < n; i++) {
             hd_edit_stats s{};
             edit_one(c, edits[i], &s);
+            c->batch_applied = i + 1;
             at += s.device_ms;
             s.host_ms = at;
             if (per_edit)
