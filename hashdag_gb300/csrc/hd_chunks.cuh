@@ -1,5 +1,6 @@
 // How the persistent edit kernel (hd_edit_persist.cu) splits a level over its
-// CTAs: plain arithmetic, also compiled by a host compiler (its test).
+// CTAs, and its grid barrier's word: plain arithmetic, also compiled by a host
+// compiler (its test).
 #pragma once
 
 #include <cstdint>
@@ -45,5 +46,13 @@ HD_SPLIT uint32_t sort_chunks(uint32_t n, uint32_t G)
                                                 : (n + kChunkAlign - 1) / kChunkAlign;
     return want < 1 ? 1 : want < G ? want : G;
 }
+
+// The grid barrier's word: the arrivals of a launch, which only grow, and on top
+// the flag of a CTA that gave up (63 bits of arrivals never reach it).
+constexpr unsigned long long kBarrierAbort = 1ull << 63;
+HD_SPLIT unsigned long long barrier_arrivals(unsigned long long word) { return word & ~kBarrierAbort; }
+HD_SPLIT bool barrier_aborted(unsigned long long word) { return (word & kBarrierAbort) != 0; }
+// The arrivals at which the k-th barrier of G CTAs is passed
+HD_SPLIT unsigned long long barrier_target(uint32_t k, uint32_t G) { return (unsigned long long)k * G; }
 
 } // namespace hd

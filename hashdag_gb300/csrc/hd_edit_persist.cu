@@ -72,15 +72,13 @@ struct Cmd {
 // read: it writes the slot of the next barrier, which no CTA reads until
 // every CTA has left this one.
 struct Ctl {
-    // grid barrier arrivals of the launch, and the flag of a CTA that gave up
-    // (read together, as one word)
-    uint32_t arrived, abort;
+    unsigned long long arrived; // the grid barrier's word (hd_chunks.cuh)
     uint32_t stop;
     uint32_t idx;       // edit being applied
     uint32_t phase;     // the grid step CTA 0 asks for (kPh*)
     uint32_t level;     // its level
     uint32_t deepest;   // deepest level of the current edit
-    uint32_t pad;
+    uint32_t pad;       // (the commands on 8-byte boundaries)
     Cmd cmd[2];
     uint32_t ncand[HD_MAX_DEPTH]; // big levels: candidates for find-or-add
     uint32_t nruns[HD_MAX_DEPTH]; // big levels: long runs of repeats
@@ -139,7 +137,7 @@ HD_D uint32_t ld_acquire(const uint32_t* p)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-HD_D unsigned long long ld_acquire64(const void* p)
+HD_D unsigned long long ld_acquire64(const unsigned long long* p)
 {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -150,11 +148,13 @@ HD_D unsigned long long ld_acquire64(const void* p)
 // wait ran out or another CTA gave up (the caller returns).  The arrival
 // count only grows (the control block starts at zero every launch), so the
 // k-th barrier is passed once k x CTAs have arrived: no reset, and no
-// generation word for the last CTA to publish after its arrival.  Bound by
-// L2 round trips: a poll is one acquire of the arrivals and the abort flag
-// together, without a pause until it has waited long (with two reads and a
-// pause a poll, and a fence after, a grid step of almost no work took 2.7-4.3
-// us, now 2.4-3.5).
+// generation word for the last CTA to publish after its arrival.  Arrivals and
+// the flag of a CTA that gave up are one 64-bit word, which every access to it
+// takes whole: an acquire of a word orders nothing behind an atomic of half of
+// it.  Bound by
+// L2 round trips: a poll is one acquire, without a pause until it has waited
+// long (with two reads and a pause a poll, and a fence after, a grid step of
+// almost no work took 2.7-4.3 us, now 2.4-3.5).
 HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
 {
     __shared__ uint32_t ok;
@@ -164,18 +164,18 @@ HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
         nbar++;
         if (blockIdx.x == 0)
             __stcg(&ctl->bars0, nbar);
-        const uint32_t target = nbar * gridDim.x;
+        const unsigned long long target = barrier_target(nbar, gridDim.x);
         __threadfence();
-        if (atomicAdd(&ctl->arrived, 1u) + 1u == target) {
+        if (barrier_arrivals(atomicAdd(&ctl->arrived, 1ull)) + 1 == target) {
             __threadfence(); // the last to arrive acquires here
         } else {
             unsigned long long t0 = 0;
             uint32_t spins = 0;
             for (;;) {
-                const unsigned long long both = ld_acquire64(&ctl->arrived);
-                if (int32_t(uint32_t(both) - target) >= 0)
+                const unsigned long long word = ld_acquire64(&ctl->arrived);
+                if (barrier_arrivals(word) >= target)
                     break;
-                if (uint32_t(both >> 32)) {
+                if (barrier_aborted(word)) {
                     ok = 0;
                     break;
                 }
@@ -185,11 +185,11 @@ HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
                     const unsigned long long set_ns = __ldcg(&ctl->wait_ns);
                     const unsigned long long limit = set_ns ? set_ns : kWaitNs;
                     if (now_ns() - t0 > limit) {
-                        if (atomicExch(&ctl->abort, 1u) == 0) {
+                        if (!barrier_aborted(atomicOr(&ctl->arrived, kBarrierAbort))) {
                             ctl->diag[0] = blockIdx.x;
                             ctl->diag[1] = nbar;
-                            ctl->diag[2] = ld_acquire(&ctl->arrived);
-                            ctl->diag[3] = target;
+                            ctl->diag[2] = uint32_t(barrier_arrivals(ld_acquire64(&ctl->arrived)));
+                            ctl->diag[3] = uint32_t(target);
                             ctl->diag[4] = ld_acquire(&ctl->bars0);
                             ctl->diag[5] = ld_acquire(&ctl->phase);
                             ctl->diag[6] = ld_acquire(&ctl->level);
@@ -997,7 +997,7 @@ HD_D void local_advance(const Table& t, const PArgs& a, uint32_t ls, uint32_t L,
             if (threadIdx.x == 0) {
                 const unsigned long long set_ns = __ldcg(&ctl->wait_ns);
                 ctl->phase = kPhNone;
-                meet = int32_t(ld_acquire(&ctl->arrived) - (nbar * G + G - 1)) < 0 ||
+                meet = barrier_arrivals(ld_acquire64(&ctl->arrived)) + 1 < barrier_target(nbar + 1, G) ||
                        now_ns() - t_in > (set_ns ? set_ns : kWaitNs) / 16;
             }
             __syncthreads();
@@ -1532,7 +1532,7 @@ void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const Pe
         elapsed_before += launch_ms;
         done += ok;
         c->batch_applied = done;
-        if (fin.abort)
+        if (barrier_aborted(fin.arrived))
             persist_timeout(c, fin, done);
         if (fin.stop == kDone)
             break;
@@ -1584,7 +1584,7 @@ bool edit_geometry_persistent(hd_ctx* c, const Editor& ed, const PersistLevels& 
     HD_CUDA(cudaMemcpyAsync(&back, a.ctl, sizeof(back), cudaMemcpyDeviceToHost, st));
     HD_CUDA(cudaStreamSynchronize(st));
     const Ctl& fin = back.ctl;
-    if (fin.abort)
+    if (barrier_aborted(fin.arrived))
         persist_timeout(c, fin, 0);
     if (fin.stop == kCapacity)
         return false;
