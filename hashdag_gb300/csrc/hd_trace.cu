@@ -575,6 +575,7 @@ template <int FMA, bool SAFE>
 HD_D uint32_t split_walks(Walker<FMA, SAFE>& w, const SharedStack& stack, bool& active)
 {
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    __syncwarp(); // the givers' stack entries and mask bytes are written (the votes below order no memory)
     const uint32_t idle = __ballot_sync(0xffffffffu, !active);
     const uint32_t givers = __ballot_sync(0xffffffffu, active && w.pending != 0);
     const uint32_t n = min(__popc(idle), __popc(givers));
