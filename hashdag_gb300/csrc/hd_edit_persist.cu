@@ -498,8 +498,12 @@ HD_D uint32_t tiny_candidates(const Table& t, const PArgs& a, TinyState& ts, uin
     const Level child = L < deepest ? held_level(a, ts, L + 1) : Level{};
     const uint32_t key = lane < n ? candidate_entry<true>(t, L, lv, child, lane) : kNoBucket;
     const uint32_t cb = __ballot_sync(0xffffffffu, key != kNoBucket);
-    if (!cb)
+    if (!cb) {
+        // entries resolved at once: the level above reads their results on
+        // other lanes
+        __syncwarp();
         return 0;
+    }
     const uint32_t peers = __match_any_sync(0xffffffffu, key) & cb;
     const bool lead = key != kNoBucket && (peers & lt) == 0;
     const uint32_t leads = __ballot_sync(0xffffffffu, lead);

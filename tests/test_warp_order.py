@@ -26,3 +26,11 @@ def test_split_walks_reads_a_givers_stack_behind_its_writes():
     # after the givers' writes (before the call), and before their next ones
     assert len(reads) == 2
     assert any(s < min(reads) for s in syncs) and any(s > max(reads) for s in syncs)
+
+
+def test_tiny_candidates_returns_behind_a_warp_barrier():
+    """Its entries' results are read by other lanes at the level above."""
+    b = body("hd_edit_persist.cu", "tiny_candidates")
+    for m in re.finditer(r"\breturn\b", b):
+        before = b[:m.start()].rstrip()
+        assert re.search(r"__syncwarp\(\);(\s*\{)?$", before), before[-120:]
