@@ -507,9 +507,10 @@ class HashDAG:
         self._check(lib().hd_set_fp_mode(self._h, int(mode)))
 
     def set_test_barrier_skip(self, cta_plus_one, wait_ms=50):
-        """Test hook (hd_set_test_barrier_skip): the next persistent batch
+        """Test hook (hd_set_test_barrier_skip): the next persistent edit
         launch leaves one CTA out of its grid barriers, so the others' waits
-        run out after wait_ms and the call fails with HD_ERR_TIMEOUT."""
+        run out after wait_ms (a batch fails with HD_ERR_TIMEOUT, a single edit
+        is made level by level), or, for a CTA past the grid, is refused."""
         self._check(lib().hd_set_test_barrier_skip(self._h, int(cta_plus_one), int(wait_ms)))
 
     def set_page_reserve(self, pages):

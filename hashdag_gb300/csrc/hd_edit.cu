@@ -162,7 +162,8 @@ static void fill_stats(hd_ctx* c, const EditCounters& h, std::chrono::steady_clo
 // an edit at 2^10), 16 carves of radius 16-48 at 2^10 went from 18.2 to 4.0 ms
 // and 8 mixed edits of radius 4-512 at 2^15 from 16-17 to 4.1 ms (2.1 and 1.9-2.2
 // with what the launch itself has gained since).  Edits whose
-// levels may hold over kOneEditEntries entries stay with that path.
+// levels may hold over kOneEditEntries entries stay with that path, and those
+// that the launch could not finish (edit_geometry_persistent) come back to it.
 void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
 {
     if (c->needs_gc)

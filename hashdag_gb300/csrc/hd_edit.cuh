@@ -1043,9 +1043,13 @@ inline bool two_pass_sort(const Geom& g) { return g.top_bits <= kMaxSortBits && 
 // Buffers for one edit, or null when its levels may hold more entries than
 // the persistent launch is used for, or have too many buckets.
 const PersistLevels* one_edit_levels(hd_ctx* c, const Editor& ed);
-// Runs one edit's geometry in one persistent launch; false when it does not
-// apply (a level outgrew its bound, or the kernel does not fit on an SM): the
-// table is then untouched.  hold_root: the root is left for the caller to set.
+// Runs one edit's geometry in one persistent launch; false when the edit is to
+// be made level by level: a level outgrew its bound, the device did not take
+// the launch, or a grid barrier ran out of time (another stream's kernels held
+// SMs for seconds).  The root and the history are then as before; after a
+// barrier that ran out the table may hold nodes of the edit already, some of
+// which the edit then appends again (no scan compares a bucket's last node).
+// hold_root: the root is left for the caller to set.
 bool edit_geometry_persistent(hd_ctx* c, const Editor& ed, const PersistLevels& pl, bool hold_root, EditGeometry& out);
 // One edit, level by level from the host (hd_edit.cu).
 void edit_by_levels(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats);

@@ -1460,10 +1460,39 @@ PArgs persist_args(hd_ctx* c, const PersistLevels& pl, uint32_t grid, uint32_t n
 }
 static_assert(sizeof(Ctl) % alignof(EditOut) == 0, "EditOut follows Ctl");
 
-void persist_launch(hd_ctx* c, const PersistShape& shape, PArgs& a)
+// The control block at its start; hd_set_test_barrier_skip's hook, for one
+// launch only (it switches itself off).  Returns the CTAs to ask for.
+uint32_t persist_begin(hd_ctx* c, const PersistShape& shape, const PArgs& a)
+{
+    cudaStream_t st = c->stream;
+    HD_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(Ctl), st));
+    const uint32_t skip = c->test_skip_cta;
+    if (!skip)
+        return shape.grid;
+    const unsigned long long wait = c->test_wait_ns;
+    c->test_skip_cta = 0;
+    c->test_wait_ns = 0;
+    if (skip > shape.grid)
+        return 64 * shape.grid; // more than any SM holds: the launch is refused
+    HD_CUDA(cudaMemcpyAsync(&a.ctl->skip_cta, &skip, 4, cudaMemcpyHostToDevice, st));
+    HD_CUDA(cudaMemcpyAsync(&a.ctl->wait_ns, &wait, 8, cudaMemcpyHostToDevice, st));
+    HD_CUDA(cudaStreamSynchronize(st));
+    return shape.grid;
+}
+
+// False when the device has no room for all CTAs at once (fewer SMs to use
+// than it says): nothing was launched.
+bool persist_launch(hd_ctx* c, const PersistShape& shape, uint32_t grid, PArgs& a)
 {
     void* args[] = {&c->t, &a};
-    HD_CUDA(cudaLaunchCooperativeKernel(shape.kern, dim3(shape.grid), dim3(kPT), args, persist_smem(), c->stream));
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel(shape.kern, dim3(grid), dim3(kPT), args, persist_smem(), c->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return false;
+    }
+    HD_CUDA(e);
+    return true;
 }
 
 [[noreturn]] void persist_timeout(hd_ctx* c, const Ctl& fin, uint32_t edit)
@@ -1502,19 +1531,10 @@ void edit_batch_persistent(hd_ctx* c, const hd_edit* edits, uint32_t n, const Pe
         a.edits = d_edits;
         a.n_edits = m;
         HD_CUDA(cudaMemcpyAsync(d_edits, edits + done, sizeof(hd_edit) * m, cudaMemcpyHostToDevice, st));
-        HD_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(Ctl), st));
-        if (c->test_skip_cta) {
-            // one launch only: the hook switches itself off
-            const uint32_t skip = c->test_skip_cta;
-            const unsigned long long wait = c->test_wait_ns;
-            HD_CUDA(cudaMemcpyAsync(&a.ctl->skip_cta, &skip, 4, cudaMemcpyHostToDevice, st));
-            HD_CUDA(cudaMemcpyAsync(&a.ctl->wait_ns, &wait, 8, cudaMemcpyHostToDevice, st));
-            HD_CUDA(cudaStreamSynchronize(st));
-            c->test_skip_cta = 0;
-            c->test_wait_ns = 0;
-        }
+        const uint32_t grid = persist_begin(c, shape, a);
         HD_CUDA(cudaEventRecord(c->ev0, st));
-        persist_launch(c, shape, a);
+        if (!persist_launch(c, shape, grid, a))
+            throw CudaError{cudaErrorCooperativeLaunchTooLarge, "the persistent edit kernel's launch"};
         HD_CUDA(cudaEventRecord(c->ev1, st));
         HD_CUDA(cudaMemcpyAsync(back.data(), a.ctl, sizeof(Ctl) + sizeof(EditOut) * m, cudaMemcpyDeviceToHost, st));
         HD_CUDA(cudaStreamSynchronize(st));
@@ -1577,8 +1597,8 @@ bool edit_geometry_persistent(hd_ctx* c, const Editor& ed, const PersistLevels& 
     a.n_edits = 1;
     a.hold_root = hold_root;
     a.one = ed;
-    HD_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(Ctl), st));
-    persist_launch(c, shape, a);
+    if (!persist_launch(c, shape, persist_begin(c, shape, a), a))
+        return false;
     if (!hold_root)
         HD_CUDA(cudaEventRecord(c->ev1, st)); // with colours the edit goes on
     struct {
@@ -1588,8 +1608,14 @@ bool edit_geometry_persistent(hd_ctx* c, const Editor& ed, const PersistLevels& 
     HD_CUDA(cudaMemcpyAsync(&back, a.ctl, sizeof(back), cudaMemcpyDeviceToHost, st));
     HD_CUDA(cudaStreamSynchronize(st));
     const Ctl& fin = back.ctl;
-    if (barrier_aborted(fin.arrived))
-        persist_timeout(c, fin, 0);
+    if (barrier_aborted(fin.arrived)) {
+        check_error(c);
+        // CTA 0 may have finished the edit, if its levels were small, and
+        // waited for the others only then; else what it appended stays, whole
+        // nodes within their buckets' sizes
+        if (fin.idx != 1)
+            return false;
+    }
     if (fin.stop == kCapacity)
         return false;
     if (fin.stop == kEmptyScene)

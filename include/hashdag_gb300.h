@@ -250,8 +250,10 @@ hd_status hd_get_values(hd_ctx* ctx, const uint32_t* d_xyz, uint64_t n, uint8_t*
  * (should_edit / is_empty / is_full, hash_dag_edits.h:356-444), the 64-voxel
  * leaf rebuild (:451-546), then bottom-up find_or_add of every changed node
  * (hash_table.h:470-560), level by level, in depth-first order.  The geometry
- * runs in one persistent launch whose grid barriers are bounded waits: one
- * that runs out gives HD_ERR_TIMEOUT. */
+ * runs in one persistent launch of a CTA per SM whose grid barriers are bounded
+ * waits; where the device does not take the launch, or a wait runs out (another
+ * stream's kernels hold SMs for seconds), the edit is made by a launch per level
+ * and step instead. */
 hd_status hd_edit_apply(hd_ctx* ctx, const hd_edit* edit, hd_edit_stats* stats);
 /* Batched form of HashDAG::edit_threads over a list of edits: the same
  * result as calling hd_edit_apply for each in order (same table, same
@@ -460,14 +462,16 @@ hd_status hd_gc_ex(hd_ctx* ctx, uint32_t* h_extra_roots, uint32_t n_extra, uint3
  * edit's). */
 hd_status hd_set_page_reserve(hd_ctx* ctx, uint32_t pages);
 
-/* A test of the persistent batch's failure path: in the next persistent
- * hd_edit_batch launch (only), CTA cta_plus_one - 1 returns at once without
- * ever reaching a grid barrier, and every barrier wait is bounded by wait_ms
- * (0: the default 2 s).  The other CTAs' waits run out, the launch ends and
- * the call returns HD_ERR_TIMEOUT; the edits finished before stay applied
+/* A test of the persistent edit kernel's failure paths: in its next launch
+ * (only), CTA cta_plus_one - 1 returns at once without ever reaching a grid
+ * barrier, and every barrier wait is bounded by wait_ms (0: the default 2 s).
+ * The other CTAs' waits run out and the launch ends.  hd_edit_batch then
+ * returns HD_ERR_TIMEOUT; the edits finished before stay applied
  * (hd_edit_batch_ex fills their per-edit results), the root is the last
- * finished edit's, and the context stays usable.  cta_plus_one 0 clears
- * it. */
+ * finished edit's, and the context stays usable.  hd_edit_apply makes its edit
+ * level by level.  A CTA past the grid: the launch asks for more CTAs than the
+ * device takes and is refused (hd_edit_batch: HD_ERR_CUDA).  cta_plus_one 0
+ * clears it. */
 hd_status hd_set_test_barrier_skip(hd_ctx* ctx, uint32_t cta_plus_one, uint32_t wait_ms);
 
 /* ---- files (serializer.h:11-121) ---------------------------------------- */

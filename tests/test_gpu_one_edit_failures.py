@@ -1,0 +1,66 @@
+"""Single edits whose persistent launch cannot finish: a CTA that never reaches a
+grid barrier (bounded waits, tests' hook), or a launch that the device refuses.
+The edit is then made level by level: the same voxels, colours and counters as
+without the failure, one undo frame, and the context goes on."""
+import numpy as np
+import pytest
+
+import hashdag_gb300 as hd
+from hashdag_gb300 import scene, workloads
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+DEPTH = 10
+SKIP, REFUSED = 5, 1 << 20
+
+
+def _context(colors):
+    d = hd.HashDAG(DEPTH)
+    d.generate_scene(workloads.SEED_SCENE, shell=colors)
+    if colors:
+        d.colors_from_scene(workloads.SEED_COLORS)
+    return d
+
+
+def _fingerprint(d):
+    t = d.export_table()
+    ot = po.Table(po.default_config(DEPTH, pool_pages=int(t["pool"].size // 512) + 8))
+    ot.import_(t)
+    return ot.fingerprint()
+
+
+@pytest.mark.parametrize("cta", [SKIP, REFUSED])
+@pytest.mark.parametrize("colors", [False, True])
+# by CTA 0 alone; with grid steps; a copy, which is not the same when made twice
+@pytest.mark.parametrize("kind", ["small", "large", "copy"])
+def test_edit_is_made_level_by_level(gpu, kind, colors, cta):
+    rng = np.random.default_rng(11)
+    near = scene.surface_points(workloads.SEED_SCENE, DEPTH, 300, rng)
+    near = near[np.argsort(np.abs(near - 512.0).sum(axis=1))]
+    c = tuple(float(v) for v in near[0])
+    edit = {"small": hd.SphereEditor(c, 5.0, adding=False),
+            "large": hd.SphereEditor(c, 150.0, adding=False),
+            "copy": hd.CopyEditor(c, 20.0, c, tuple(v + 16.0 for v in c))}[kind]
+    after = hd.SphereEditor(tuple(float(v) for v in near[40]), 30.0, adding=True)
+    want, got = _context(colors), _context(colors)
+    a = want.edit_threads(edit)
+    got.set_test_barrier_skip(cta, 20)
+    b = got.edit_threads(edit)
+    assert (a.num_voxels, a.num_nodes, a.find_or_add_calls) == (b.num_voxels, b.num_nodes, b.find_or_add_calls)
+    if cta == REFUSED:  # nothing had been appended
+        assert a.nodes_added == b.nodes_added and want.firstNodeIndex == got.firstNodeIndex
+    assert got.history() == (1, 0)
+    for d in (want, got):  # (the failure was for that one launch)
+        d.edit_batch([after])
+    pts = np.clip(np.concatenate([near, np.array(c) + rng.uniform(-160, 160, (30000, 3))]), 0, 1023).astype(np.uint32)
+    for _ in range(3):  # after both edits, with one undone, with both
+        v = want.get_values(pts)
+        assert np.array_equal(v, got.get_values(pts))
+        if colors:
+            assert np.array_equal(want.get_colors(pts[v != 0]), got.get_colors(pts[v != 0]))
+        assert _fingerprint(want) == _fingerprint(got)
+        if got.history()[0]:
+            for d in (want, got):
+                d.undo()
+    want.free()
+    got.free()
