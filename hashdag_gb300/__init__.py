@@ -513,6 +513,11 @@ class HashDAG:
         is made level by level), or, for a CTA past the grid, is refused."""
         self._check(lib().hd_set_test_barrier_skip(self._h, int(cta_plus_one), int(wait_ms)))
 
+    def set_test_scratch_limit(self, limit):
+        """Test hook (hd_set_test_scratch_limit): scratch allocations past
+        `limit` bytes in all fail; 0 lifts it."""
+        self._check(lib().hd_set_test_scratch_limit(self._h, int(limit)))
+
     def set_page_reserve(self, pages):
         """Keeps `pages` pool pages back from edits for the GC's rebuild
         (hd_set_page_reserve)."""

@@ -248,6 +248,14 @@ hd_status hd_set_test_barrier_skip(hd_ctx* c, uint32_t cta_plus_one, uint32_t wa
     return HD_OK;
 }
 
+hd_status hd_set_test_scratch_limit(hd_ctx* c, uint64_t bytes)
+{
+    if (!c)
+        return HD_ERR_INVALID;
+    c->scratch.set_limit(size_t(bytes));
+    return HD_OK;
+}
+
 hd_status hd_set_fp_mode(hd_ctx* c, uint32_t mode)
 {
     if (!c || mode > 1)

@@ -164,16 +164,14 @@ static void fill_stats(hd_ctx* c, const EditCounters& h, std::chrono::steady_clo
 // with what the launch itself has gained since).  Edits whose
 // levels may hold over kOneEditEntries entries stay with that path, and those
 // that the launch could not finish (edit_geometry_persistent) come back to it.
-void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
+static bool edit_in_one_launch(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
 {
-    if (c->needs_gc)
-        throw StatusError{HD_ERR_STATE, "the table was loaded without bucket sizes; run hd_gc before editing"};
     const auto t0 = std::chrono::steady_clock::now();
     cudaStream_t st = c->stream;
     Editor ed = make_editor(e);
     const PersistLevels* pl = one_edit_levels(c, ed);
     if (!pl)
-        return edit_by_levels(c, e, stats);
+        return false;
     HD_CUDA(cudaEventRecord(c->ev0, st));
     if (e.tool == HD_TOOL_COPY)
         copy_source(c, ed); // the source region as it is before the edit
@@ -183,7 +181,7 @@ void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
     frame.root = c->root;
     EditGeometry geo{};
     if (!edit_geometry_persistent(c, ed, *pl, c->colors, geo))
-        return edit_by_levels(c, e, stats);
+        return false;
     if (c->colors) {
         std::vector<Level> lv(pl->lv);
         ColorsBack back;
@@ -196,6 +194,26 @@ void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
     c->root = geo.root;
     push_undo(c, std::move(frame));
     fill_stats(c, geo.ctr, t0, stats);
+    return true;
+}
+
+void edit_one(hd_ctx* c, const hd_edit& e, hd_edit_stats* stats)
+{
+    if (c->needs_gc)
+        throw StatusError{HD_ERR_STATE, "the table was loaded without bucket sizes; run hd_gc before editing"};
+    try {
+        if (edit_in_one_launch(c, e, stats))
+            return;
+    } catch (const StatusError& x) {
+        // The launch's level arrays are sized by upper bounds and kept.  Where
+        // the device has no room for them, or for the colours' arrays beside
+        // them, they go, and the edit takes arrays of the entries there are.
+        if (x.status != HD_ERR_OOM)
+            throw;
+        HD_CUDA(cudaStreamSynchronize(c->stream));
+        drop_batch_levels(c);
+    }
+    edit_by_levels(c, e, stats);
 }
 
 // One edit level by level: the host sizes every level from the previous one

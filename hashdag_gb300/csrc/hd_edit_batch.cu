@@ -545,8 +545,17 @@ static const BatchBuffers& batch_levels(hd_ctx* c, std::vector<uint64_t>& cap, u
     return bg.buffers;
 }
 
+void drop_batch_levels(hd_ctx* c)
+{
+    if (c->batch)
+        c->batch->have = false;
+    c->scratch.drop_all("eb_");
+    c->scratch.drop_all("ep_");
+}
+
 // The persistent launch takes an edit whose levels hold at most this many
-// entries each (about 350 MB of level arrays); beyond, the level-by-level
+// entries each (89 B an entry, 109 with colours, and a quarter in reserve: some
+// 0.5 GB for the leaf level, 0.6 to 0.8 in all); beyond, the level-by-level
 // path's arrays, sized by the entries there are, and its kernels over all of
 // them serve as well.
 constexpr uint64_t kOneEditEntries = 1ull << 22;

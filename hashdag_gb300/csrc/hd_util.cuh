@@ -47,7 +47,7 @@ public:
             b.bytes = 0;
             epoch_++;
             size_t want = bytes + bytes / 4 + 256;
-            if (cudaMalloc(&b.ptr, want) != cudaSuccess) {
+            if ((limit_ && total() + want > limit_) || cudaMalloc(&b.ptr, want) != cudaSuccess) {
                 cudaGetLastError();
                 throw StatusError{HD_ERR_OOM, std::string("scratch allocation failed: ") + name + " (" +
                                                   std::to_string(want >> 20) + " MiB)"};
@@ -73,6 +73,22 @@ public:
         bufs_.erase(it);
         epoch_++;
     }
+    // frees every buffer whose name begins so
+    void drop_all(const std::string& prefix)
+    {
+        for (auto it = bufs_.begin(); it != bufs_.end();) {
+            if (it->first.compare(0, prefix.size(), prefix) != 0) {
+                ++it;
+                continue;
+            }
+            if (it->second.ptr)
+                cudaFree(it->second.ptr);
+            it = bufs_.erase(it);
+        }
+        epoch_++;
+    }
+    // tests: allocations past `bytes` in all fail (0: none do)
+    void set_limit(size_t bytes) { limit_ = bytes; }
     // changes whenever a buffer moves or goes: pointers kept from get() hold
     // while it stays
     uint64_t epoch() const { return epoch_; }
@@ -104,7 +120,7 @@ private:
         size_t bytes = 0;
     };
     std::unordered_map<std::string, Buf> bufs_;
-    size_t peak_ = 0;
+    size_t peak_ = 0, limit_ = 0;
     uint64_t epoch_ = 0;
 };
 

@@ -473,6 +473,10 @@ hd_status hd_set_page_reserve(hd_ctx* ctx, uint32_t pages);
  * device takes and is refused (hd_edit_batch: HD_ERR_CUDA).  cta_plus_one 0
  * clears it. */
 hd_status hd_set_test_barrier_skip(hd_ctx* ctx, uint32_t cta_plus_one, uint32_t wait_ms);
+/* Tests of a full device: scratch allocations that would bring the context's
+ * scratch buffers ([2] of hd_memory_stats) over `bytes` fail as cudaMalloc does
+ * (0: none do). */
+hd_status hd_set_test_scratch_limit(hd_ctx* ctx, uint64_t bytes);
 
 /* ---- files (serializer.h:11-121) ---------------------------------------- */
 

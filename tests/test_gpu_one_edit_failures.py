@@ -64,3 +64,46 @@ def test_edit_is_made_level_by_level(gpu, kind, colors, cta):
                 d.undo()
     want.free()
     got.free()
+
+
+@pytest.mark.parametrize("share", [0.99, 0.95, 0.62])
+@pytest.mark.parametrize("colors", [False, True])
+def test_edit_without_room_for_its_bounds(gpu, colors, share):
+    """The launch's arrays are bounds on an edit's entries.  An edit that does
+    not get them (or the colours' beside them) takes the entries' own: half the
+    memory, the same result."""
+    rng = np.random.default_rng(12)
+    near = scene.surface_points(workloads.SEED_SCENE, DEPTH, 300, rng)
+    near = near[np.argsort(np.abs(near - 512.0).sum(axis=1))]
+    c = tuple(float(v) for v in near[0])
+    edits = [hd.SpherePaintEditor(c, 150.0), hd.SphereEditor((512.0, 512.0, 512.0), 300.0, adding=False),
+             hd.SphereEditor(c, 20.0, adding=True)]
+    for edit in edits[:2]:
+        want, got = _context(colors), _context(colors)
+        a = want.edit_threads(edit)
+        before = got.memory_stats()["scratch"]
+        limit = before + int(share * (want.memory_stats()["scratch"] - before))
+        got.set_test_scratch_limit(limit)
+        b = got.edit_threads(edit)
+        assert got.memory_stats()["scratch"] <= limit
+        assert (a.num_voxels, a.num_nodes, a.find_or_add_calls) == (b.num_voxels, b.num_nodes, b.find_or_add_calls)
+        for d in (want, got):
+            d.edit_threads(edits[2])
+        assert got.history() == (2, 0)
+        got.set_test_scratch_limit(0)
+        pts = np.clip(np.concatenate([near, 512.0 + rng.uniform(-310, 310, (30000, 3))]), 0, 1023).astype(np.uint32)
+        v = want.get_values(pts)
+        assert np.array_equal(v, got.get_values(pts))
+        if colors:
+            assert np.array_equal(want.get_colors(pts[v != 0]), got.get_colors(pts[v != 0]))
+        assert _fingerprint(want) == _fingerprint(got)
+        # too little for that as well is an error, and leaves the context as it is
+        root = got.firstNodeIndex
+        got.set_test_scratch_limit(1)
+        if share < 0.9:
+            with pytest.raises(hd.HashDagError) as ei:
+                got.edit_threads(hd.SphereEditor((512.0, 512.0, 512.0), 460.0, adding=False))
+            assert ei.value.status == hd._capi.HD_ERR_OOM
+            assert got.firstNodeIndex == root and got.history() == (2, 0)
+        want.free()
+        got.free()
