@@ -135,6 +135,9 @@ void bloom_clear_level(hd_ctx* c, uint32_t level);
 void download_pages(hd_ctx* c, uint32_t* h_page_table, uint32_t* h_pool, uint64_t pages);
 void upload_pages(hd_ctx* c, const uint32_t* h_page_table, const uint32_t* h_pool, uint64_t pages);
 
+// hd_edit_batch.cu: frees the batched edits' buffers
+void drop_batch_levels(hd_ctx* c);
+
 // hd_io.cu: keeps a copy of the BasicDAG words (host or device pointer)
 void keep_basic(hd_ctx* c, const uint32_t* words, uint64_t n);
 

@@ -1043,8 +1043,6 @@ inline bool two_pass_sort(const Geom& g) { return g.top_bits <= kMaxSortBits && 
 // Buffers for one edit, or null when its levels may hold more entries than
 // the persistent launch is used for, or have too many buckets.
 const PersistLevels* one_edit_levels(hd_ctx* c, const Editor& ed);
-// Frees the batched forms' buffers.
-void drop_batch_levels(hd_ctx* c);
 // Runs one edit's geometry in one persistent launch; false when the edit is to
 // be made level by level: a level outgrew its bound, the device did not take
 // the launch, or a grid barrier ran out of time (another stream's kernels held

@@ -429,7 +429,9 @@ struct ReserveOpen {
 };
 } // namespace
 
-void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
+// stage: the inner levels' nodes may be staged.  HD_ERR_OOM comes before
+// anything changes.
+static void gc_run(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages, bool stage)
 {
     cudaStream_t st = c->stream;
     Scratch& s = c->scratch;
@@ -494,7 +496,7 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
     uint64_t inner = 0;
     for (uint32_t L = 0; L < leafl; L++)
         inner += nlive[L];
-    if (36 * inner <= kGcStageBytes) {
+    if (stage && 36 * inner <= kGcStageBytes) {
         uint32_t* at = s.get<uint32_t>("gc_staged", 9 * inner + 1);
         for (uint32_t L = 0; L < leafl; L++) {
             staged[L] = at;
@@ -565,6 +567,7 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
     }
     // rebuild bottom-up
     uint32_t* gathered = s.get<uint32_t>("gc_content", uint64_t(staged[0] ? nlive[leafl] : maxn) * 9);
+    uint32_t* d_roots = s.get<uint32_t>("gc_roots", roots.size());
     for (int32_t L = int32_t(leafl); L >= 0; L--) {
         const uint32_t n = nlive[L];
         const uint32_t* dry_sizes = dry_all + g.level_first_bucket(uint32_t(L));
@@ -601,7 +604,6 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
         k_gc_write<<<grid_for(n, 256), 256, 0, st>>>(c->t, uint32_t(L), content, newaddr[L], n);
         HD_LAUNCH_CHECK();
     }
-    uint32_t* d_roots = s.get<uint32_t>("gc_roots", roots.size());
     HD_CUDA(cudaMemcpyAsync(d_roots, roots.data(), roots.size() * 4, cudaMemcpyHostToDevice, st));
     k_gc_remap_roots<<<1, 1, 0, st>>>(live[0], nlive[0], newaddr[0], d_roots, uint32_t(roots.size()), c->d_root);
     HD_LAUNCH_CHECK();
@@ -612,6 +614,21 @@ void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
         throw StatusError{hd_status(e), "garbage collection failed on the device"};
     c->root = roots[0];
     c->edit_head_ready = false;
+}
+
+void gc(hd_ctx* c, std::vector<uint32_t>& roots, bool release_pages)
+{
+    try {
+        return gc_run(c, roots, release_pages, true);
+    } catch (const StatusError& e) {
+        if (e.status != HD_ERR_OOM)
+            throw;
+    }
+    // without what GCs and edits keep for speed
+    HD_CUDA(cudaStreamSynchronize(c->stream));
+    c->scratch.drop("gc_staged");
+    drop_batch_levels(c);
+    gc_run(c, roots, release_pages, false);
 }
 
 } // namespace hd
