@@ -131,6 +131,21 @@ void table_reset(hd_ctx* c)
 // time through a staging buffer.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kIoPages = 32768; // 64 MB
+constexpr uint32_t kIoPagesLeast = 64;
+
+// The staging buffer for `pages` pages, in as many pieces of n as a device with
+// little room left takes.
+static uint32_t* io_staging(hd_ctx* c, uint64_t pages, uint64_t& n)
+{
+    for (n = std::min<uint64_t>(pages, kIoPages);; n = std::max<uint64_t>(n / 4, kIoPagesLeast)) {
+        try {
+            return c->scratch.get<uint32_t>("io_staging", n * kPage);
+        } catch (const StatusError&) {
+            if (n <= kIoPagesLeast)
+                throw;
+        }
+    }
+}
 
 __global__ void k_direct_entries(Table t, uint64_t n)
 {
@@ -174,9 +189,10 @@ void download_pages(hd_ctx* c, uint32_t* h_page_table, uint32_t* h_pool, uint64_
     if (h_pool && pages && !c->t.direct)
         HD_CUDA(cudaMemcpyAsync(h_pool, c->t.pool, pages * kPage * 4, cudaMemcpyDeviceToHost, st));
     if (h_pool && pages && c->t.direct) {
-        uint32_t* staging = c->scratch.get<uint32_t>("io_staging", std::min<uint64_t>(pages, kIoPages) * kPage);
-        for (uint64_t a = 0; a < pages; a += kIoPages) {
-            const uint64_t n = std::min<uint64_t>(pages - a, kIoPages);
+        uint64_t piece;
+        uint32_t* staging = io_staging(c, pages, piece);
+        for (uint64_t a = 0; a < pages; a += piece) {
+            const uint64_t n = std::min<uint64_t>(pages - a, piece);
             HD_CUDA(cudaMemsetAsync(staging, 0, n * kPage * 4, st)); // the null page and pages on the free list
             k_move_pages<true><<<grid_for(nv, 256), 256, 0, st>>>(c->t, nv, uint32_t(a), uint32_t(a + n), staging);
             HD_LAUNCH_CHECK();
@@ -199,9 +215,10 @@ void upload_pages(hd_ctx* c, const uint32_t* h_page_table, const uint32_t* h_poo
     k_direct_entries<<<grid_for(nv, 256), 256, 0, st>>>(c->t, nv);
     HD_LAUNCH_CHECK();
     if (pages) {
-        uint32_t* staging = c->scratch.get<uint32_t>("io_staging", std::min<uint64_t>(pages, kIoPages) * kPage);
-        for (uint64_t a = 0; a < pages; a += kIoPages) {
-            const uint64_t n = std::min<uint64_t>(pages - a, kIoPages);
+        uint64_t piece;
+        uint32_t* staging = io_staging(c, pages, piece);
+        for (uint64_t a = 0; a < pages; a += piece) {
+            const uint64_t n = std::min<uint64_t>(pages - a, piece);
             HD_CUDA(cudaMemcpyAsync(staging, h_pool + a * kPage, n * kPage * 4, cudaMemcpyHostToDevice, st));
             k_move_pages<false><<<grid_for(nv, 256), 256, 0, st>>>(c->t, nv, uint32_t(a), uint32_t(a + n), staging);
             HD_LAUNCH_CHECK();
