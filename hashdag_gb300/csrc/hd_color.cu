@@ -671,7 +671,7 @@ void copy_source(hd_ctx* c, Editor& ed)
 // (tens to a few thousand entries), and a launch per level and per scan, with
 // waits in between, took longer than its work: 60 launches and 12 waits an
 // edit.  One block of kTreeThreads threads goes through all of it in three
-// launches (k_col_down, k_col_sizes, k_col_up), whatever the edit's size: with
+// launches (k_col_down, k_col_sizes, k_col_up), whatever the number of tasks: with
 // several entries per thread in flight a level of 50,000 entries takes it some
 // 25 us.  Twelve edits of radius 8 to 64 at 2^13 with their undos: 10.0 ms with
 // the launches per level, 5.6 so.
@@ -1073,9 +1073,14 @@ __global__ void __launch_bounds__(256) k_col_count(uint32_t n, uint32_t n_pieces
 // The pieces' sums: blocks and bits before each piece (bits modulo 2^32; a task
 // has fewer).  Then each task's macro and weight words and where they begin,
 // its rank among the tasks that need a new slot (with colours and without a
-// unique leaf of their own) and among those with colours.  One block.
+// unique leaf of their own) and among those with colours.  One block.  The sums
+// of more than kSumPieces pieces are made by a scan over the grid before it
+// (summed): boxes of 2^14, 2^15, 2^16, 2^19 and 31 million pieces filled at 2^13
+// take 0.376, 0.50, 0.65, 2.09 and 103 ms with all of it in one block, 0.390,
+// 0.50, 0.607, 1.45 and 63.5 with the scan (its launches cost some 15 us).
+constexpr uint32_t kSumPieces = 1u << 15;
 __global__ void __launch_bounds__(kTreeThreads)
-    k_col_sizes(uint32_t n, uint32_t n_pieces, Level lvT, const uint32_t* __restrict__ first,
+    k_col_sizes(uint32_t n, uint32_t n_pieces, bool summed, Level lvT, const uint32_t* __restrict__ first,
                 const uint64_t* __restrict__ len, const uint32_t* __restrict__ piece_blocks,
                 const uint32_t* __restrict__ piece_bits, uint32_t* blocks_before, uint32_t* bits_before, uint32_t* nm,
                 uint32_t* nw, uint32_t* mo, uint32_t* wo, uint32_t* need_new, uint32_t* rank, uint32_t* row,
@@ -1085,7 +1090,9 @@ __global__ void __launch_bounds__(kTreeThreads)
     __shared__ Pair sums[33];
     constexpr uint32_t kPieces = 8;
     Pair done{0, 0};
-    for (uint64_t p0 = 0; p0 < n_pieces; p0 += kTreeThreads * kPieces) {
+    if (summed)
+        done = {blocks_before[n_pieces], bits_before[n_pieces]};
+    for (uint64_t p0 = summed ? n_pieces : 0; p0 < n_pieces; p0 += kTreeThreads * kPieces) {
         Pair v[kPieces], mine{0, 0}, total;
 #pragma unroll
         for (uint32_t j = 0; j < kPieces; j++) {
@@ -1110,7 +1117,7 @@ __global__ void __launch_bounds__(kTreeThreads)
         done.a += total.a;
         done.b += total.b;
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && !summed) {
         blocks_before[n_pieces] = done.a;
         bits_before[n_pieces] = done.b;
     }
@@ -1375,7 +1382,12 @@ void edit_colors(hd_ctx* c, const Editor& ed, std::vector<Level>& lv, const std:
     const uint32_t piece_grid = grid_for(uint64_t(n_pieces) * 32, 256, 152 * 16);
     k_col_count<<<piece_grid, 256, 0, st>>>(nT, n_pieces, first, len, base, out, piece_blocks, piece_bits);
     HD_LAUNCH_CHECK();
-    k_col_sizes<<<1, kTreeThreads, 0, st>>>(nT, n_pieces, lv[T], first, len, piece_blocks, piece_bits, blocks_before,
+    const bool summed = n_pieces > kSumPieces;
+    if (summed) {
+        exclusive_scan<uint32_t, uint32_t>(s, piece_blocks, blocks_before, n_pieces, blocks_before + n_pieces, st);
+        exclusive_scan<uint32_t, uint32_t>(s, piece_bits, bits_before, n_pieces, bits_before + n_pieces, st);
+    }
+    k_col_sizes<<<1, kTreeThreads, 0, st>>>(nT, n_pieces, summed, lv[T], first, len, piece_blocks, piece_bits, blocks_before,
                                             bits_before, nm, nw, mo, wo, need_new, rank, row, head);
     HD_LAUNCH_CHECK();
     h = read_scalar(head, st);
