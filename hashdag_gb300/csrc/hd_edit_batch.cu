@@ -19,6 +19,7 @@
 // hd_autotune_batch on a copy of the table.
 #include <chrono>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "hd_edit.cuh"
@@ -453,31 +454,34 @@ struct BatchGraph {
     }
 };
 
-static Level batch_level(Scratch& s, uint32_t L, uint64_t n, bool leaf, bool colors)
+// The arrays of a level of n entries, carved from the buffer whose next byte is
+// `at` (a null buffer: their bytes alone are counted).
+static Level batch_level(uint8_t* base, uint64_t& at, uint64_t n, bool leaf, bool colors)
 {
-    char nm[48];
-    auto buf = [&](const char* what, size_t bytes) {
-        snprintf(nm, sizeof(nm), "eb_%s_%u", what, L);
-        return s.get(nm, bytes);
+    auto part = [&](auto*& p, uint64_t words) {
+        using T = std::remove_reference_t<decltype(*p)>;
+        p = base ? reinterpret_cast<T*>(base + at) : nullptr;
+        at += (words * sizeof(T) + 255) / 256 * 256;
     };
     Level l{};
-    l.x = static_cast<uint32_t*>(buf("x", n * 4));
-    l.y = static_cast<uint32_t*>(buf("y", n * 4));
-    l.z = static_cast<uint32_t*>(buf("z", n * 4));
-    l.old = static_cast<uint32_t*>(buf("old", n * 4));
-    l.state = static_cast<uint8_t*>(buf("state", n));
-    l.res = static_cast<uint32_t*>(buf("res", n * 4));
-    l.cnt = static_cast<uint32_t*>(buf("cnt", n * 4));
-    l.flag = static_cast<uint32_t*>(buf("flag", n * 4));
-    l.exp = static_cast<uint32_t*>(buf("exp", n * 4));
-    l.leaf = leaf ? static_cast<uint64_t*>(buf("leaf", n * 8)) : nullptr;
-    l.cand = static_cast<uint32_t*>(buf("cand", n * 4 * kRow));
+    part(l.x, n);
+    part(l.y, n);
+    part(l.z, n);
+    part(l.old, n);
+    part(l.state, n);
+    part(l.res, n);
+    part(l.cnt, n);
+    part(l.flag, n);
+    part(l.exp, n);
+    if (leaf)
+        part(l.leaf, n);
+    part(l.cand, n * kRow);
     if (colors) {
-        l.ocnt = static_cast<uint32_t*>(buf("ocnt", n * 4));
-        l.cn = static_cast<uint32_t*>(buf("cn", n * 4));
-        l.noff = static_cast<uint32_t*>(buf("noff", n * 4));
-        l.ooff = static_cast<uint32_t*>(buf("ooff", n * 4));
-        l.task = static_cast<uint32_t*>(buf("task", n * 4));
+        part(l.ocnt, n);
+        part(l.cn, n);
+        part(l.noff, n);
+        part(l.ooff, n);
+        part(l.task, n);
     }
     return l;
 }
@@ -496,9 +500,17 @@ static BatchBuffers batch_buffers(hd_ctx* c, const std::vector<uint64_t>& cap64,
         b.caps[L] = uint32_t(v);
         maxn = std::max(maxn, v);
     }
+    // All levels in one buffer: with one an array, a first edit of a size that
+    // outgrows them freed and allocated some 150.
     b.lv.resize(levels);
-    for (uint32_t L = 0; L < levels; L++)
-        b.lv[L] = batch_level(s, L, b.caps[L], L == g.leaf_level, c->colors);
+    uint8_t* base = nullptr;
+    for (int pass = 0; pass < 2; pass++) {
+        uint64_t at = 0;
+        for (uint32_t L = 0; L < levels; L++)
+            b.lv[L] = batch_level(base, at, b.caps[L], L == g.leaf_level, c->colors);
+        if (!base)
+            base = s.get<uint8_t>("eb_levels", at);
+    }
     b.keys = s.get<uint32_t>("eb_keys", maxn);
     b.vals = s.get<uint32_t>("eb_vals", maxn);
     b.keys2 = s.get<uint32_t>("eb_keys2", maxn);
