@@ -127,17 +127,21 @@ void table_reset(hd_ctx* c)
 // Tables in host memory and in files number their pages in claim order
 // (1, 2, ...), with a page table of those numbers.  That is how a pool filled
 // in claim order lies; the pages of a direct-mapped one are gathered on the
-// way out and spread on the way in by their numbers (page_ids), kIoPages at a
-// time through a staging buffer.
+// way out and spread on the way in by their numbers (page_ids) in a staging
+// buffer.  It holds all pages, for one copy: one in pieces of 64 MB into host
+// memory that was never written and is to get 512 MB pages (large numpy arrays)
+// takes 1 ms a MB (a 1 GB table 840-900 ms, in one copy 39).  A small one is
+// kept, as an allocation and its release would be a third of a 2^10 table's
+// export.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kIoPages = 32768; // 64 MB
-constexpr uint32_t kIoPagesLeast = 64;
+constexpr uint64_t kIoPagesKept = 8192; // 16 MB
+constexpr uint64_t kIoPagesLeast = 64;
 
 // The staging buffer for `pages` pages, in as many pieces of n as a device with
 // little room left takes.
 static uint32_t* io_staging(hd_ctx* c, uint64_t pages, uint64_t& n)
 {
-    for (n = std::min<uint64_t>(pages, kIoPages);; n = std::max<uint64_t>(n / 4, kIoPagesLeast)) {
+    for (n = pages;; n = std::max<uint64_t>(n / 4, kIoPagesLeast)) {
         try {
             return c->scratch.get<uint32_t>("io_staging", n * kPage);
         } catch (const StatusError&) {
@@ -145,6 +149,11 @@ static uint32_t* io_staging(hd_ctx* c, uint64_t pages, uint64_t& n)
                 throw;
         }
     }
+}
+static void io_staging_done(hd_ctx* c, uint64_t pages)
+{
+    if (c->t.direct && pages > kIoPagesKept)
+        c->scratch.drop("io_staging");
 }
 
 __global__ void k_direct_entries(Table t, uint64_t n)
@@ -200,7 +209,7 @@ void download_pages(hd_ctx* c, uint32_t* h_page_table, uint32_t* h_pool, uint64_
         }
     }
     HD_CUDA(cudaStreamSynchronize(st));
-    c->scratch.drop("io_staging");
+    io_staging_done(c, pages);
 }
 
 void upload_pages(hd_ctx* c, const uint32_t* h_page_table, const uint32_t* h_pool, uint64_t pages)
@@ -225,7 +234,7 @@ void upload_pages(hd_ctx* c, const uint32_t* h_page_table, const uint32_t* h_poo
         }
     }
     HD_CUDA(cudaStreamSynchronize(st));
-    c->scratch.drop("io_staging");
+    io_staging_done(c, pages);
 }
 
 void set_claim_limit(hd_ctx* c, bool gc)
