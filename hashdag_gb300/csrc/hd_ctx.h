@@ -162,12 +162,14 @@ void trace_colors(hd_ctx* c, const uint32_t* d_paths, uint32_t w, uint32_t h, ui
 void copy_source(hd_ctx* c, Editor& ed);
 void tool_buffers(hd_ctx* c, Editor& ed); // hd_tools.cu
 void color_spawn(hd_ctx* c, uint32_t level, uint32_t n, const Level& lv, const Level& next);
-struct ColorsBack { // results of an edit's colour phase, in host memory
-    std::vector<uint8_t> bytes;
+struct ColorsBack { // results of an edit's colour phase, on their way to host memory
+    std::vector<uint8_t> bytes;             // the counts and, of a few replaced leaves, these
+    std::vector<uint32_t> leaf;             // many replaced leaves
+    std::vector<LeafDesc> prev, next;
 };
 void edit_colors(hd_ctx* c, const Editor& ed, std::vector<Level>& lv, const std::vector<uint32_t>& count,
                  uint32_t deepest, bool spawned, ColorsBack& back);
-void edit_colors_done(hd_ctx* c, const ColorsBack& back, UndoFrame& frame);
+void edit_colors_done(hd_ctx* c, ColorsBack& back, UndoFrame& frame);
 bool undo_step(hd_ctx* c, bool redo);
 void push_undo(hd_ctx* c, UndoFrame&& f);
 
