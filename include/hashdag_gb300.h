@@ -389,11 +389,12 @@ typedef struct hd_serve_config {
                                    edits run, edits in arrival order           */
     uint32_t max_renders;    /* render slots (continuous)                      */
     uint32_t realtime;       /* 1: a request is available at its arrival time  */
-    float gc_free_fraction;  /* GC (keeping the undo history) when the free
-                                pool pages fall below this fraction of the
-                                pool, and once more when an edit finds the
-                                pool full (then the edit is retried); 0 =
-                                never.  Above 0 the loop keeps
+    float gc_free_fraction;  /* GC (keeping the undo history) before an edit
+                                when the free pool pages are below this
+                                fraction of the pool and at least 1/128 of the
+                                pool was claimed since the last one, and once
+                                more when an edit finds the pool full (then
+                                the edit is retried); 0 = never.  Above 0 the loop keeps
                                 max(hd_set_page_reserve's pages, pool / 64)
                                 pages back for its GCs                        */
     float light[3];
