@@ -702,9 +702,24 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
     bool plain = c->colors || !two_pass_sort(c->g);
     for (uint32_t i = 0; i < n && !plain; i++)
         plain = edits[i].tool > HD_TOOL_BOX_ADD;
+    const BatchBuffers* buffers = nullptr;
+    if (!plain) {
+        std::vector<uint64_t> cap(c->g.leaf_level + 1, 0);
+        for (uint32_t i = 0; i < n; i++)
+            edit_caps(c->g, make_editor(edits[i]), cap);
+        try {
+            buffers = &batch_levels(c, cap, n);
+        } catch (const StatusError& x) {
+            if (x.status != HD_ERR_OOM)
+                throw;
+            drop_batch_levels(c);
+            plain = true;
+        }
+    }
     if (plain) {
-        // colours, paint, copy and tables of too many buckets for the sort
-        // take the one-edit path, edit by edit
+        // colours, paint, copy, tables of too many buckets for the sort and
+        // batches without room for the bounds of all their edits take the
+        // one-edit path, edit by edit
         float at = 0;
         c->batch_applied = 0;
         for (uint32_t i = 0; i < n; i++) {
@@ -727,10 +742,7 @@ void edit_batch(hd_ctx* c, const hd_edit* edits, uint32_t n, hd_edit_stats* per_
             *total = sum;
         return;
     }
-    std::vector<uint64_t> cap(c->g.leaf_level + 1, 0);
-    for (uint32_t i = 0; i < n; i++)
-        edit_caps(c->g, make_editor(edits[i]), cap);
-    const BatchBuffers& b = batch_levels(c, cap, n);
+    const BatchBuffers& b = *buffers;
     BatchGraph& bg = *c->batch;
     if (c->tuning.mode == HD_BATCH_PERSISTENT) {
         std::vector<EditCounters> ctr(n);

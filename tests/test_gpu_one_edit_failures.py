@@ -107,3 +107,21 @@ def test_edit_without_room_for_its_bounds(gpu, colors, share):
             assert got.firstNodeIndex == root and got.history() == (2, 0)
         want.free()
         got.free()
+
+
+@pytest.mark.parametrize("mode", [1, 0])
+def test_batch_without_room_for_its_bounds(gpu, mode):
+    """A batch whose level arrays do not fit is made edit by edit."""
+    edits = [hd.editor_from_tuple(e) for e in workloads.mixed_edits(DEPTH, 10, (8.0, 60.0), seed=9)]
+    edits.insert(4, hd.SphereEditor((512.0, 512.0, 512.0), 300.0, adding=False))
+    want, got = _context(False), _context(False)
+    for d in (want, got):
+        d.batch_tuning = hd.BatchTuning(4, 4, 304, mode)
+    _, a = want.edit_batch(edits, per_edit=True)
+    got.set_test_scratch_limit(want.memory_stats()["scratch"] * 6 // 10)
+    _, b = got.edit_batch(edits, per_edit=True)
+    assert [(s.num_voxels, s.num_nodes, s.find_or_add_calls, s.nodes_added) for s in a] == \
+        [(s.num_voxels, s.num_nodes, s.find_or_add_calls, s.nodes_added) for s in b]
+    assert want.firstNodeIndex == got.firstNodeIndex and want.history() == got.history() == (11, 0)
+    want.free()
+    got.free()
