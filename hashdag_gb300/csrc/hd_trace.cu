@@ -810,8 +810,9 @@ HD_D uint4* view_paths(uint4* out, uint4* out_copied, uint32_t v, uint64_t frame
 // shadow pass's set-up is fused in: a pixel whose primary ray
 // hit appends its shadow ray (origin on the hit voxel, as shadow_origin) to
 // the list, warp by warp; a miss gets mask 2 at once.  12 blocks an SM: with 16
-// (32 registers) the walk spilled, 22 M local loads in 16 views; 8 views to the
-// host 2366 -> 2335 us, a served trace 6830 -> 6760.
+// (32 registers) the walk spilled, 22 M local loads in 16 views.  The times do
+// not tell 11 to 16 blocks apart: 8 views to the host took 2366 us with 16 and
+// 2335 with 12, and boxes differ by 10 %.
 template <int FMA>
 __global__ void __launch_bounds__(128, 12)
     k_trace_views(__grid_constant__ const Table t, const uint32_t* __restrict__ d_root,
