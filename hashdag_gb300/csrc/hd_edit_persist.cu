@@ -27,7 +27,8 @@
 //    then find-or-add, one warp per bucket run; from kRepeatLevel candidates
 //    on, the repeats and the runs' starts are marked before it.
 //  * Grid barriers are bounded waits: a wait longer than kWaitNs sets
-//    HD_ERR_TIMEOUT and every CTA returns; the host reports the error.
+//    HD_ERR_TIMEOUT and every CTA returns; the host reports a batch's and makes
+//    a single edit level by level.
 //  * Nodes and pages that an edit appends are read by the following edits in
 //    the same launch: every table read uses L2-coherent loads.
 // The graph-per-edit form (hd_edit_batch.cu) stays as the other batch mode.
@@ -151,10 +152,9 @@ HD_D unsigned long long ld_acquire64(const unsigned long long* p)
 // generation word for the last CTA to publish after its arrival.  Arrivals and
 // the flag of a CTA that gave up are one 64-bit word, which every access to it
 // takes whole: an acquire of a word orders nothing behind an atomic of half of
-// it.  Bound by
-// L2 round trips: a poll is one acquire, without a pause until it has waited
-// long (with two reads and a pause a poll, and a fence after, a grid step of
-// almost no work took 2.7-4.3 us, now 2.4-3.5).
+// it.  Bound by L2 round trips: a poll is one acquire, without a pause until it
+// has waited long (with two reads and a pause a poll, and a fence after, a grid
+// step of almost no work took 2.7-4.3 us, now 2.4-3.5).
 HD_D bool grid_sync(Ctl* ctl, uint32_t* err, uint32_t& nbar)
 {
     __shared__ uint32_t ok;
